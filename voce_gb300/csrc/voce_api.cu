@@ -557,6 +557,47 @@ long long voce_rve_footprint(const int dims[3], int precision)
            (precision == VOCE_PREC_FP64 ? nspec * 9 * 8 : 0);
 }
 
+}  // extern "C"
+
+namespace {
+
+// Whether d's slip table is the {111}<110> family with an integral exponent:
+// each system's Schmid 5-vector (crystal axes), scaled to the y variables of
+// voce_fcc.cuh, is one of the 12 canonical coefficient rows or its negative,
+// each row once.  Sets canon and flip.  The rows' entries are small integers
+// met by normalised vectors to a few ulp; 1e-12 separates them from any other
+// table.  (The gam0, n and tau of one slip mode are the same for all systems.)
+bool fcc_table(RveDesc &d)
+{
+    if (d.nsys != VOCE_NS || d.ipow_n < 1) return false;
+    const double w[5] = {std::sqrt(12.0), 2.0, std::sqrt(12.0), std::sqrt(12.0), std::sqrt(12.0)};
+    bool used[VOCE_NS] = {};
+    for (int k = 0; k < VOCE_NS; ++k) {
+        int found = -1, flip = 0;
+        for (int c = 0; c < VOCE_NS && found < 0; ++c) {
+            const int z = c / 4;
+            const double a = (c % 4 == 0 || c % 4 == 2) ? 1.0 : -1.0;     // coefficient of the shear a
+            const double b = (c % 4 == 0 || c % 4 == 3) ? 1.0 : -1.0;     // and of b
+            const double row[3][5] = {{1, -1, 0, b, a}, {-1, -1, b, 0, a}, {-2, 0, b, a, 0}};
+            for (int s = 0; s < 2 && found < 0; ++s) {
+                bool same = true;
+                for (int q = 0; q < 5; ++q)
+                    same = same && std::fabs(d.schxt[5 * k + q] * w[q] - (s ? -1.0 : 1.0) * row[z][q]) < 1e-12;
+                if (same && !used[c]) { found = c; flip = s; }
+            }
+        }
+        if (found < 0) return false;
+        used[found] = true;
+        d.canon[k] = found;
+        d.flip[k] = flip;
+    }
+    return true;
+}
+
+}  // namespace
+
+extern "C" {
+
 // ---------------------------------------------------------------------------
 // SetupJob (init.c:617-828)
 // ---------------------------------------------------------------------------
@@ -711,6 +752,8 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
                 d.hard[q * VOCE_NS + p] = v;
             }
     }
+    // crystal-axes Newton for the {111}<110> family, FP64 Newton forms
+    d.fcc = (precision == VOCE_PREC_FP64 || precision == VOCE_PREC_MIXED) && fcc_table(d) ? 1 : 0;
     // boundary conditions: Udot, Scauchy, creep (init.c:716-745)
     const double *vb = nl->VelGrad_BC, *sb = nl->Stress_BC;
     const double U[9] = {vb[0], vb[5], vb[4], vb[5], vb[1], vb[3], vb[4], vb[3], vb[2]};
@@ -763,7 +806,7 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
     // and precision.
     const long long sm_count = 152;
     long long nb = (nv + 127) / 128;
-    const long long cap = std::max<long long>(sm_count * 2, nr_resident_blocks(nr_kind(r->precision)));
+    const long long cap = std::max<long long>(sm_count * 2, nr_resident_blocks(nr_kind(d)));
     r->npart = (int)(nb < cap ? nb : cap);
     d.npart = r->npart;
     int rc = alloc_device(r);
@@ -805,7 +848,10 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
     if (!lu_inv66(S066)) return fail(VOCE_ERR_SINGULAR, "singular reference stiffness C066");
     std::memcpy(d.S0, S066, sizeof(S066));
     for (int q = 0; q < 36; ++q) d.S0f[q] = (float)d.S0[q];
+    d.P55 = sc.sxt[35] + d.S0[35];   // pressure entry of S_g + S0, the same in every cubic grain
+    d.iP55 = 1.0 / d.P55;
     if (d.nr32 || d.ir) CUDA_TRY(launch_fill_p32(d, r->stream));
+    CUDA_TRY(launch_fill_fcc(d, r->stream));
     double C0t[81];
     c66_to_t4(&C066[0][0], C0t);
     c66_to_t4(&S066[0][0], d.S0t);
@@ -1591,7 +1637,7 @@ long long snapshot_write(voce_rve *r, char *out)
     SnapHead h;
     std::memset(&h, 0, sizeof(h));
     std::memcpy(h.magic, kSnapMagic, 8);
-    h.version = 3;
+    h.version = 4;
     h.desc_size = sizeof(RveDesc);
     h.macro_size = sizeof(MacroDev);
     h.nl_size = sizeof(voce_namelist);
@@ -1683,6 +1729,15 @@ const char *snapshot_desc_problem(const SnapHead &h, const RveDesc &d, const voc
     if (h.npart < 1 || d.npart != h.npart || h.npart > std::max<long long>(1, (d.nv + 127) / 128))
         return "work split";
     if (d.nsys < 1 || d.nsys > VOCE_NS) return "number of slip systems";
+    if (d.fcc != 0) {
+        unsigned seen = 0;
+        for (int k = 0; k < VOCE_NS; ++k) {
+            if (d.canon[k] < 0 || d.canon[k] >= VOCE_NS || d.flip[k] < 0 || d.flip[k] > 1) return "slip table";
+            seen |= 1u << d.canon[k];
+        }
+        if (d.fcc != 1 || d.nsys != VOCE_NS || d.ipow_n < 1 || d.nr32 || d.ir || seen != (1u << VOCE_NS) - 1)
+            return "slip table";
+    }
     if (d.iter_max < 0 || d.iter_max != nl.IterMax) return "IterMax";
     if (d.ipow_n != -1 && (d.ipow_n < 1 || d.ipow_n > 256)) return "flow exponent";
     return nullptr;
@@ -1744,7 +1799,7 @@ int voce_rve_restore(const void *buf, long long size, voce_rve **out)
     if (size < (long long)sizeof(h)) return fail(VOCE_ERR_PARSE, "snapshot too short");
     std::memcpy(&h, in, sizeof(h));
     if (std::memcmp(h.magic, kSnapMagic, 8) != 0) return fail(VOCE_ERR_PARSE, "not an RVE snapshot");
-    if (h.version != 3 || h.desc_size != sizeof(RveDesc) || h.macro_size != sizeof(MacroDev) ||
+    if (h.version != 4 || h.desc_size != sizeof(RveDesc) || h.macro_size != sizeof(MacroDev) ||
         h.nl_size != sizeof(voce_namelist) || h.incr_size != sizeof(voce_increment))
         return fail(VOCE_ERR_UNSUPPORTED, "snapshot written by a different build of the library");
     if (h.total != size) return fail(VOCE_ERR_PARSE, "snapshot of %lld bytes, header says %lld", size, (long long)h.total);

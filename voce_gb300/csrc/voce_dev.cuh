@@ -88,6 +88,9 @@ struct RveDesc {
     long long nv, nspec;
     int solid[3];        // solid[phase id 1..2]
     int nsys, ipow_n;    // ipow_n >= 0: n integral, |r|^(n-1) by multiplication
+    int fcc;             // the slip table is the {111}<110> family: Newton in crystal axes (voce_fcc.cuh)
+    int canon[VOCE_NS];  // fcc: canonical index of each system, and whether its
+    int flip[VOCE_NS];   // direction is the canonical one reversed
     int update_flag, hard_flag, creep, iter_max;
     int mixed;           // spectrum precision: 0 double, 1 float
     int chord;           // FP64 Newton: reuse the last Jacobian once the update is below 1e-4
@@ -107,6 +110,7 @@ struct RveDesc {
     double bn[VOCE_NS * 3], bb[VOCE_NS * 3];
     double S0[36];       // S066 (B basis)
     float S0f[36];       // float copy (mixed-precision error norms)
+    double P55, iP55;    // fcc: pressure entry of S_g + S0 and its reciprocal
     double S0t[81];      // S0 as 3x3x3x3 (get_smacro's dDisGradAvg)
     double Kq[36];       // acoustic tensor coefficients: K6 = Kq * nn6
     float Kqf[36];       // float copy (Green operator of the mixed forms)

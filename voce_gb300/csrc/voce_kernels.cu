@@ -6,6 +6,7 @@
 //   k_fft_x(+1,aacc) -> k_fft_y(+1,aacc) -> k_fft_z_inv(rotl) ->
 //   k_incr_end -> k_finalize_incr
 #include "voce_dev.cuh"
+#include "voce_fcc.cuh"
 #include "voce_kernels.h"
 
 #include <math.h>
@@ -146,6 +147,67 @@ __device__ void schmid_from_tm(const RveDesc &d, long long v, const double (&T)[
         }
 }
 
+// The crystal-axes columns of voxel v (voce_fcc.cuh) for the orientation T
+// (crystal -> sample): U, P_y, S0_y, and y of the stress the voxel has.
+// Column c of the rotation's deviatoric block is the basis tensor B_c turned
+// to sample axes, T B_c T^T; written out tensor by tensor (its columns are
+// products of two columns of T) everything stays in registers.
+__device__ __forceinline__ void fcc_frame(const RveDesc &d, long long v, const double (&T)[3][3])
+{
+    const long long nv = d.nv;
+    double *fx = d.sch + v;
+    const int I6[6] = {0, 1, 2, 1, 0, 0}, J6[6] = {0, 1, 2, 2, 2, 1};
+    double U[5][5], b6[6], z[6];
+    double s[5], t[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int i = 0; i < 5; ++i) s[i] = d.sig[i * nv + v];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const int i = I6[q], j = J6[q];
+            if (c == 0) z[q] = RSQ2 * (T[i][1] * T[j][1] - T[i][0] * T[j][0]);
+            else if (c == 1) z[q] = RSQ6 * (2.0 * T[i][2] * T[j][2] - T[i][0] * T[j][0] - T[i][1] * T[j][1]);
+            else {
+                const int p = c == 2 ? 1 : 0, r = c == 4 ? 1 : 2;
+                z[q] = RSQ2 * (T[i][p] * T[j][r] + T[i][r] * T[j][p]);
+            }
+        }
+        t6_to_b<double>(z, b6);
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            U[i][c] = b6[i] * (c == 1 ? 2.0 : 3.4641016151377545871);   // sqrt 12
+            fx[(FCC_U + 5 * i + c) * nv] = U[i][c];
+            t[c] = fma(U[i][c], s[i], t[c]);
+        }
+        fx[(FCC_Y + c) * nv] = t[c] * (1.0 / fcc_w2(c));
+    }
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        double p0[5], p1[5];   // columns k of S0 U and S_g U
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            p0[i] = p1[i] = 0.0;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                p0[i] = fma(d.S0[i * 6 + j], U[j][k], p0[i]);
+                p1[i] = fma(__ldg(d.sg + (long long)sym6(i, j) * nv + v), U[j][k], p1[i]);
+            }
+        }
+#pragma unroll
+        for (int c = 0; c <= k; ++c) {
+            double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                a0 = fma(U[i][c], p0[i], a0);
+                a1 = fma(U[i][c], p1[i], a1);
+            }
+            fx[(FCC_S0 + sym5(c, k)) * nv] = a0;
+            fx[(FCC_P + sym5(c, k)) * nv] = a0 + a1;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // setup: per-voxel rotation, grain stiffness/compliance, Schmid tensors,
 // initial stress (InitMicroStruct init.c:393-442, InitFields init.c:486-534,
@@ -227,8 +289,8 @@ __global__ void __launch_bounds__(128) k_setup(RveDesc d, SetupConst sc, const d
         for (int k = 0; k < d.nsys; ++k) {
             d.crss[(2 * k) * nv + v] = d.tau0[k];
             d.crss[(2 * k + 1) * nv + v] = d.tau0b[k];
-            d.itau[(2 * k) * nv + v] = 1.0 / d.tau0[k];
-            d.itau[(2 * k + 1) * nv + v] = 1.0 / d.tau0b[k];
+            d.itau[itau_col(d, k, 0) * nv + v] = 1.0 / d.tau0[k];
+            d.itau[itau_col(d, k, 1) * nv + v] = 1.0 / d.tau0b[k];
             if (d.itau32) {
                 put_pair(d.itau32, d.itau_lo, (2 * k) * nv + v, 1.0 / d.tau0[k]);
                 put_pair(d.itau32, d.itau_lo, (2 * k + 1) * nv + v, 1.0 / d.tau0b[k]);
@@ -237,7 +299,7 @@ __global__ void __launch_bounds__(128) k_setup(RveDesc d, SetupConst sc, const d
         double T[3][3];
         for (int i = 0; i < 3; ++i)
             for (int j = 0; j < 3; ++j) T[i][j] = a[j][i];
-        schmid_from_tm(d, v, T);
+        if (!d.fcc) schmid_from_tm(d, v, T);   // (the crystal-axes columns wait for S0: k_fill_fcc)
     }
     // voxel count and C066 partial sums (37 values) in three passes of 15
     // (the 16th slot of block_partials is a max and stays unused)
@@ -1617,6 +1679,167 @@ __device__ void nr_unit(const RveDesc &d, int unit, int nunits)
 }
 
 
+// ---------------------------------------------------------------------------
+// UpdateStress (evolution.c:3-168) for an RVE of the {111}<110> family in
+// crystal axes (voce_fcc.cuh), FP64: the FP64 and VOCE_PREC_MIXED forms.  The
+// same Newton iteration as newton_fp64 -- the exact Jacobian, the stop test of
+// evolution.c:112, the strain rate and the norms at the stress before the last
+// update -- in the variables y, so its iterates agree to rounding.
+//
+// Bound: the FP64 pipe (64 cycles of an SM quarter's pipe per warp
+// instruction).  A Newton iteration takes about 335 FP64 operations instead
+// of about 680 in sample axes: 26 instead of 60 for the resolved shears, 32
+// instead of 60 for the strain rate, 40 + 15 instead of 240 + 15 for the
+// tangent, 85 instead of 125 for the 5x5 solve (the pressure decouples).
+// Measured per launch against kb_nr (FP64 form, first increment): 64^3 879 ->
+// 495 us, 128^3 10.4 -> 5.6 ms, 16^3 (a grain per voxel) 86 -> 50 us.  kb_nr
+// stays for every other slip table and for non-integral exponents.
+// CHORD: chord steps as in newton_fp64 (VOCE_PREC_MIXED with d.chord).
+// ---------------------------------------------------------------------------
+template <bool CHORD>
+__device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
+{
+    __shared__ double s_acc[VOCE_NPART][VOCE_NR_THREADS];
+    __shared__ int s_it[2][VOCE_NR_THREADS];
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < VOCE_NPART; ++q) s_acc[q][tid] = 0.0;
+    s_it[0][tid] = 0;
+    s_it[1][tid] = 0;
+    const long long nv = d.nv;
+    const double dtg = d.dt * d.gam0[0], dtgn = dtg * d.nrs[0];
+    for (long long v = (long long)unit * blockDim.x + threadIdx.x; v < nv;
+         v += (long long)nunits * blockDim.x) {
+        const int ph = d.phase[v];
+        if (!d.solid[ph]) {
+#pragma unroll
+            for (int c = 0; c < 6; ++c) { d.sig[c * nv + v] = 0.0; d.sigp[c * nv + v] = 0.0; }
+            continue;
+        }
+        double *fx = d.sch + v;
+        // y of the Green iterate, cc_y = U^T (eps - dg) - S0_y y, and the
+        // pressure component of both
+        double yl[5], cc[5];
+        const double s5l = d.sig[5 * nv + v], g5 = -d.dgs[5 * nv + v];
+        {
+            double e6[5];
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                yl[c] = fx[(FCC_Y + c) * nv];
+                e6[c] = d.eps[c * nv + v] - d.dgs[c * nv + v];
+            }
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                double s = 0.0;
+#pragma unroll
+                for (int i = 0; i < 5; ++i) s = fma(fx[(FCC_U + 5 * i + c) * nv], e6[i], s);
+                cc[c] = s;
+            }
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+#pragma unroll
+                for (int j = i; j < 5; ++j) {
+                    const double q = fx[(FCC_S0 + sym5(i, j)) * nv];
+                    cc[i] = fma(-q, yl[j], cc[i]);
+                    if (i != j) cc[j] = fma(-q, yl[i], cc[j]);
+                }
+        }
+        const double cc5 = fma(-d.S0[35], s5l, g5);
+        // sqrt(cnr)/signorm > 1e-7 (evolution.c:112) tested as cnr > 1e-14 signorm^2
+        const double thr = 1e-14 * fma(s5l, s5l, fcc_norm2<double>(yl));
+        double y[5], yp[5], Rl[5], s5 = s5l, s5p = s5l, R5 = 0.0;
+#pragma unroll
+        for (int c = 0; c < 5; ++c) { y[c] = yl[c]; yp[c] = yl[c]; Rl[c] = 0.0; }
+        int it = 0;
+        bool go = true, fresh = true;
+        double L[15];
+        (void)fresh;
+        while (go && it < 100) {
+            ++it;
+            double E[5], x[5], J[15];
+#pragma unroll
+            for (int c = 0; c < 5; ++c) yp[c] = y[c];
+            s5p = s5;
+            if (!CHORD || fresh) fcc_flow<true>(d, v, y, E, J);
+            else fcc_flow<false>(d, v, y, E, J);
+#pragma unroll
+            for (int c = 0; c < 5; ++c) x[c] = fma(dtg, E[c], cc[c]);
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+#pragma unroll
+                for (int j = i; j < 5; ++j) {
+                    const double q = __ldg(fx + (FCC_P + sym5(i, j)) * nv);
+                    x[i] = fma(q, y[j], x[i]);
+                    if (i != j) x[j] = fma(q, y[i], x[j]);
+                    if (!CHORD || fresh) L[sym5(i, j)] = fma(dtgn, J[sym5(i, j)], q);
+                }
+#pragma unroll
+            for (int c = 0; c < 5; ++c) Rl[c] = x[c];
+            R5 = fma(d.P55, s5, cc5);
+            if (!CHORD || fresh) fcc_factor(L);
+            fcc_solve<double>(L, x);
+            const double x5 = R5 * d.iP55;
+#pragma unroll
+            for (int c = 0; c < 5; ++c) y[c] -= x[c];
+            s5 -= x5;
+            const double cnr = fma(x5, x5, fcc_norm2<double>(x));
+            go = cnr > thr;
+            if (CHORD) fresh = !d.chord || cnr > 1e6 * thr;
+        }
+        // |sig - lam| and the strain-compatibility norm |Rl - S0 (sp - lam)|
+        // (evolution.c:118-123)
+        double ncs, nce;
+        {
+            double dy[5], te[5];
+#pragma unroll
+            for (int c = 0; c < 5; ++c) { dy[c] = y[c] - yl[c]; te[c] = Rl[c]; }
+            const double d5 = s5 - s5l;
+            ncs = sqrt(fma(d5, d5, fcc_norm2<double>(dy)));
+#pragma unroll
+            for (int c = 0; c < 5; ++c) dy[c] = yp[c] - yl[c];
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+#pragma unroll
+                for (int j = i; j < 5; ++j) {
+                    const double q = reread(fx + (FCC_S0 + sym5(i, j)) * nv);
+                    te[i] = fma(-q, dy[j], te[i]);
+                    if (i != j) te[j] = fma(-q, dy[i], te[j]);
+                }
+            const double t5 = fma(-d.S0[35], s5p - s5l, R5);
+            nce = sqrt(fma(t5, t5, fcc_dual2<double>(te)));
+        }
+        s_acc[0][tid] += ncs;
+        s_acc[1][tid] += nce;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) {
+            double s = s5;
+            if (i < 5) {
+                s = 0.0;
+#pragma unroll
+                for (int c = 0; c < 5; ++c) s = fma(reread(fx + (FCC_U + 5 * i + c) * nv), y[c], s);
+                fx[(FCC_Y + i) * nv] = y[i];
+            }
+            d.sig[i * nv + v] = s;
+            d.sigp[i * nv + v] = i < 5 ? yp[i < 5 ? i : 0] : s5p;
+            s_acc[2 + i][tid] += s;
+            if (ph == 1 && !d.all_ph1) s_acc[8 + i][tid] += s;
+        }
+        s_it[0][tid] += it;
+        s_it[1][tid] = max(s_it[1][tid], it);
+    }
+    double acc[VOCE_NPART];
+#pragma unroll
+    for (int q = 0; q < VOCE_NPART; ++q) acc[q] = s_acc[q][tid];
+    if (d.all_ph1) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) acc[8 + c] = acc[2 + c];
+    }
+    acc[14] = (double)s_it[0][tid];
+    acc[15] = (double)s_it[1][tid];
+    block_partials(acc, d.part + (long long)unit * VOCE_NPART);
+}
+
+
 __device__ double vm_strain(const double *t)  // VonMises, evolution.c:243-262
 {
     double tr = t[0] + t[4] + t[8], vm = 0.0;
@@ -1824,8 +2047,8 @@ __device__ void harden_voxel(const RveDesc &d, long long v, const double *gd)
         const double c1 = d.crss[(2 * i + 1) * nv + v] + inc;
         d.crss[(2 * i) * nv + v] = c0;
         d.crss[(2 * i + 1) * nv + v] = c1;
-        d.itau[(2 * i) * nv + v] = 1.0 / c0;
-        d.itau[(2 * i + 1) * nv + v] = 1.0 / c1;
+        d.itau[itau_col(d, i, 0) * nv + v] = 1.0 / c0;
+        d.itau[itau_col(d, i, 1) * nv + v] = 1.0 / c1;
         if (d.itau32) {
             put_pair(d.itau32, d.itau_lo, (2 * i) * nv + v, 1.0 / c0);
             put_pair(d.itau32, d.itau_lo, (2 * i + 1) * nv + v, 1.0 / c1);
@@ -1861,6 +2084,46 @@ __device__ void orientation(double (&tran)[3][3], double (&rot)[3][3])
         }
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 3; ++b) tran[a][b] = tn[a][b];
+}
+
+// The flow rule of the increment's end for the crystal-axes form: the stress
+// sp = (y, s5) in, its sample 6-vector out; shear rates gd and tx = |r|^(n-1)
+// n gam0 / tau of every system in file order, strain rate ed in sample axes
+__device__ void fcc_flow_out(const RveDesc &d, long long v, double (&sp)[6], double (&ed)[5], double (&gd)[VOCE_NS],
+                             double (&tx)[VOCE_NS])
+{
+    const long long nv = d.nv;
+    double y[5], E[5];
+    for (int c = 0; c < 5; ++c) y[c] = sp[c];
+    sfor<0, 3>([&](auto zc) {
+        constexpr int Z = decltype(zc)::v;
+        double c[4], g[4];
+        fcc_rss<Z, double>(y, c);
+        for (int k = 0; k < 4; ++k) {
+            const int neg = __double2hiint(c[k]) < 0;
+            const double it = d.itau[(long long)(2 * (4 * Z + k) + neg) * nv + v];
+            const double r = c[k] * it;
+            const double q = d.gam0[0] * pow_abs_e(fabs(r), d.ipow_n - 1);
+            g[k] = q * r;
+            for (int s = 0; s < VOCE_NS; ++s)
+                if (d.canon[s] == 4 * Z + k) {
+                    gd[s] = d.flip[s] ? -g[k] : g[k];
+                    tx[s] = (q * it) * d.nrs[s];
+                }
+        }
+        fcc_edot<Z, double>(g, E);
+    });
+    const double *fx = d.sch + v;
+    for (int i = 0; i < 5; ++i) {
+        double s = 0.0, e = 0.0;
+        for (int c = 0; c < 5; ++c) {
+            const double u = fx[(FCC_U + 5 * i + c) * nv];
+            s += u * y[c];
+            e += u * (E[c] / fcc_w2(c));
+        }
+        sp[i] = s;
+        ed[i] = e;
+    }
 }
 
 // increment epilogue (evolution.c:433-530; update_orient constitutive.c:171-248; harden :250-310;
@@ -1900,7 +2163,8 @@ __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
         if (d.solid[ph]) {
             double sp[6], gd[VOCE_NS], tx[VOCE_NS];
             for (int c = 0; c < 6; ++c) sp[c] = d.sigp[c * nv + v];
-            flow_rule<false, true, double>(d, v, sp, ed, (double *)nullptr, gd, tx);
+            if (d.fcc) fcc_flow_out(d, v, sp, ed, gd, tx);
+            else flow_rule<false, true, double>(d, v, sp, ed, (double *)nullptr, gd, tx);
             for (int k = 0; k < d.nsys; ++k) {
                 d.gamdot[k * nv + v] = gd[k];
                 d.taux[k * nv + v] = tx[k];
@@ -1943,7 +2207,16 @@ __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
             // resolved shear stresses for the diagnostics, with the Schmid
             // tensors of this increment (the reorientation below replaces them)
             double rss[VOCE_NS];
-            if (hrd)
+            if (hrd && d.fcc) {
+                double y[5], c[4];
+                for (int q = 0; q < 5; ++q) y[q] = d.sch[(FCC_Y + q) * nv + v];
+                sfor<0, 3>([&](auto zc) {
+                    constexpr int Z = decltype(zc)::v;
+                    fcc_rss<Z, double>(y, c);
+                    for (int k = 0; k < d.nsys; ++k)
+                        if (d.canon[k] / 4 == Z) rss[k] = d.flip[k] ? -c[d.canon[k] % 4] : c[d.canon[k] % 4];
+                });
+            } else if (hrd)
                 for (int k = 0; k < d.nsys; ++k) {
                     const double *sc = d.sch + (long long)(5 * k) * nv + v;
                     rss[k] = sc[0] * s6[0] + sc[nv] * s6[1] + sc[2 * nv] * s6[2] + sc[3 * nv] * s6[3] +
@@ -1982,7 +2255,8 @@ __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
                 orientation(T, Rot);
                 for (int a = 0; a < 3; ++a)
                     for (int b = 0; b < 3; ++b) d.tm[(3 * a + b) * nv + v] = T[a][b];
-                schmid_from_tm(d, v, T);
+                if (d.fcc) fcc_frame(d, v, T);
+                else schmid_from_tm(d, v, T);
             }
             if (hrd) {
                 harden_voxel(d, v, gd);
@@ -2404,6 +2678,20 @@ kb_nr(const RveDesc *descs, const int2 *map, int total)
     }
 }
 
+#ifndef VOCE_NR_FCC_BLOCKS
+#define VOCE_NR_FCC_BLOCKS 3
+#endif
+template <bool CHORD>
+__global__ void __launch_bounds__(128, VOCE_NR_FCC_BLOCKS) kb_nr_fcc(const RveDesc *descs, const int2 *map, int total)
+{
+    for (int w = blockIdx.x; w < total; w += gridDim.x) {
+        const int2 e = map[w];
+        const RveDesc &d = descs[e.x];
+        if (!unit_on(d, MASK_ACTIVE)) continue;
+        nr_fcc_unit<CHORD>(d, e.y, d.npart);
+    }
+}
+
 __global__ void __launch_bounds__(128) kb_incr_end(const RveDesc *descs, const int2 *map, int total)
 {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
@@ -2514,6 +2802,8 @@ static size_t smem_lines(int L, int NL)
 void batch_units(const RveDesc &d, int u[BP_COUNT])
 {
     u[BP_NP] = d.npart;
+    u[BP_NG] = d.fcc ? 0 : d.npart;
+    u[BP_NF] = d.fcc ? d.npart : 0;
     u[BP_ZF] = d.nx * (d.ny / d.zrows);
     u[BP_Y6] = 6 * d.nzh * (d.nx / d.yxt);
     u[BP_XG] = d.nzh * (d.ny / d.xkc);
@@ -2576,8 +2866,8 @@ static const int kNrStageBytes = VOCE_STAGE_FLOATS * VOCE_NR_THREADS * (int)size
 int nr_resident_blocks(int kind)
 {
     // several host threads may ask at once: each computes the same value
-    static std::atomic<int> cached[3];
-    std::atomic<int> &c = cached[(kind >= 0 && kind < 3) ? kind : 0];
+    static std::atomic<int> cached[4];
+    std::atomic<int> &c = cached[(kind >= 0 && kind < 4) ? kind : 0];
     if (!c.load()) {
         int dev = 0, sms = 152, per = 2;
         cudaGetDevice(&dev);
@@ -2590,6 +2880,11 @@ int nr_resident_blocks(int kind)
                                  kNrStageBytes);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr<false, false, true>, VOCE_NR_THREADS,
                                                           kNrStageBytes);
+        } else if (kind == 3) {
+            int chord = 2;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr_fcc<false>, VOCE_NR_THREADS, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&chord, kb_nr_fcc<true>, VOCE_NR_THREADS, 0);
+            per = std::min(per, chord);
         } else {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr<false>, VOCE_NR_THREADS, 0);
         }
@@ -2633,20 +2928,26 @@ static void plan_iteration_t(const BatchPlan &bp, cudaStream_t s, Prof &pf, cuda
     pf.begin(K_FFT_Z_INV, s);
     kb_fft_z_inv<R><<<grid_for(bp.total[BP_ZI], FG), 256, bp.smem[BP_ZI], s>>>(D, bp.map[BP_ZI], bp.total[BP_ZI], 0);
     pf.end(K_FFT_Z_INV, s);
+    // a plan's RVEs of the {111}<110> family and the others: one launch each,
+    // where there are any
     pf.begin(K_NR, s);
-    if (bp.nr32)
-        kb_nr<true><<<grid_for(bp.total[BP_NP], nr_resident_blocks(1)), VOCE_NR_THREADS, kNrStageBytes, s>>>(
-            D, bp.map[BP_NP], bp.total[BP_NP]);
-    else if (bp.ir)
-        kb_nr<false, false, true><<<grid_for(bp.total[BP_NP], nr_resident_blocks(2)), VOCE_NR_THREADS,
-                                    kNrStageBytes, s>>>(D, bp.map[BP_NP], bp.total[BP_NP]);
-    else if (bp.mixed)
-        kb_nr<false, true><<<grid_for(bp.total[BP_NP], nr_resident_blocks(0)), VOCE_NR_THREADS, 0, s>>>(
-            D, bp.map[BP_NP], bp.total[BP_NP]);
-    else
-        kb_nr<false><<<grid_for(bp.total[BP_NP], nr_resident_blocks(0)), VOCE_NR_THREADS, 0, s>>>(
-            D, bp.map[BP_NP], bp.total[BP_NP]);
-    pf.end(K_NR, s);
+    int launched = 0;
+    if (const int n = bp.total[BP_NF]) {
+        const int g = grid_for(n, nr_resident_blocks(3));
+        if (bp.mixed) kb_nr_fcc<true><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
+        else kb_nr_fcc<false><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
+        ++launched;
+    }
+    if (const int n = bp.total[BP_NG]) {
+        const int kind = bp.nr32 ? 1 : bp.ir ? 2 : 0;
+        const int g = grid_for(n, nr_resident_blocks(kind));
+        if (bp.nr32) kb_nr<true><<<g, VOCE_NR_THREADS, kNrStageBytes, s>>>(D, bp.map[BP_NG], n);
+        else if (bp.ir) kb_nr<false, false, true><<<g, VOCE_NR_THREADS, kNrStageBytes, s>>>(D, bp.map[BP_NG], n);
+        else if (bp.mixed) kb_nr<false, true><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NG], n);
+        else kb_nr<false><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NG], n);
+        ++launched;
+    }
+    pf.end(K_NR, s, launched);
     pf.begin(K_FIN_ITER, s);
     kb_finalize<<<grid_for(bp.nrve, 152 * 4), 256, 0, s>>>(D, bp.nrve, 0, cond, use_cond);
     pf.end(K_FIN_ITER, s);
@@ -2873,6 +3174,28 @@ cudaError_t launch_fill_p32(const RveDesc &d, cudaStream_t s)
     int blocks = (int)((d.nv + 255) / 256);
     if (blocks > 152 * 8) blocks = 152 * 8;
     k_fill_p32<<<blocks, 256, 0, s>>>(d);
+    return cudaGetLastError();
+}
+
+// the crystal-axes columns of every solid voxel, once S0 is known
+__global__ void __launch_bounds__(128) k_fill_fcc(RveDesc d)
+{
+    for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < d.nv;
+         v += (long long)gridDim.x * blockDim.x) {
+        if (!d.solid[d.phase[v]]) continue;
+        double T[3][3];
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j) T[i][j] = d.tm[(3 * i + j) * d.nv + v];
+        fcc_frame(d, v, T);
+    }
+}
+
+cudaError_t launch_fill_fcc(const RveDesc &d, cudaStream_t s)
+{
+    if (!d.fcc) return cudaSuccess;
+    int blocks = (int)((d.nv + 127) / 128);
+    if (blocks > 152 * 8) blocks = 152 * 8;
+    k_fill_fcc<<<blocks, 128, 0, s>>>(d);
     return cudaGetLastError();
 }
 

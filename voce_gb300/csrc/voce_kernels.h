@@ -54,7 +54,8 @@ struct Prof {
 
 // Work lists of one batch (device memory): per phase, (rve, unit) pairs.
 enum BatchPhase {
-    BP_NP = 0,   // Newton / increment-end / prelude units (npart per RVE)
+    BP_NP = 0,   // increment-end / prelude units (npart per RVE)
+    BP_NG, BP_NF,   // Newton units: RVEs with a general slip table, of the {111}<110> family
     BP_ZF, BP_Y6, BP_XG, BP_ZI, BP_X3, BP_Y3, BP_Z3, BP_COUNT
 };
 struct BatchPlan {
@@ -101,10 +102,12 @@ cudaError_t launch_voronoi(int nx, int ny, int nz, int ns, const double *seeds, 
 cudaError_t launch_fill_green(const RveDesc &d, cudaStream_t s);
 // the mixed form's float (S_g + S0), once S0 is set in d
 cudaError_t launch_fill_p32(const RveDesc &d, cudaStream_t s);
-// Newton-kernel instance of a precision form: 0 FP64 Newton (FP64 and
-// mixed forms), 1 FP32 Newton (mixed_nr32), 2 FP64 residual with an FP32
-// Jacobian (mixed_ir)
-inline int nr_kind(int precision) { return precision == 2 ? 1 : precision == 3 ? 2 : 0; }
+// the crystal-axes columns of an RVE of the {111}<110> family, once S0 is set in d
+cudaError_t launch_fill_fcc(const RveDesc &d, cudaStream_t s);
+// Newton-kernel instance of an RVE: 0 FP64 Newton (FP64 and mixed forms),
+// 1 FP32 Newton (mixed_nr32), 2 FP64 residual with an FP32 Jacobian
+// (mixed_ir), 3 FP64 Newton in crystal axes
+inline int nr_kind(const RveDesc &d) { return d.fcc ? 3 : d.nr32 ? 1 : d.ir ? 2 : 0; }
 // kb_nr blocks resident on the current GPU (SMs x blocks per SM) for an
 // instance of nr_kind
 int nr_resident_blocks(int kind);
