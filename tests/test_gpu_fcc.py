@@ -6,8 +6,12 @@ The general path is reached with the same table moved off the family by a
 relative 4e-11 in one component of every plane normal.  That moves the Schmid
 tensors by a few 1e-11, the converged stress by as much, and the strain rate
 (power n = 20) by some 20 times that: below the 1e-9 bound the FP64 form is
-held to against the reference.  The single-precision-spectrum forms are held
-to ten single-precision roundings instead (1e-6)."""
+held to against the reference.  The forms with a single-precision spectrum are
+held to what separates them from the FP64 form: mixed (FP64 Newton) ten
+single-precision roundings, 1e-6; mixed_ir, whose strain rate is evaluated at
+the start of its FP64 steps, the 1e-5 it keeps to an exact-Jacobian Newton;
+mixed_nr32, where an increment that ends at IterMax may end on a solution in
+single precision alone (a few 1e-6), n = 20 times that for the rates, 2e-4."""
 import numpy as np
 import pytest
 
@@ -15,7 +19,7 @@ from voce_gb300 import capi, synth
 
 pytestmark = pytest.mark.gpu
 
-TOL = {capi.PREC_FP64: 1e-9, capi.PREC_MIXED: 1e-6}
+TOL = {capi.PREC_FP64: 1e-9, capi.PREC_MIXED: 1e-6, capi.PREC_MIXED_IR: 1e-5, capi.PREC_MIXED_NR32: 2e-4}
 
 
 def _slip(order, signs, shift=0.0, nrs=20.0, tau_back=None):
@@ -74,7 +78,8 @@ def test_crystal_axes_newton_against_the_general_one(prec, dims, nrs, tau_back, 
     n = 4                                  # through reorientation (2) and hardening (3)
     inc, out = _solve(prec, nl, _slip(order, signs, 0.0, nrs, tau_back), mesh, n)
     inc0, out0 = _solve(prec, nl, _slip(order, signs, 4e-11, nrs, tau_back), mesh, n)
-    assert [x["iters"] for x in inc] == [x["iters"] for x in inc0]
+    slack = 0 if prec in (capi.PREC_FP64, capi.PREC_MIXED) else 1
+    assert all(abs(x["iters"] - y["iters"]) <= slack for x, y in zip(inc, inc0))
     for f, a in out.items():
         b = out0[f]
         assert np.all(np.isfinite(a))
@@ -84,7 +89,8 @@ def test_crystal_axes_newton_against_the_general_one(prec, dims, nrs, tau_back, 
             assert np.abs(np.array(a[k]) - b[k]).max() <= TOL[prec] * np.abs(b[k]).max(), k
 
 
-def test_batch_of_both_newton_paths(voce_lib):
+@pytest.mark.parametrize("prec", sorted(TOL))
+def test_batch_of_both_newton_paths(prec, voce_lib):
     """A batch that mixes RVEs of the family with one off it gives each the
     bits it has alone."""
     rng = np.random.Generator(np.random.PCG64(93))
@@ -92,10 +98,10 @@ def test_batch_of_both_newton_paths(voce_lib):
     nls = [_namelist(m.dims, synth.random_traceless_load(rng), 40) for m in meshes]
     plain = [(k, np.ones(2, dtype=int)) for k in range(12)]
     slips = [_slip([p[0] for p in plain], [p[1] for p in plain], s) for s in (0.0, 1e-3, 0.0)]
-    alone = [_solve(capi.PREC_FP64, nl, s, m, 2) for nl, s, m in zip(nls, slips, meshes)]
-    rves = [capi.Rve.create(nl, s, m.euler_deg, m.grain, m.phase, capi.PREC_FP64)
+    alone = [_solve(prec, nl, s, m, 2) for nl, s, m in zip(nls, slips, meshes)]
+    rves = [capi.Rve.create(nl, s, m.euler_deg, m.grain, m.phase, prec)
             for nl, s, m in zip(nls, slips, meshes)]
-    with capi.Batch(capi.PREC_FP64) as b:
+    with capi.Batch(prec) as b:
         for r in rves:
             b.add(r, 2)
         assert b.run() == 0

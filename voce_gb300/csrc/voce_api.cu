@@ -521,8 +521,15 @@ void for_state(RveDesc &d, F &&f)
     f((void **)&d.taux, 12 * nv * D);    f((void **)&d.svm, nv * D);
     f((void **)&d.evm, nv * D);          f((void **)&d.rotl, 3 * nv * D);
     f((void **)&d.diag, 3 * nv * D);     f((void **)&d.phase, nv * sizeof(int));
-    if (d.ir) f((void **)&d.sgp, 21 * nv * D);
-    if (d.nr32 || d.ir) {
+    // (what the crystal-axes Newton does not use is left out)
+    if (d.ir && !d.fcc) f((void **)&d.sgp, 21 * nv * D);
+    if (d.fcc && (d.nr32 || d.ir)) {
+        if (d.nr32) f((void **)&d.sch32, 15 * nv * S);
+        f((void **)&d.itau32, 24 * nv * S);
+        f((void **)&d.sgp32, 15 * nv * S);
+        f((void **)&d.itau_lo, 24 * nv * S);
+        f((void **)&d.sgp_lo, 15 * nv * S);
+    } else if (d.nr32 || d.ir) {
         f((void **)&d.sch32, 60 * nv * S);
         f((void **)&d.itau32, 24 * nv * S);
         f((void **)&d.sgp32, 21 * nv * S);
@@ -752,8 +759,7 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
                 d.hard[q * VOCE_NS + p] = v;
             }
     }
-    // crystal-axes Newton for the {111}<110> family, FP64 Newton forms
-    d.fcc = (precision == VOCE_PREC_FP64 || precision == VOCE_PREC_MIXED) && fcc_table(d) ? 1 : 0;
+    d.fcc = fcc_table(d) ? 1 : 0;   // crystal-axes Newton
     // boundary conditions: Udot, Scauchy, creep (init.c:716-745)
     const double *vb = nl->VelGrad_BC, *sb = nl->Stress_BC;
     const double U[9] = {vb[0], vb[5], vb[4], vb[5], vb[1], vb[3], vb[4], vb[3], vb[2]};
@@ -850,7 +856,7 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
     for (int q = 0; q < 36; ++q) d.S0f[q] = (float)d.S0[q];
     d.P55 = sc.sxt[35] + d.S0[35];   // pressure entry of S_g + S0, the same in every cubic grain
     d.iP55 = 1.0 / d.P55;
-    if (d.nr32 || d.ir) CUDA_TRY(launch_fill_p32(d, r->stream));
+    if ((d.nr32 || d.ir) && !d.fcc) CUDA_TRY(launch_fill_p32(d, r->stream));
     CUDA_TRY(launch_fill_fcc(d, r->stream));
     double C0t[81];
     c66_to_t4(&C066[0][0], C0t);
@@ -1735,7 +1741,7 @@ const char *snapshot_desc_problem(const SnapHead &h, const RveDesc &d, const voc
             if (d.canon[k] < 0 || d.canon[k] >= VOCE_NS || d.flip[k] < 0 || d.flip[k] > 1) return "slip table";
             seen |= 1u << d.canon[k];
         }
-        if (d.fcc != 1 || d.nsys != VOCE_NS || d.ipow_n < 1 || d.nr32 || d.ir || seen != (1u << VOCE_NS) - 1)
+        if (d.fcc != 1 || d.nsys != VOCE_NS || d.ipow_n < 1 || seen != (1u << VOCE_NS) - 1)
             return "slip table";
     }
     if (d.iter_max < 0 || d.iter_max != nl.IterMax) return "IterMax";

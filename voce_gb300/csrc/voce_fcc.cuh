@@ -34,7 +34,11 @@
 //   40..54 S0_y                    55..59 y of the current stress,
 // `sigp` the penultimate stress as (y, s5), and `itau` the reciprocal CRSS
 // in canonical order: column 2 c + (resolved shear < 0) of canonical system
-// c = 4 z + {0: D + (a + b), 1: D - (a + b), 2: D + (a - b), 3: D - (a - b)}.
+// c = 4 z + {0: D + (a + b), 1: D - (a + b), 2: D + (a - b), 3: D - (a - b)}
+// (so do its float pairs); sgp32 and sgp_lo hold P_y's 15 float pairs, and in
+// the mixed_nr32 form sch32 the 15 floats of S0_y.  The other arrays of the
+// general Newton forms (sch_lo, sgp) stay allocated, because the footprint of
+// an RVE does not depend on its slip table, but are not used.
 #pragma once
 #include "voce_dev.cuh"
 
@@ -143,27 +147,87 @@ __device__ __forceinline__ void fcc_tangent(const T (&h)[4], T (&J)[15])
     }
 }
 
+// all three families: canonical system 4 z + k
+template <typename T>
+__device__ __forceinline__ void fcc_rss12(const T (&y)[5], T (&c)[12])
+{
+    T q[4];
+    fcc_rss<0, T>(y, q);
+    c[0] = q[0]; c[1] = q[1]; c[2] = q[2]; c[3] = q[3];
+    fcc_rss<1, T>(y, q);
+    c[4] = q[0]; c[5] = q[1]; c[6] = q[2]; c[7] = q[3];
+    fcc_rss<2, T>(y, q);
+    c[8] = q[0]; c[9] = q[1]; c[10] = q[2]; c[11] = q[3];
+}
+template <typename T>
+__device__ __forceinline__ void fcc_edot12(const T (&g)[12], T (&E)[5])
+{
+    fcc_edot<0, T>({g[0], g[1], g[2], g[3]}, E);
+    fcc_edot<1, T>({g[4], g[5], g[6], g[7]}, E);
+    fcc_edot<2, T>({g[8], g[9], g[10], g[11]}, E);
+}
+template <typename T>
+__device__ __forceinline__ void fcc_tangent12(const T (&h)[12], T (&J)[15])
+{
+    fcc_tangent<0, T>({h[0], h[1], h[2], h[3]}, J);
+    fcc_tangent<1, T>({h[4], h[5], h[6], h[7]}, J);
+    fcc_tangent<2, T>({h[8], h[9], h[10], h[11]}, J);
+}
+
+// p[k] = |r[k]|^e, e = n - 1.  The exponent is tested once for all N, so that
+// their loads and products stay in one straight run of instructions.
+template <int N, typename T>
+__device__ __forceinline__ void fcc_pow(const T (&r)[N], int e, T (&p)[N])
+{
+    if (e == 19) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const T a2 = r[k] * r[k], a4 = a2 * a2, a8 = a4 * a4, a16 = a8 * a8;
+            p[k] = (a16 * a2) * (sizeof(T) == 4 ? (T)fabsf((float)r[k]) : (T)fabs((double)r[k]));
+        }
+    } else {
+        T b[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            p[k] = T(1);
+            b[k] = sizeof(T) == 4 ? (T)fabsf((float)r[k]) : (T)fabs((double)r[k]);
+        }
+        for (; e; e >>= 1) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                if (e & 1) p[k] *= b[k];
+                b[k] *= b[k];
+            }
+        }
+    }
+}
+
 // One family of the flow rule (constitutive.c:126-194) in FP64, without
-// gam0: g_k = |r|^n sign(r), and with JAC the tangent's h_k = |r|^(n-1)/tau
-// (times gam0 n it is d gdot/d rss).
+// gam0: g = |r|^n sign(r), and with JAC the tangent's h = |r|^(n-1)/tau
+// (times gam0 n it is d gdot / d rss).  The FP64 Newton goes family by family:
+// it is bound by the FP64 pipe, and four systems at a time leave its
+// registers to the matrix (twelve at a time spilled: 528 us at 64^3 against
+// 495 us).
 template <int Z, bool JAC>
 __device__ __forceinline__ void fcc_flow_family(const RveDesc &d, long long v, const double (&y)[5],
                                                 double (&E)[5], double (&J)[15])
 {
-    double c[4], g[4], h[4];
-    fcc_rss<Z, double>(y, c);
-    const int e = d.ipow_n - 1;
+    double r[4], it[4], p[4];
+    fcc_rss<Z, double>(y, r);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const int neg = __double2hiint(c[k]) < 0;
-        const double it = __ldg(d.itau + (long long)(2 * (4 * Z + k) + neg) * d.nv + v);
-        const double r = c[k] * it;
-        const double p = pow_abs_e(fabs(r), e);
-        g[k] = p * r;
-        if (JAC) h[k] = p * it;
+        const int neg = __double2hiint(r[k]) < 0;
+        it[k] = __ldg(d.itau + (long long)(2 * (4 * Z + k) + neg) * d.nv + v);
+        r[k] *= it[k];
     }
-    fcc_edot<Z, double>(g, E);
-    if (JAC) fcc_tangent<Z, double>(h, J);
+    fcc_pow<4, double>(r, d.ipow_n - 1, p);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        r[k] *= p[k];
+        if (JAC) p[k] *= it[k];
+    }
+    fcc_edot<Z, double>(r, E);
+    if (JAC) fcc_tangent<Z, double>(p, J);
 }
 
 template <bool JAC>
@@ -173,6 +237,40 @@ __device__ __forceinline__ void fcc_flow(const RveDesc &d, long long v, const do
     fcc_flow_family<0, JAC>(d, v, y, E, J);
     fcc_flow_family<1, JAC>(d, v, y, E, J);
     fcc_flow_family<2, JAC>(d, v, y, E, J);
+}
+
+// The strain rate of the mixed_ir form's FP64 steps (without gam0): fcc_flow
+// without the tangent, |r|^20 by five products and the sign put on the high
+// word.  Returns whether a ratio |r| reaches 60 (tested on the high word),
+// where the float tangent could overflow.
+__device__ __forceinline__ bool fcc_edot_fp64(const RveDesc &d, long long v, const double (&y)[5], double (&E)[5])
+{
+    double r[12], it[12];
+    fcc_rss12<double>(y, r);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        const int neg = __double2hiint(r[k]) < 0;
+        it[k] = __ldg(d.itau + (long long)(2 * k + neg) * d.nv + v);
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) r[k] *= it[k];
+    bool big = false;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) big = big || (__double2hiint(r[k]) & 0x7fffffff) >= 0x404E0000;
+    if (d.ipow_n == 20) {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            const double a2 = r[k] * r[k], a4 = a2 * a2, a5 = a4 * fabs(r[k]), a10 = a5 * a5, a20 = a10 * a10;
+            r[k] = __hiloint2double(__double2hiint(a20) | (__double2hiint(r[k]) & (int)0x80000000), __double2loint(a20));
+        }
+    } else {
+        double p[12];
+        fcc_pow<12, double>(r, d.ipow_n - 1, p);
+#pragma unroll
+        for (int k = 0; k < 12; ++k) r[k] *= p[k];
+    }
+    fcc_edot12<double>(r, E);
+    return big;
 }
 
 // LDL^T of the symmetric positive definite 5x5 M (packed upper triangle, in
@@ -224,4 +322,225 @@ __device__ __forceinline__ double reread(const double *a)
 __device__ __forceinline__ int itau_col(const RveDesc &d, int k, int f)
 {
     return d.fcc ? 2 * d.canon[k] + (f ^ d.flip[k]) : 2 * k + f;
+}
+
+// ---------------------------------------------------------------------------
+// The same family in single precision and in float pairs, for the forms whose
+// Newton runs on the FP32 pipe (VOCE_PREC_MIXED_IR's start, VOCE_PREC_MIXED_NR32)
+// ---------------------------------------------------------------------------
+
+// fcc_flow in single precision; false when a resolved-shear ratio is too large
+// for |r|^n in single precision, or not a number
+__device__ __forceinline__ bool fcc_flow_f32(const RveDesc &d, long long v, const float (&y)[5], float (&E)[5],
+                                             float (&J)[15])
+{
+    float r[12], it[12], p[12];
+    fcc_rss12<float>(y, r);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) it[k] = __ldg(d.itau32 + (long long)(2 * k + (r[k] < 0.0f)) * d.nv + v);
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        r[k] *= it[k];
+        ok = ok && fabsf(r[k]) < 60.0f;
+    }
+    fcc_pow<12, float>(r, d.ipow_n - 1, p);
+#pragma unroll
+    for (int k = 0; k < 12; ++k) { r[k] *= p[k]; p[k] *= it[k]; }
+    fcc_edot12<float>(r, E);
+    fcc_tangent12<float>(p, J);
+    return ok;
+}
+
+// single-precision fcc_factor, the pivots' reciprocals as in ldlt_solve6f
+__device__ __forceinline__ void fcc_factor(float (&M)[15])
+{
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+        float di, w[5];
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(di) : "f"(M[sym5(j, j)]));
+#pragma unroll
+        for (int i = j + 1; i < 5; ++i) {
+            w[i] = M[sym5(j, i)];
+            M[sym5(j, i)] = w[i] * di;
+        }
+#pragma unroll
+        for (int i = j + 1; i < 5; ++i)
+#pragma unroll
+            for (int k = i; k < 5; ++k) M[sym5(i, k)] = fmaf(-M[sym5(j, i)], w[k], M[sym5(i, k)]);
+        M[sym5(j, j)] = di;
+    }
+}
+
+// sums of float pairs that stay unnormalised (a product renormalises first)
+__device__ __forceinline__ ff32 ffs_add(ff32 a, ff32 b)
+{
+    ff32 r;
+    float e;
+    two_sum(a.h, b.h, r.h, e);
+    r.l = e + (a.l + b.l);
+    return r;
+}
+__device__ __forceinline__ ff32 ffs_neg(ff32 a)
+{
+    a.h = -a.h;
+    a.l = -a.l;
+    return a;
+}
+__device__ __forceinline__ ff32 ffs_sub(ff32 a, ff32 b) { return ffs_add(a, ffs_neg(b)); }
+__device__ __forceinline__ ff32 ffs_sum(float a, float b)
+{
+    ff32 r;
+    two_sum(a, b, r.h, r.l);
+    return r;
+}
+
+// the resolved shears of family Z as float pairs (y: exact floats)
+template <int Z>
+__device__ __forceinline__ void fcc_rss_ff(const float (&y)[5], ff32 *c)
+{
+    ff32 D;
+    if (Z == 0) D = ffs_sum(y[0], -y[1]);
+    else if (Z == 1) D = ffs_sum(-y[0], -y[1]);
+    else { D.h = -2.0f * y[0]; D.l = 0.0f; }
+    const float a = Z == 2 ? y[3] : y[4], b = Z == 0 ? y[3] : y[2];
+    const ff32 u = ffs_sum(a, b), w = ffs_sum(a, -b);
+    c[0] = ffs_add(D, u);
+    c[1] = ffs_sub(D, u);
+    c[2] = ffs_add(D, w);
+    c[3] = ffs_sub(D, w);
+}
+
+// E += the strain-rate sums of family Z (as fcc_edot)
+template <int Z>
+__device__ __forceinline__ void fcc_edot_ff(const ff32 *g, ff32 (&E)[5])
+{
+    const ff32 G = ffs_add(ffs_add(g[0], g[1]), ffs_add(g[2], g[3]));
+    const ff32 gu = ffs_sub(g[0], g[1]), gw = ffs_sub(g[2], g[3]);
+    const ff32 ea = ffs_add(gu, gw), eb = ffs_sub(gu, gw);
+    if (Z == 0) {
+        E[0] = G;
+        E[1] = ffs_neg(G);
+        E[4] = ea;
+        E[3] = eb;
+    } else if (Z == 1) {
+        E[0] = ffs_sub(E[0], G);
+        E[1] = ffs_sub(E[1], G);
+        E[4] = ffs_add(E[4], ea);
+        E[2] = eb;
+    } else {
+        ff32 G2;
+        G2.h = 2.0f * G.h;
+        G2.l = 2.0f * G.l;
+        E[0] = ffs_sub(E[0], G2);
+        E[3] = ffs_add(E[3], ea);
+        E[2] = ffs_add(E[2], eb);
+    }
+}
+
+// the strain rate (without gam0) as float pairs at the single-precision point
+// y; false when a ratio leaves the float range
+__device__ __forceinline__ bool fcc_flow_ff(const RveDesc &d, long long v, const float (&y)[5], ff32 (&E)[5])
+{
+    ff32 r[12];
+    float ih[12], il[12];
+    fcc_rss_ff<0>(y, r);
+    fcc_rss_ff<1>(y, r + 4);
+    fcc_rss_ff<2>(y, r + 8);
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        const long long col = (long long)(2 * k + (r[k].h < 0.0f)) * d.nv + v;
+        ih[k] = __ldg(d.itau32 + col);
+        il[k] = __ldg(d.itau_lo + col);
+    }
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        r[k] = ff_mul(ff_norm(r[k].h, r[k].l), ih[k], il[k]);
+        ok = ok && fabsf(r[k].h) < 60.0f;
+    }
+    // |r|^n sign(r)
+    if (d.ipow_n == 20) {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            const ff32 a2 = ff_mul(r[k], r[k].h, r[k].l), a4 = ff_mul(a2, a2.h, a2.l), a8 = ff_mul(a4, a4.h, a4.l);
+            const ff32 a16 = ff_mul(a8, a8.h, a8.l), a20 = ff_mul(a16, a4.h, a4.l);
+            r[k] = r[k].h < 0.0f ? ffs_neg(a20) : a20;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 12; ++k) {
+            const bool neg = r[k].h < 0.0f;
+            const ff32 p = ff_ipow(neg ? ffs_neg(r[k]) : r[k], d.ipow_n);
+            r[k] = neg ? ffs_neg(p) : p;
+        }
+    }
+    fcc_edot_ff<0>(r, E);
+    fcc_edot_ff<1>(r + 4, E);
+    fcc_edot_ff<2>(r + 8, E);
+    return ok;
+}
+
+// Single-precision Newton from the Green iterate y: steps down to a relative
+// update of sqrt(tol) (at most `most`), the last step's factored matrix left
+// in L.  False when a ratio leaves the float range, a value is not finite or
+// the steps run out.
+__device__ __forceinline__ bool fcc_newton_f32(const RveDesc &d, long long v, const float (&cc)[5], float thr,
+                                               int most, float (&y)[5], const float (&P)[15], float (&L)[15], int &it)
+{
+    const float dtg = (float)d.dt * d.gam0f[0], dtgn = dtg * d.nrsf[0];
+    for (int p = 0; p < most; ++p) {
+        float E[5], x[5];
+        if (!fcc_flow_f32(d, v, y, E, L)) return false;
+#pragma unroll
+        for (int c = 0; c < 5; ++c) x[c] = fmaf(dtg, E[c], cc[c]);
+#pragma unroll
+        for (int i = 0; i < 5; ++i)
+#pragma unroll
+            for (int j = i; j < 5; ++j) {
+                const float q = P[sym5(i, j)];
+                x[i] = fmaf(q, y[j], x[i]);
+                if (i != j) x[j] = fmaf(q, y[i], x[j]);
+                L[sym5(i, j)] = fmaf(dtgn, L[sym5(i, j)], q);
+            }
+        fcc_factor(L);
+        fcc_solve<float>(L, x);
+        const float dn = fcc_norm2<float>(x);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) y[c] -= x[c];
+        ++it;
+        if (!(dn <= 3.0e38f)) return false;   // not finite
+        if (dn < thr) return true;
+    }
+    return false;
+}
+
+// One step on the float-float residual (residual_ff's accuracy, about 48
+// bits) from the single-precision point y with the factors L; x receives the
+// correction.  False when a ratio leaves the float range.
+__device__ __forceinline__ bool fcc_step_ff(const RveDesc &d, long long v, const float (&y)[5], const double (&cc)[5],
+                                            const float (&P)[15], const float (&L)[15], float dtgh, float dtgl,
+                                            float (&x)[5])
+{
+    ff32 E[5], t[5];
+    if (!fcc_flow_ff(d, v, y, E)) return false;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        ff32 c;
+        c.h = (float)cc[i];
+        c.l = (float)(cc[i] - (double)c.h);
+        t[i] = ffs_add(c, ff_mul(ff_norm(E[i].h, E[i].l), dtgh, dtgl));
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+#pragma unroll
+        for (int j = i; j < 5; ++j) {
+            const float q = P[sym5(i, j)], ql = __ldg(d.sgp_lo + (long long)sym5(i, j) * d.nv + v);
+            ff_acc(t[i], q, ql, y[j]);
+            if (i != j) ff_acc(t[j], q, ql, y[i]);
+        }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) x[i] = t[i].h + t[i].l;
+    fcc_solve<float>(L, x);
+    return true;
 }

@@ -204,6 +204,8 @@ __device__ __forceinline__ void fcc_frame(const RveDesc &d, long long v, const d
             }
             fx[(FCC_S0 + sym5(c, k)) * nv] = a0;
             fx[(FCC_P + sym5(c, k)) * nv] = a0 + a1;
+            if (d.sgp32) put_pair(d.sgp32, d.sgp_lo, sym5(c, k) * nv + v, a0 + a1);
+            if (d.nr32) d.sch32[sym5(c, k) * nv + v] = (float)a0;
         }
     }
 }
@@ -292,8 +294,8 @@ __global__ void __launch_bounds__(128) k_setup(RveDesc d, SetupConst sc, const d
             d.itau[itau_col(d, k, 0) * nv + v] = 1.0 / d.tau0[k];
             d.itau[itau_col(d, k, 1) * nv + v] = 1.0 / d.tau0b[k];
             if (d.itau32) {
-                put_pair(d.itau32, d.itau_lo, (2 * k) * nv + v, 1.0 / d.tau0[k]);
-                put_pair(d.itau32, d.itau_lo, (2 * k + 1) * nv + v, 1.0 / d.tau0b[k]);
+                put_pair(d.itau32, d.itau_lo, itau_col(d, k, 0) * nv + v, 1.0 / d.tau0[k]);
+                put_pair(d.itau32, d.itau_lo, itau_col(d, k, 1) * nv + v, 1.0 / d.tau0b[k]);
             }
         }
         double T[3][3];
@@ -1681,22 +1683,173 @@ __device__ void nr_unit(const RveDesc &d, int unit, int nunits)
 
 // ---------------------------------------------------------------------------
 // UpdateStress (evolution.c:3-168) for an RVE of the {111}<110> family in
-// crystal axes (voce_fcc.cuh), FP64: the FP64 and VOCE_PREC_MIXED forms.  The
-// same Newton iteration as newton_fp64 -- the exact Jacobian, the stop test of
-// evolution.c:112, the strain rate and the norms at the stress before the last
-// update -- in the variables y, so its iterates agree to rounding.
+// crystal axes (voce_fcc.cuh), one kernel instance per form.
 //
-// Bound: the FP64 pipe (64 cycles of an SM quarter's pipe per warp
-// instruction).  A Newton iteration takes about 335 FP64 operations instead
-// of about 680 in sample axes: 26 instead of 60 for the resolved shears, 32
-// instead of 60 for the strain rate, 40 + 15 instead of 240 + 15 for the
-// tangent, 85 instead of 125 for the 5x5 solve (the pressure decouples).
-// Measured per launch against kb_nr (FP64 form, first increment): 64^3 879 ->
-// 495 us, 128^3 10.4 -> 5.6 ms, 16^3 (a grain per voxel) 86 -> 50 us.  kb_nr
-// stays for every other slip table and for non-integral exponents.
-// CHORD: chord steps as in newton_fp64 (VOCE_PREC_MIXED with d.chord).
+// FCC_FP64, FCC_CHORD (the FP64 form; VOCE_PREC_MIXED, which may take chord
+// steps as in newton_fp64): the Newton iteration of newton_fp64 -- the exact
+// Jacobian, the stop test of evolution.c:112, the strain rate and the norms at
+// the stress before the last update -- in the variables y, so its iterates
+// agree to rounding.  Bound: the FP64 pipe (64 cycles of an SM quarter's pipe
+// per warp instruction).  A Newton iteration takes about 335 FP64 operations
+// instead of about 680 in sample axes: 26 instead of 60 for the resolved
+// shears, 32 instead of 60 for the strain rate, 40 + 15 instead of 240 + 15
+// for the tangent, 85 instead of 125 for the 5x5 solve (the pressure
+// decouples).  Measured per launch against kb_nr (FP64 form, first
+// increment): 64^3 879 -> 477 us, 128^3 10.4 -> 5.6 ms, 16^3 (a grain per
+// voxel) 86 -> 50 us.
+//
+// FCC_IR (VOCE_PREC_MIXED_IR): newton_ir in the same variables: the start in
+// single precision and float pairs, then steps whose residual, flow rule and
+// stop test are FP64 and whose correction is solved in FP32 with the start's
+// last matrix; 64^3 363 -> 240 us, 256^3 29.9 -> 16.4 ms.  FCC_NR32
+// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 331 us.  Nothing is staged
+// in shared memory any more: the single-precision steps read 15 + 12 floats
+// per voxel instead of 21 + 72.
+//
+// kb_nr stays for every other slip table and for non-integral exponents.
 // ---------------------------------------------------------------------------
+enum { FCC_FP64 = 0, FCC_CHORD = 1, FCC_IR = 2, FCC_NR32 = 3 };
+
+// x += P y with P_y of voxel v in FP64
+__device__ __forceinline__ void fcc_add_Py(const double *fx, long long nv, const double (&y)[5], double (&x)[5])
+{
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+#pragma unroll
+        for (int j = i; j < 5; ++j) {
+            const double q = __ldg(fx + (FCC_P + sym5(i, j)) * nv);
+            x[i] = fma(q, y[j], x[i]);
+            if (i != j) x[j] = fma(q, y[i], x[j]);
+        }
+}
+
+// x := M^-1 x with the FP64 Jacobian at y, for the rare step whose
+// resolved-shear ratio leaves the float range; out of line so that its
+// registers do not weigh on the common path
+__device__ __noinline__ void fcc_fp64_step(const RveDesc &d, long long v, const double *yp, double *xp)
+{
+    double y[5], x[5], E[5], J[15];
+    for (int c = 0; c < 5; ++c) { y[c] = yp[c]; x[c] = xp[c]; }
+    fcc_flow<true>(d, v, y, E, J);
+    const double dtgn = d.dt * d.gam0[0] * d.nrs[0];
+#pragma unroll
+    for (int q = 0; q < 15; ++q) J[q] = fma(dtgn, J[q], d.sch[(FCC_P + q) * d.nv + v]);
+    fcc_factor(J);
+    fcc_solve<double>(J, x);
+    for (int c = 0; c < 5; ++c) xp[c] = x[c];
+}
+
+// the same from registers: the copies keep y and x out of local memory
+__device__ __forceinline__ void fcc_rare_step(const RveDesc &d, long long v, const double (&y)[5], double (&x)[5])
+{
+    double yt[5], xt[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) { yt[c] = y[c]; xt[c] = x[c]; }
+    fcc_fp64_step(d, v, yt, xt);
+#pragma unroll
+    for (int c = 0; c < 5; ++c) x[c] = xt[c];
+}
+
+// The FP64 Newton steps with the exact Jacobian from y (s5 its pressure
+// part): y, s5 the new stress, yp, s5p the stress before the last update, Rl,
+// R5 the residual there
 template <bool CHORD>
+__device__ __forceinline__ void fcc_newton(const RveDesc &d, long long v, const double (&cc)[5], double cc5,
+                                           double thr, double (&y)[5], double &s5, double (&yp)[5], double &s5p,
+                                           double (&Rl)[5], double &R5, int &it)
+{
+    const long long nv = d.nv;
+    const double *fx = d.sch + v;
+    const double dtg = d.dt * d.gam0[0], dtgn = dtg * d.nrs[0];
+    bool go = true, fresh = true;
+    double L[15];
+    (void)fresh;
+    while (go && it < 100) {
+        ++it;
+        double E[5], x[5], J[15];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) yp[c] = y[c];
+        s5p = s5;
+        if (!CHORD || fresh) fcc_flow<true>(d, v, y, E, J);
+        else fcc_flow<false>(d, v, y, E, J);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) x[c] = fma(dtg, E[c], cc[c]);
+        fcc_add_Py(fx, nv, y, x);
+        if (!CHORD || fresh) {
+#pragma unroll
+            for (int q = 0; q < 15; ++q) L[q] = fma(dtgn, J[q], __ldg(fx + (FCC_P + q) * nv));
+            fcc_factor(L);
+        }
+#pragma unroll
+        for (int c = 0; c < 5; ++c) Rl[c] = x[c];
+        R5 = fma(d.P55, s5, cc5);
+        fcc_solve<double>(L, x);
+        const double x5 = R5 * d.iP55;
+#pragma unroll
+        for (int c = 0; c < 5; ++c) y[c] -= x[c];
+        s5 -= x5;
+        const double cnr = fma(x5, x5, fcc_norm2<double>(x));
+        go = cnr > thr;
+        if (CHORD) fresh = !d.chord || cnr > 1e6 * thr;
+    }
+}
+
+// The steps of newton_ir: FP64 residual, flow rule and stop test, the
+// correction in FP32 with the factors L (started: the start's last matrix,
+// kept for every step; otherwise the Jacobian of each step)
+__device__ __forceinline__ void fcc_newton_ir(const RveDesc &d, long long v, bool started, float (&L)[15],
+                                              const double (&cc)[5], double cc5, double thr, double (&y)[5],
+                                              double &s5, double (&yp)[5], double &s5p, double (&Rl)[5], double &R5,
+                                              int &it)
+{
+    const long long nv = d.nv;
+    const double *fx = d.sch + v;
+    const double dtg = d.dt * d.gam0[0];
+    bool go = true;
+    while (go && it < 100) {
+        ++it;
+        double E[5], x[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) yp[c] = y[c];
+        s5p = s5;
+        const bool big = fcc_edot_fp64(d, v, y, E);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) x[c] = fma(dtg, E[c], cc[c]);
+        fcc_add_Py(fx, nv, y, x);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) Rl[c] = x[c];
+        R5 = fma(d.P55, s5, cc5);
+        const double x5 = R5 * d.iP55;
+        bool fp64 = big;
+        if (!big) {
+            float xf[5];
+            if (!started) {
+                const float dtgn = (float)d.dt * d.gam0f[0] * d.nrsf[0];
+                float yf[5], Ef[5];
+#pragma unroll
+                for (int c = 0; c < 5; ++c) yf[c] = (float)y[c];
+                fp64 = !fcc_flow_f32(d, v, yf, Ef, L);   // (the ratio in float may round up to the limit)
+#pragma unroll
+                for (int q = 0; q < 15; ++q) L[q] = fmaf(dtgn, L[q], __ldg(d.sgp32 + (long long)q * nv + v));
+                fcc_factor(L);
+            }
+            if (!fp64) {
+#pragma unroll
+                for (int c = 0; c < 5; ++c) xf[c] = (float)(x[c]);
+                fcc_solve<float>(L, xf);
+#pragma unroll
+                for (int c = 0; c < 5; ++c) x[c] = (double)(xf[c]);
+            }
+        }
+        if (fp64) fcc_rare_step(d, v, y, x);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) y[c] -= x[c];
+        s5 -= x5;
+        go = fma(x5, x5, fcc_norm2<double>(x)) > thr;
+    }
+}
+
+template <int FORM>
 __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
 {
     __shared__ double s_acc[VOCE_NPART][VOCE_NR_THREADS];
@@ -1706,8 +1859,15 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
     for (int q = 0; q < VOCE_NPART; ++q) s_acc[q][tid] = 0.0;
     s_it[0][tid] = 0;
     s_it[1][tid] = 0;
+    bool polish = true;
+    if (FORM == FCC_NR32) {
+        const MacroDev *m = d.macro;
+        polish = !m->first_iter && fmax(fabs(m->Err_e), fabs(m->Err_s)) <= VOCE_POLISH_ERR;
+    }
+    // dt gam0 as a float pair
+    const float dtgh = (float)(d.dt * d.gam0[0]), dtgl = (float)(d.dt * d.gam0[0] - (double)dtgh);
+    (void)polish; (void)dtgh; (void)dtgl;
     const long long nv = d.nv;
-    const double dtg = d.dt * d.gam0[0], dtgn = dtg * d.nrs[0];
     for (long long v = (long long)unit * blockDim.x + threadIdx.x; v < nv;
          v += (long long)nunits * blockDim.x) {
         const int ph = d.phase[v];
@@ -1745,56 +1905,91 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
                 }
         }
         const double cc5 = fma(-d.S0[35], s5l, g5);
+        const double sn2 = fma(s5l, s5l, fcc_norm2<double>(yl));
         // sqrt(cnr)/signorm > 1e-7 (evolution.c:112) tested as cnr > 1e-14 signorm^2
-        const double thr = 1e-14 * fma(s5l, s5l, fcc_norm2<double>(yl));
+        const double thr = 1e-14 * sn2;
         double y[5], yp[5], Rl[5], s5 = s5l, s5p = s5l, R5 = 0.0;
 #pragma unroll
         for (int c = 0; c < 5; ++c) { y[c] = yl[c]; yp[c] = yl[c]; Rl[c] = 0.0; }
         int it = 0;
-        bool go = true, fresh = true;
-        double L[15];
-        (void)fresh;
-        while (go && it < 100) {
-            ++it;
-            double E[5], x[5], J[15];
+        bool converged = false;   // FCC_NR32: the start's point is taken as the solution
+        (void)converged;
+        if constexpr (FORM == FCC_FP64 || FORM == FCC_CHORD) {
+            fcc_newton<FORM == FCC_CHORD>(d, v, cc, cc5, thr, y, s5, yp, s5p, Rl, R5, it);
+        } else {
+            float yf[5], ccf[5], P[15], L[15], xf[5];
+            bool ok = false;
+            if (FORM == FCC_NR32 || d.ir_pred) {
 #pragma unroll
-            for (int c = 0; c < 5; ++c) yp[c] = y[c];
-            s5p = s5;
-            if (!CHORD || fresh) fcc_flow<true>(d, v, y, E, J);
-            else fcc_flow<false>(d, v, y, E, J);
+                for (int q = 0; q < 15; ++q) P[q] = __ldg(d.sgp32 + (long long)q * nv + v);
 #pragma unroll
-            for (int c = 0; c < 5; ++c) x[c] = fma(dtg, E[c], cc[c]);
+                for (int c = 0; c < 5; ++c) { yf[c] = (float)(yl[c]); ccf[c] = (float)(cc[c]); }
+                // before a float-float step single precision stops at a
+                // relative update of 1e-4 (its rounding floor can lie near
+                // 1e-5), alone at 1e-5
+                const float thr32 = (FORM == FCC_NR32 && !polish ? 1e-10f : 1e-8f) * (float)sn2;
+                ok = fcc_newton_f32(d, v, ccf, thr32, FORM == FCC_NR32 ? 24 : 12, yf, P, L, it);
+                if (ok && polish) {
+                    ok = fcc_step_ff(d, v, yf, cc, P, L, dtgh, dtgl, xf);
+                    ++it;
+                } else {
 #pragma unroll
-            for (int i = 0; i < 5; ++i)
-#pragma unroll
-                for (int j = i; j < 5; ++j) {
-                    const double q = __ldg(fx + (FCC_P + sym5(i, j)) * nv);
-                    x[i] = fma(q, y[j], x[i]);
-                    if (i != j) x[j] = fma(q, y[i], x[j]);
-                    if (!CHORD || fresh) L[sym5(i, j)] = fma(dtgn, J[sym5(i, j)], q);
+                    for (int c = 0; c < 5; ++c) xf[c] = 0.0f;
                 }
+                if (ok) {
+                    // the pressure component is linear: its root at once
+                    s5 = -cc5 * d.iP55;
 #pragma unroll
-            for (int c = 0; c < 5; ++c) Rl[c] = x[c];
-            R5 = fma(d.P55, s5, cc5);
-            if (!CHORD || fresh) fcc_factor(L);
-            fcc_solve<double>(L, x);
-            const double x5 = R5 * d.iP55;
+                    for (int c = 0; c < 5; ++c) y[c] = (double)(yf[c]) - (double)(xf[c]);
+                    if (FORM == FCC_NR32) converged = !polish || fcc_norm2<float>(xf) <= (float)(1e-10 * sn2);
+                }
+            }
+            if constexpr (FORM == FCC_IR) {
+                if (!ok) it = 0;
+                fcc_newton_ir(d, v, ok, L, cc, cc5, thr, y, s5, yp, s5p, Rl, R5, it);
+            } else if (converged) {
+                // taken as the converged point: no residual, and the stress
+                // the strain rate is later evaluated at
 #pragma unroll
-            for (int c = 0; c < 5; ++c) y[c] -= x[c];
-            s5 -= x5;
-            const double cnr = fma(x5, x5, fcc_norm2<double>(x));
-            go = cnr > thr;
-            if (CHORD) fresh = !d.chord || cnr > 1e6 * thr;
+                for (int c = 0; c < 5; ++c) yp[c] = y[c];
+                s5p = s5;
+            } else {
+                fcc_newton<false>(d, v, cc, cc5, thr, y, s5, yp, s5p, Rl, R5, it);
+            }
         }
         // |sig - lam| and the strain-compatibility norm |Rl - S0 (sp - lam)|
         // (evolution.c:118-123)
         double ncs, nce;
-        {
+        if constexpr (FORM == FCC_NR32) {
+            // in single precision: they only steer the Green iteration's stop
+            // test at 1e-5
+            float dy[5], te[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+            float d5 = (float)(s5 - s5l), r5 = 0.0f;
+#pragma unroll
+            for (int c = 0; c < 5; ++c) dy[c] = (float)(y[c] - yl[c]);
+            ncs = (double)sqrtf(fmaf(d5, d5, fcc_norm2<float>(dy)));
+            if (!converged) {   // (a point taken as converged: yp = y, no residual)
+#pragma unroll
+                for (int c = 0; c < 5; ++c) { dy[c] = (float)(yp[c] - yl[c]); te[c] = (float)Rl[c]; }
+                d5 = (float)(s5p - s5l);
+                r5 = (float)R5;
+            }
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+#pragma unroll
+                for (int j = i; j < 5; ++j) {
+                    const float q = __ldg(d.sch32 + (long long)sym5(i, j) * nv + v);
+                    te[i] = fmaf(-q, dy[j], te[i]);
+                    if (i != j) te[j] = fmaf(-q, dy[i], te[j]);
+                }
+            const float t5 = fmaf(-d.S0f[35], d5, r5);
+            nce = (double)sqrtf(fmaf(t5, t5, fcc_dual2<float>(te)));
+        } else {
             double dy[5], te[5];
 #pragma unroll
             for (int c = 0; c < 5; ++c) { dy[c] = y[c] - yl[c]; te[c] = Rl[c]; }
             const double d5 = s5 - s5l;
-            ncs = sqrt(fma(d5, d5, fcc_norm2<double>(dy)));
+            const double cs = fma(d5, d5, fcc_norm2<double>(dy));
 #pragma unroll
             for (int c = 0; c < 5; ++c) dy[c] = yp[c] - yl[c];
 #pragma unroll
@@ -1806,7 +2001,11 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
                     if (i != j) te[j] = fma(-q, dy[i], te[j]);
                 }
             const double t5 = fma(-d.S0[35], s5p - s5l, R5);
-            nce = sqrt(fma(t5, t5, fcc_dual2<double>(te)));
+            const double ce = fma(t5, t5, fcc_dual2<double>(te));
+            // the mixed_ir form's norms by a Newton-Raphson square root
+            // (about 1e-13 relative); the other forms' correctly rounded
+            ncs = FORM == FCC_IR ? sqrt_nr(cs) : sqrt(cs);
+            nce = FORM == FCC_IR ? sqrt_nr(ce) : sqrt(ce);
         }
         s_acc[0][tid] += ncs;
         s_acc[1][tid] += nce;
@@ -2050,8 +2249,8 @@ __device__ void harden_voxel(const RveDesc &d, long long v, const double *gd)
         d.itau[itau_col(d, i, 0) * nv + v] = 1.0 / c0;
         d.itau[itau_col(d, i, 1) * nv + v] = 1.0 / c1;
         if (d.itau32) {
-            put_pair(d.itau32, d.itau_lo, (2 * i) * nv + v, 1.0 / c0);
-            put_pair(d.itau32, d.itau_lo, (2 * i + 1) * nv + v, 1.0 / c1);
+            put_pair(d.itau32, d.itau_lo, itau_col(d, i, 0) * nv + v, 1.0 / c0);
+            put_pair(d.itau32, d.itau_lo, itau_col(d, i, 1) * nv + v, 1.0 / c1);
         }
     }
     d.gamacum[v] = gamtot + deltgam;
@@ -2681,14 +2880,17 @@ kb_nr(const RveDesc *descs, const int2 *map, int total)
 #ifndef VOCE_NR_FCC_BLOCKS
 #define VOCE_NR_FCC_BLOCKS 3
 #endif
-template <bool CHORD>
-__global__ void __launch_bounds__(128, VOCE_NR_FCC_BLOCKS) kb_nr_fcc(const RveDesc *descs, const int2 *map, int total)
+#ifndef VOCE_NR_FCC32_BLOCKS
+#define VOCE_NR_FCC32_BLOCKS 3
+#endif
+template <int FORM>
+__global__ void __launch_bounds__(128, FORM >= FCC_IR ? VOCE_NR_FCC32_BLOCKS : VOCE_NR_FCC_BLOCKS) kb_nr_fcc(const RveDesc *descs, const int2 *map, int total)
 {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int2 e = map[w];
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, MASK_ACTIVE)) continue;
-        nr_fcc_unit<CHORD>(d, e.y, d.npart);
+        nr_fcc_unit<FORM>(d, e.y, d.npart);
     }
 }
 
@@ -2866,8 +3068,8 @@ static const int kNrStageBytes = VOCE_STAGE_FLOATS * VOCE_NR_THREADS * (int)size
 int nr_resident_blocks(int kind)
 {
     // several host threads may ask at once: each computes the same value
-    static std::atomic<int> cached[4];
-    std::atomic<int> &c = cached[(kind >= 0 && kind < 4) ? kind : 0];
+    static std::atomic<int> cached[6];
+    std::atomic<int> &c = cached[(kind >= 0 && kind < 6) ? kind : 0];
     if (!c.load()) {
         int dev = 0, sms = 152, per = 2;
         cudaGetDevice(&dev);
@@ -2882,9 +3084,13 @@ int nr_resident_blocks(int kind)
                                                           kNrStageBytes);
         } else if (kind == 3) {
             int chord = 2;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr_fcc<false>, VOCE_NR_THREADS, 0);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&chord, kb_nr_fcc<true>, VOCE_NR_THREADS, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr_fcc<FCC_FP64>, VOCE_NR_THREADS, 0);
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&chord, kb_nr_fcc<FCC_CHORD>, VOCE_NR_THREADS, 0);
             per = std::min(per, chord);
+        } else if (kind == 4) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr_fcc<FCC_IR>, VOCE_NR_THREADS, 0);
+        } else if (kind == 5) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr_fcc<FCC_NR32>, VOCE_NR_THREADS, 0);
         } else {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr<false>, VOCE_NR_THREADS, 0);
         }
@@ -2933,9 +3139,11 @@ static void plan_iteration_t(const BatchPlan &bp, cudaStream_t s, Prof &pf, cuda
     pf.begin(K_NR, s);
     int launched = 0;
     if (const int n = bp.total[BP_NF]) {
-        const int g = grid_for(n, nr_resident_blocks(3));
-        if (bp.mixed) kb_nr_fcc<true><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
-        else kb_nr_fcc<false><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
+        const int g = grid_for(n, nr_resident_blocks(bp.nr32 ? 5 : bp.ir ? 4 : 3));
+        if (bp.nr32) kb_nr_fcc<FCC_NR32><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
+        else if (bp.ir) kb_nr_fcc<FCC_IR><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
+        else if (bp.mixed) kb_nr_fcc<FCC_CHORD><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
+        else kb_nr_fcc<FCC_FP64><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
         ++launched;
     }
     if (const int n = bp.total[BP_NG]) {

@@ -106,8 +106,8 @@ cudaError_t launch_fill_p32(const RveDesc &d, cudaStream_t s);
 cudaError_t launch_fill_fcc(const RveDesc &d, cudaStream_t s);
 // Newton-kernel instance of an RVE: 0 FP64 Newton (FP64 and mixed forms),
 // 1 FP32 Newton (mixed_nr32), 2 FP64 residual with an FP32 Jacobian
-// (mixed_ir), 3 FP64 Newton in crystal axes
-inline int nr_kind(const RveDesc &d) { return d.fcc ? 3 : d.nr32 ? 1 : d.ir ? 2 : 0; }
+// (mixed_ir); 3, 5 and 4 the same in crystal axes
+inline int nr_kind(const RveDesc &d) { return (d.fcc ? 3 : 0) + (d.nr32 ? (d.fcc ? 2 : 1) : d.ir ? (d.fcc ? 1 : 2) : 0); }
 // kb_nr blocks resident on the current GPU (SMs x blocks per SM) for an
 // instance of nr_kind
 int nr_resident_blocks(int kind);
