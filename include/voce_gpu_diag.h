@@ -129,7 +129,10 @@ int voce_rve_fft_schedule_count(const voce_rve *r, int axis);
  * before the last update, so those move by up to ~1e-8 relative.  That is
  * far inside the mixed form's error (single-precision spectrum) and outside
  * the FP64 form's parity bound, so the FP64 form never takes chord steps.
- * On (1) by default; applies to RVEs created afterwards. */
+ * On (1) by default; applies to RVEs created afterwards.  RVEs whose slip
+ * table is the {111}<110> family refresh the Jacobian in every step whatever
+ * the switch says: their correction is solved on the FP32 pipe, and a chord
+ * step would save nothing. */
 int voce_set_newton_chord(int on);
 /* Start of the VOCE_PREC_MIXED_IR Newton (no counterpart in the reference):
  * before its FP64-residual iterations, each voxel's stress is moved from the

@@ -204,10 +204,7 @@ __device__ __forceinline__ void fcc_pow(const T (&r)[N], int e, T (&p)[N])
 
 // One family of the flow rule (constitutive.c:126-194) in FP64, without
 // gam0: g = |r|^n sign(r), and with JAC the tangent's h = |r|^(n-1)/tau
-// (times gam0 n it is d gdot / d rss).  The FP64 Newton goes family by family:
-// it is bound by the FP64 pipe, and four systems at a time leave its
-// registers to the matrix (twelve at a time spilled: 528 us at 64^3 against
-// 495 us).
+// (times gam0 n it is d gdot / d rss).
 template <int Z, bool JAC>
 __device__ __forceinline__ void fcc_flow_family(const RveDesc &d, long long v, const double (&y)[5],
                                                 double (&E)[5], double (&J)[15])
@@ -322,6 +319,43 @@ __device__ __forceinline__ double reread(const double *a)
 __device__ __forceinline__ int itau_col(const RveDesc &d, int k, int f)
 {
     return d.fcc ? 2 * d.canon[k] + (f ^ d.flip[k]) : 2 * k + f;
+}
+
+// ---------------------------------------------------------------------------
+// Conversions between double and float with integer operations, which keeps
+// them off the FP64 pipe (a hardware conversion holds it as long as an FP64
+// product).  d2f truncates; values below the smallest normal float become
+// zero, and the caller keeps |x| < 2^127 (finite).  f2d is exact for normal
+// floats and zero; subnormal floats become zero, infinities and NaN are the
+// caller's to exclude.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float d2f(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    // exponent bias 1023 -> 127: the low eight exponent bits with the top one
+    // of them flipped
+    const unsigned m = ((__funnelshift_l(lo, hi, 3) & 0x7fffffffu) ^ 0x40000000u) | (hi & 0x80000000u);
+    return __uint_as_float((hi & 0x7fffffffu) < 0x38100000u ? 0u : m);
+}
+
+__device__ __forceinline__ double f2d(float f)
+{
+    const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+    const unsigned hi = ((a >> 3) + 0x38000000u) | (u & 0x80000000u);
+    return __hiloint2double(a < 0x00800000u ? 0 : (int)hi, a < 0x00800000u ? 0 : (int)(u << 29));
+}
+
+// x = h + l to about 2^-47: h = d2f(x), l from the 29 significand bits below h
+__device__ __forceinline__ ff32 d2ff(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    ff32 r;
+    r.h = d2f(x);
+    // 2^(exponent of x - 52) as a float, zero where that is below the floats
+    const int e = (int)((hi >> 20) & 0x7ffu) - (1023 - 127) - 52;
+    const float s = __uint_as_float((e > 0 ? (unsigned)e << 23 : 0u) | (hi & 0x80000000u));
+    r.l = (float)(lo & 0x1fffffffu) * s;
+    return r;
 }
 
 // ---------------------------------------------------------------------------
@@ -526,9 +560,7 @@ __device__ __forceinline__ bool fcc_step_ff(const RveDesc &d, long long v, const
     if (!fcc_flow_ff(d, v, y, E)) return false;
 #pragma unroll
     for (int i = 0; i < 5; ++i) {
-        ff32 c;
-        c.h = (float)cc[i];
-        c.l = (float)(cc[i] - (double)c.h);
+        const ff32 c = d2ff(cc[i]);
         t[i] = ffs_add(c, ff_mul(ff_norm(E[i].h, E[i].l), dtgh, dtgl));
     }
 #pragma unroll
@@ -543,4 +575,161 @@ __device__ __forceinline__ bool fcc_step_ff(const RveDesc &d, long long v, const
     for (int i = 0; i < 5; ++i) x[i] = t[i].h + t[i].l;
     fcc_solve<float>(L, x);
     return true;
+}
+
+// ---------------------------------------------------------------------------
+// The correction of the FP64 Newton step, M dy = x with the exact tangent, in
+// float pairs: about 47 bits.  A correction wrong by 1e-13 of itself moves the
+// next iterate by 1e-13 of a step that is itself a small part of the stress,
+// which is below the rounding of the FP64 residual that the next iterate is
+// measured by; the residual, the flow rule, the stop test and the iterate stay
+// FP64.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ ff32 ffs_norm(ff32 a) { return ff_norm(a.h, a.l); }
+__device__ __forceinline__ ff32 ffs_mul(ff32 a, ff32 b) { return ff_mul(a, b.h, b.l); }
+
+// 1 / a: the hardware's approximate reciprocal and one Newton-Raphson step
+__device__ __forceinline__ ff32 ff_rcp(ff32 a)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a.h));
+    const float e = fmaf(-a.l, r, fmaf(-a.h, r, 1.0f));
+    return ff_norm(r, r * e);
+}
+
+// the tangent of family Z from its four h (see fcc_tangent)
+template <int Z>
+__device__ __forceinline__ void fcc_tangent_ff(const ff32 (&h)[4], ff32 (&J)[15])
+{
+    const ff32 pu = ffs_add(h[0], h[1]), pw = ffs_add(h[2], h[3]);
+    const ff32 mu = ffs_sub(h[0], h[1]), mw = ffs_sub(h[2], h[3]);
+    const ff32 s = ffs_add(pu, pw), dl = ffs_sub(pu, pw), a = ffs_add(mu, mw), b = ffs_sub(mu, mw);
+    auto twice = [](ff32 x) { x.h *= 2.0f; x.l *= 2.0f; return x; };
+    auto add = [&](int i, int j, ff32 x) { J[sym5(i, j)] = ffs_add(J[sym5(i, j)], x); };
+    auto sub = [&](int i, int j, ff32 x) { J[sym5(i, j)] = ffs_sub(J[sym5(i, j)], x); };
+    if (Z == 0) {
+        add(0, 0, s);
+        sub(0, 1, s);
+        add(1, 1, s);
+        add(3, 3, s);
+        add(4, 4, s);
+        add(0, 4, a);
+        sub(1, 4, a);
+        add(0, 3, b);
+        sub(1, 3, b);
+        add(3, 4, dl);
+    } else if (Z == 1) {
+        add(0, 0, s);
+        add(0, 1, s);
+        add(1, 1, s);
+        add(4, 4, s);
+        add(2, 2, s);
+        sub(0, 4, a);
+        sub(1, 4, a);
+        sub(0, 2, b);
+        sub(1, 2, b);
+        add(2, 4, dl);
+    } else {
+        add(0, 0, twice(twice(s)));
+        add(3, 3, s);
+        add(2, 2, s);
+        sub(0, 3, twice(a));
+        sub(0, 2, twice(b));
+        add(2, 3, dl);
+    }
+}
+
+// h = dtgn |r|^(n-1) / tau of family Z at y (float pairs), into the tangent
+template <int Z>
+__device__ __forceinline__ void fcc_jac_family_ff(const RveDesc &d, long long v, const ff32 (&y)[5], ff32 dtgn,
+                                                  ff32 (&J)[15])
+{
+    const ff32 D = Z == 0 ? ffs_sub(y[0], y[1]) : Z == 1 ? ffs_neg(ffs_add(y[0], y[1])) : ffs_add(ffs_neg(y[0]), ffs_neg(y[0]));
+    const ff32 a = Z == 2 ? y[3] : y[4], b = Z == 0 ? y[3] : y[2];
+    const ff32 u = ffs_add(a, b), w = ffs_sub(a, b);
+    ff32 r[4] = {ffs_add(D, u), ffs_sub(D, u), ffs_add(D, w), ffs_sub(D, w)}, h[4];
+    const int e = d.ipow_n - 1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int neg = r[k].h < 0.0f;
+        const ff32 it = d2ff(__ldg(d.itau + (long long)(2 * (4 * Z + k) + neg) * d.nv + v));
+        r[k] = ffs_mul(ffs_norm(r[k]), it);
+        if (neg) r[k] = ffs_neg(r[k]);
+        h[k] = ffs_mul(it, dtgn);
+    }
+    if (e == 19) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const ff32 a2 = ffs_mul(r[k], r[k]), a4 = ffs_mul(a2, a2), a8 = ffs_mul(a4, a4), a16 = ffs_mul(a8, a8);
+            h[k] = ffs_mul(ffs_mul(ffs_mul(a16, a2), r[k]), h[k]);
+        }
+    } else {
+        for (int q = e; q; q >>= 1) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (q & 1) h[k] = ffs_mul(h[k], r[k]);
+                r[k] = ffs_mul(r[k], r[k]);
+            }
+        }
+    }
+    fcc_tangent_ff<Z>(h, J);
+}
+
+// x := M^-1 x at the stress y.  False when a value left the float range (the
+// caller then takes the FP64 solve).
+__device__ __forceinline__ bool fcc_solve_ff(const RveDesc &d, long long v, const double (&yd)[5], double (&xd)[5],
+                                             ff32 dtgn)
+{
+    ff32 M[15];
+    {
+        ff32 y[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) y[c] = d2ff(yd[c]);
+#pragma unroll
+        for (int q = 0; q < 15; ++q) M[q] = d2ff(__ldg(d.sch + (FCC_P + q) * d.nv + v));
+        fcc_jac_family_ff<0>(d, v, y, dtgn, M);
+        fcc_jac_family_ff<1>(d, v, y, dtgn, M);
+        fcc_jac_family_ff<2>(d, v, y, dtgn, M);
+    }
+    auto fms = [](ff32 &acc, ff32 a, ff32 b) { ff_acc2(acc, -a.h, -a.l, b.h, b.l); };
+    // LDL^T in place, as fcc_factor
+#pragma unroll
+    for (int j = 0; j < 5; ++j) {
+        const ff32 di = ff_rcp(ffs_norm(M[sym5(j, j)]));
+        ff32 w[5];
+#pragma unroll
+        for (int i = j + 1; i < 5; ++i) {
+            w[i] = ffs_norm(M[sym5(j, i)]);
+            M[sym5(j, i)] = ffs_mul(w[i], di);
+        }
+#pragma unroll
+        for (int i = j + 1; i < 5; ++i)
+#pragma unroll
+            for (int k = i; k < 5; ++k) fms(M[sym5(i, k)], M[sym5(j, i)], w[k]);
+        M[sym5(j, j)] = di;
+    }
+    ff32 b[5];
+#pragma unroll
+    for (int c = 0; c < 5; ++c) b[c] = d2ff(xd[c]);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+#pragma unroll
+        for (int k = 0; k < i; ++k) fms(b[i], M[sym5(k, i)], b[k]);
+        b[i] = ffs_norm(b[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 5; ++i) b[i] = ffs_mul(b[i], M[sym5(i, i)]);
+#pragma unroll
+    for (int i = 3; i >= 0; --i) {
+#pragma unroll
+        for (int k = i + 1; k < 5; ++k) fms(b[i], M[sym5(i, k)], b[k]);
+        b[i] = ffs_norm(b[i]);
+    }
+    bool ok = true;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) {
+        ok = ok && fabsf(b[c].h) < 1e30f;
+        xd[c] = f2d(b[c].h) + f2d(b[c].l);
+    }
+    return ok;
 }

@@ -1685,30 +1685,32 @@ __device__ void nr_unit(const RveDesc &d, int unit, int nunits)
 // UpdateStress (evolution.c:3-168) for an RVE of the {111}<110> family in
 // crystal axes (voce_fcc.cuh), one kernel instance per form.
 //
-// FCC_FP64, FCC_CHORD (the FP64 form; VOCE_PREC_MIXED, which may take chord
-// steps as in newton_fp64): the Newton iteration of newton_fp64 -- the exact
-// Jacobian, the stop test of evolution.c:112, the strain rate and the norms at
-// the stress before the last update -- in the variables y, so its iterates
-// agree to rounding.  Bound: the FP64 pipe (64 cycles of an SM quarter's pipe
-// per warp instruction).  A Newton iteration takes about 335 FP64 operations
-// instead of about 680 in sample axes: 26 instead of 60 for the resolved
-// shears, 32 instead of 60 for the strain rate, 40 + 15 instead of 240 + 15
-// for the tangent, 85 instead of 125 for the 5x5 solve (the pressure
-// decouples).  Measured per launch against kb_nr (FP64 form, first
-// increment): 64^3 879 -> 477 us, 128^3 10.4 -> 5.6 ms, 16^3 (a grain per
-// voxel) 86 -> 50 us.
+// FCC_FP64 (the FP64 form and VOCE_PREC_MIXED): the Newton iteration of
+// newton_fp64 -- the exact Jacobian, the stop test of evolution.c:112, the
+// strain rate and the norms at the stress before the last update -- in the
+// variables y, so its iterates agree to rounding.  Bound: the FP64 pipe (64
+// cycles of an SM quarter's pipe per warp instruction).  A Newton iteration
+// takes about 170 FP64 operations instead of about 680 in sample axes: 21
+// instead of 60 for the resolved shears, 27 instead of 60 for the strain rate,
+// 72 for the powers, 25 for P y (the pressure decouples); the tangent and the
+// 5x5 solve, 240 + 125 there, run in float pairs on the FP32 pipe beside it.
+// Measured per launch against kb_nr (FP64 form, first increment): 64^3 879 ->
+// 358 us (477 with the solve in FP64), 16^3 (a grain per voxel) 86 -> 48 us.
+// With the solve off the FP64 pipe a chord step saves nothing, so d.chord is
+// not looked at here.
 //
 // FCC_IR (VOCE_PREC_MIXED_IR): newton_ir in the same variables: the start in
 // single precision and float pairs, then steps whose residual, flow rule and
 // stop test are FP64 and whose correction is solved in FP32 with the start's
-// last matrix; 64^3 363 -> 240 us, 256^3 29.9 -> 16.4 ms.  FCC_NR32
-// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 331 us.  Nothing is staged
-// in shared memory any more: the single-precision steps read 15 + 12 floats
-// per voxel instead of 21 + 72.
+// last matrix; 64^3 363 -> 221 us, 256^3 29.9 -> 15.6 ms.  FCC_NR32
+// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 309 us.  Nothing is staged
+// in shared memory: the single-precision steps read 15 + 12 floats per voxel
+// instead of 21 + 72.  Conversions go through the integer pipe (d2f, f2d:
+// with the hardware's, 239 and 342 us).
 //
 // kb_nr stays for every other slip table and for non-integral exponents.
 // ---------------------------------------------------------------------------
-enum { FCC_FP64 = 0, FCC_CHORD = 1, FCC_IR = 2, FCC_NR32 = 3 };
+enum { FCC_FP64 = 0, FCC_IR = 1, FCC_NR32 = 2 };
 
 // x += P y with P_y of voxel v in FP64
 __device__ __forceinline__ void fcc_add_Py(const double *fx, long long nv, const double (&y)[5], double (&x)[5])
@@ -1752,45 +1754,47 @@ __device__ __forceinline__ void fcc_rare_step(const RveDesc &d, long long v, con
 
 // The FP64 Newton steps with the exact Jacobian from y (s5 its pressure
 // part): y, s5 the new stress, yp, s5p the stress before the last update, Rl,
-// R5 the residual there
-template <bool CHORD>
+// R5 the residual there.  The correction is solved in float pairs on the FP32
+// pipe (fcc_solve_ff), except where a ratio |r| or the residual leaves the
+// float range.
 __device__ __forceinline__ void fcc_newton(const RveDesc &d, long long v, const double (&cc)[5], double cc5,
                                            double thr, double (&y)[5], double &s5, double (&yp)[5], double &s5p,
                                            double (&Rl)[5], double &R5, int &it)
 {
     const long long nv = d.nv;
     const double *fx = d.sch + v;
-    const double dtg = d.dt * d.gam0[0], dtgn = dtg * d.nrs[0];
-    bool go = true, fresh = true;
-    double L[15];
-    (void)fresh;
+    const double dtg = d.dt * d.gam0[0];
+    const ff32 dtgn = d2ff(dtg * d.nrs[0]);
+    bool go = true;
     while (go && it < 100) {
         ++it;
-        double E[5], x[5], J[15];
+        double E[5], x[5];
 #pragma unroll
         for (int c = 0; c < 5; ++c) yp[c] = y[c];
         s5p = s5;
-        if (!CHORD || fresh) fcc_flow<true>(d, v, y, E, J);
-        else fcc_flow<false>(d, v, y, E, J);
+        bool fp64 = fcc_edot_fp64(d, v, y, E) || d.ipow_n > 20;
 #pragma unroll
         for (int c = 0; c < 5; ++c) x[c] = fma(dtg, E[c], cc[c]);
         fcc_add_Py(fx, nv, y, x);
-        if (!CHORD || fresh) {
+        int top = 0;
 #pragma unroll
-            for (int q = 0; q < 15; ++q) L[q] = fma(dtgn, J[q], __ldg(fx + (FCC_P + q) * nv));
-            fcc_factor(L);
+        for (int c = 0; c < 5; ++c) {
+            Rl[c] = x[c];
+            top = max(top, __double2hiint(x[c]) & 0x7fffffff);
         }
-#pragma unroll
-        for (int c = 0; c < 5; ++c) Rl[c] = x[c];
         R5 = fma(d.P55, s5, cc5);
-        fcc_solve<double>(L, x);
         const double x5 = R5 * d.iP55;
+        fp64 = fp64 || top >= 0x46000000;   // |x| >= 2^97, or not finite
+        if (!fp64) fp64 = !fcc_solve_ff(d, v, y, x, dtgn);
+        if (fp64) {
+#pragma unroll
+            for (int c = 0; c < 5; ++c) x[c] = Rl[c];
+            fcc_rare_step(d, v, y, x);
+        }
 #pragma unroll
         for (int c = 0; c < 5; ++c) y[c] -= x[c];
         s5 -= x5;
-        const double cnr = fma(x5, x5, fcc_norm2<double>(x));
-        go = cnr > thr;
-        if (CHORD) fresh = !d.chord || cnr > 1e6 * thr;
+        go = fma(x5, x5, fcc_norm2<double>(x)) > thr;
     }
 }
 
@@ -1835,10 +1839,10 @@ __device__ __forceinline__ void fcc_newton_ir(const RveDesc &d, long long v, boo
             }
             if (!fp64) {
 #pragma unroll
-                for (int c = 0; c < 5; ++c) xf[c] = (float)(x[c]);
+                for (int c = 0; c < 5; ++c) xf[c] = d2f(x[c]);
                 fcc_solve<float>(L, xf);
 #pragma unroll
-                for (int c = 0; c < 5; ++c) x[c] = (double)(xf[c]);
+                for (int c = 0; c < 5; ++c) x[c] = f2d(xf[c]);
             }
         }
         if (fp64) fcc_rare_step(d, v, y, x);
@@ -1914,8 +1918,8 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
         int it = 0;
         bool converged = false;   // FCC_NR32: the start's point is taken as the solution
         (void)converged;
-        if constexpr (FORM == FCC_FP64 || FORM == FCC_CHORD) {
-            fcc_newton<FORM == FCC_CHORD>(d, v, cc, cc5, thr, y, s5, yp, s5p, Rl, R5, it);
+        if constexpr (FORM == FCC_FP64) {
+            fcc_newton(d, v, cc, cc5, thr, y, s5, yp, s5p, Rl, R5, it);
         } else {
             float yf[5], ccf[5], P[15], L[15], xf[5];
             bool ok = false;
@@ -1923,7 +1927,7 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
 #pragma unroll
                 for (int q = 0; q < 15; ++q) P[q] = __ldg(d.sgp32 + (long long)q * nv + v);
 #pragma unroll
-                for (int c = 0; c < 5; ++c) { yf[c] = (float)(yl[c]); ccf[c] = (float)(cc[c]); }
+                for (int c = 0; c < 5; ++c) { yf[c] = d2f(yl[c]); ccf[c] = d2f(cc[c]); }
                 // before a float-float step single precision stops at a
                 // relative update of 1e-4 (its rounding floor can lie near
                 // 1e-5), alone at 1e-5
@@ -1940,7 +1944,7 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
                     // the pressure component is linear: its root at once
                     s5 = -cc5 * d.iP55;
 #pragma unroll
-                    for (int c = 0; c < 5; ++c) y[c] = (double)(yf[c]) - (double)(xf[c]);
+                    for (int c = 0; c < 5; ++c) y[c] = f2d(yf[c]) - f2d(xf[c]);
                     if (FORM == FCC_NR32) converged = !polish || fcc_norm2<float>(xf) <= (float)(1e-10 * sn2);
                 }
             }
@@ -1954,7 +1958,7 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
                 for (int c = 0; c < 5; ++c) yp[c] = y[c];
                 s5p = s5;
             } else {
-                fcc_newton<false>(d, v, cc, cc5, thr, y, s5, yp, s5p, Rl, R5, it);
+                fcc_newton(d, v, cc, cc5, thr, y, s5, yp, s5p, Rl, R5, it);
             }
         }
         // |sig - lam| and the strain-compatibility norm |Rl - S0 (sp - lam)|
@@ -3083,10 +3087,7 @@ int nr_resident_blocks(int kind)
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr<false, false, true>, VOCE_NR_THREADS,
                                                           kNrStageBytes);
         } else if (kind == 3) {
-            int chord = 2;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr_fcc<FCC_FP64>, VOCE_NR_THREADS, 0);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&chord, kb_nr_fcc<FCC_CHORD>, VOCE_NR_THREADS, 0);
-            per = std::min(per, chord);
         } else if (kind == 4) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kb_nr_fcc<FCC_IR>, VOCE_NR_THREADS, 0);
         } else if (kind == 5) {
@@ -3142,7 +3143,6 @@ static void plan_iteration_t(const BatchPlan &bp, cudaStream_t s, Prof &pf, cuda
         const int g = grid_for(n, nr_resident_blocks(bp.nr32 ? 5 : bp.ir ? 4 : 3));
         if (bp.nr32) kb_nr_fcc<FCC_NR32><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
         else if (bp.ir) kb_nr_fcc<FCC_IR><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
-        else if (bp.mixed) kb_nr_fcc<FCC_CHORD><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
         else kb_nr_fcc<FCC_FP64><<<g, VOCE_NR_THREADS, 0, s>>>(D, bp.map[BP_NF], n);
         ++launched;
     }
