@@ -24,6 +24,9 @@
 #include <string>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 using namespace voce;
 
 namespace {
@@ -305,6 +308,23 @@ int dalloc(voce_rve *r, T *&p, size_t count)
     r->dev_allocs.push_back(q);
     p = (T *)q;
     return VOCE_OK;
+}
+
+// Fault in the pages of a host buffer that a device-to-host copy is about to
+// fill.  The copy faults untouched pages one by one: a 25 MB field into fresh
+// memory took 24 ms, into mapped memory 0.5 ms, and with the pages mapped
+// first, 0.95 ms.  MADV_POPULATE_WRITE maps a whole range in one call and
+// leaves its contents alone; a kernel or a mapping that does not take it
+// (pinned memory) leaves everything as it was.
+void populate(void *p, size_t n)
+{
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+    if (n < 65536 || page == 0 || (page & (page - 1))) return;
+    const uintptr_t b = (uintptr_t)p & ~(page - 1), e = ((uintptr_t)p + n + page - 1) & ~(page - 1);
+    madvise((void *)b, e - b, MADV_POPULATE_WRITE);
 }
 
 // exp(-2 pi i j / L) for j < L; where the length has a register-FFT split
@@ -1508,6 +1528,7 @@ int voce_rve_get_field(voce_rve *r, int field, double *host_out)
     } else {
         CUDA_TRY(launch_field_out(r->d, field, r->d_out, r->stream));
     }
+    populate(host_out, sizeof(double) * per * (size_t)r->d.nv);   // (while the kernel runs)
     CUDA_TRY(cudaMemcpyAsync(host_out, r->d_out, sizeof(double) * per * r->d.nv, cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     return VOCE_OK;
@@ -1563,6 +1584,7 @@ int noalloc_download(voce_rve *r, int field, long long n, int dev, double *host_
     // the array has to start at zero; what lies past n keeps an earlier call's
     // values and is never read.
     CUDA_TRY(launch_field_out(r->d, field, stage, r->stream));
+    populate(host_out, sizeof(double) * (size_t)n);
     CUDA_TRY(cudaMemcpyAsync(host_out, stage, sizeof(double) * n, cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     return VOCE_OK;
@@ -1792,6 +1814,7 @@ int voce_rve_snapshot(voce_rve *r, void *buf, long long size)
     if (rc) return rc;
     const long long need = snapshot_write(r, nullptr);
     if (size < need) return fail(VOCE_ERR_ARG, "snapshot buffer of %lld bytes, %lld needed", size, need);
+    populate(buf, (size_t)need);
     const long long n = snapshot_write(r, static_cast<char *>(buf));
     return n < 0 ? (int)-n : VOCE_OK;
 }
