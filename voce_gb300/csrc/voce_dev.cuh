@@ -47,9 +47,9 @@ constexpr int kSysUnroll = VOCE_SYS_UNROLL;
 #define VOCE_PI_REF 3.14159265359
 #define VOCE_TWO_PI_REF 6.28318530718
 
-// One axis's transform: Stockham radix stages rad[0..nst) (n1 = 0), or, in
-// the single-precision spectrum only, the two-pass register FFT of
-// L = n1 x (L / n1) (n1 > 0; rad then keeps the default Stockham stages).
+// One axis's transform: Stockham radix stages rad[0..nst) (n1 = 0), or the
+// two-pass register FFT of L = n1 x (L / n1) (n1 > 0; rad then keeps the
+// default Stockham stages).
 struct FftPlan1 {
     int L, nst;
     int rad[VOCE_MAXRAD];
@@ -658,11 +658,6 @@ __device__ __forceinline__ void unit_freq(const RveDesc &d, int ix, int iy, int 
     n[0] = g0 * s; n[1] = g1 * s; n[2] = g2 * s;
 }
 
-// Arithmetic type of the Green operator: double in the FP64 form, float with
-// the single-precision spectrum (the mixed forms).
-template <typename R> struct GreenT { typedef double T; };
-template <> struct GreenT<float> { typedef float T; };
-
 __device__ __forceinline__ double green_rcp(double x) { return rcp_nr(x); }
 __device__ __forceinline__ float green_rcp(float x) { return __frcp_rn(x); }
 
@@ -694,46 +689,44 @@ __device__ __forceinline__ void green_omega(const G *Kq, const G *nd, G (&w)[6])
     w[3] = c11 * id; w[4] = c12 * id; w[5] = c22 * id;
 }
 
-// dU -= wgt (omega sig^ n) (x) n, symmetric and antisymmetric parts
-template <typename R, typename G>
-__device__ __forceinline__ void green_update(const G (&w)[6], const G *nd,
-                                             const R (&sr)[6], const R (&si)[6],
-                                             R (&ur)[6], R (&ui)[6], R (&ar)[3], R (&ai)[3],
-                                             R wgt)
+// One real part of dU += -wgt (omega sig^ n) (x) n, in the 6-vector basis
+// throughout: b in the basis -> u (its symmetric part, basis) and a (its
+// antisymmetric part: 12, 02, 01).  The basis factors ride on m = n / sqrt 2,
+// so no conversion to the tensor and back is made: 47 operations instead of
+// 72 (the pass is bound by the FP64 pipe in the FP64 form).
+template <typename R>
+__device__ __forceinline__ void green_part(const R (&w)[6], const R (&n)[3], const R (&m)[3], R wgt, const R (&b)[6],
+                                           R (&u)[6], R (&a)[3])
 {
-    R w00 = R(w[0]), w01 = R(w[1]), w02 = R(w[2]);
-    R w11 = R(w[3]), w12 = R(w[4]), w22 = R(w[5]);
-    R n0 = R(nd[0]), n1 = R(nd[1]), n2 = R(nd[2]);
-    // t = sig^ n (sig^ symmetric: 00,11,22,12,02,01)
-    R t0r = sr[0] * n0 + sr[5] * n1 + sr[4] * n2, t0i = si[0] * n0 + si[5] * n1 + si[4] * n2;
-    R t1r = sr[5] * n0 + sr[1] * n1 + sr[3] * n2, t1i = si[5] * n0 + si[1] * n1 + si[3] * n2;
-    R t2r = sr[4] * n0 + sr[3] * n1 + sr[2] * n2, t2i = si[4] * n0 + si[3] * n1 + si[2] * n2;
-    R v0r = w00 * t0r + w01 * t1r + w02 * t2r, v0i = w00 * t0i + w01 * t1i + w02 * t2i;
-    R v1r = w01 * t0r + w11 * t1r + w12 * t2r, v1i = w01 * t0i + w11 * t1i + w12 * t2i;
-    R v2r = w02 * t0r + w12 * t1r + w22 * t2r, v2i = w02 * t0i + w12 * t1i + w22 * t2i;
-    // dU = -v (x) n ; weight wgt (1 or 1/2 on the Nyquist planes)
-    R h = -wgt;
-    R hh = R(0.5) * h;
-    ur[0] += h * v0r * n0;                 ui[0] += h * v0i * n0;
-    ur[1] += h * v1r * n1;                 ui[1] += h * v1i * n1;
-    ur[2] += h * v2r * n2;                 ui[2] += h * v2i * n2;
-    ur[3] += hh * (v1r * n2 + v2r * n1);   ui[3] += hh * (v1i * n2 + v2i * n1);
-    ur[4] += hh * (v0r * n2 + v2r * n0);   ui[4] += hh * (v0i * n2 + v2i * n0);
-    ur[5] += hh * (v0r * n1 + v1r * n0);   ui[5] += hh * (v0i * n1 + v1i * n0);
-    ar[0] += hh * (v1r * n2 - v2r * n1);   ai[0] += hh * (v1i * n2 - v2i * n1);
-    ar[1] += hh * (v0r * n2 - v2r * n0);   ai[1] += hh * (v0i * n2 - v2i * n0);
-    ar[2] += hh * (v0r * n1 - v1r * n0);   ai[2] += hh * (v0i * n1 - v1i * n0);
+    const R c5 = R(RSQ3) * b[5], c1 = R(RSQ6) * b[1], p = c5 - c1;
+    const R s00 = p - R(RSQ2) * b[0], s11 = p + R(RSQ2) * b[0], s22 = c5 + R(2) * c1;
+    const R t0 = s00 * n[0] + b[4] * m[1] + b[3] * m[2];
+    const R t1 = s11 * n[1] + b[4] * m[0] + b[2] * m[2];
+    const R t2 = s22 * n[2] + b[3] * m[0] + b[2] * m[1];
+    // v = wgt omega t; dU = -v (x) n
+    const R v0 = wgt * (w[0] * t0 + w[1] * t1 + w[2] * t2);
+    const R v1 = wgt * (w[1] * t0 + w[3] * t1 + w[4] * t2);
+    const R v2 = wgt * (w[2] * t0 + w[4] * t1 + w[5] * t2);
+    const R q0 = v0 * n[0], q1 = v1 * n[1], q2 = v2 * n[2], q01 = q0 + q1;
+    u[0] += v0 * m[0] - v1 * m[1];
+    u[1] += R(RSQ6) * (q01 - R(2) * q2);
+    u[2] -= v1 * m[2] + v2 * m[1];
+    u[3] -= v0 * m[2] + v2 * m[0];
+    u[4] -= v0 * m[1] + v1 * m[0];
+    u[5] -= R(RSQ3) * (q01 + q2);
+    const R h0 = R(0.5) * n[0], h1 = R(0.5) * n[1], h2 = R(0.5) * n[2];
+    a[0] -= v1 * h2 - v2 * h1;
+    a[1] -= v0 * h2 - v2 * h0;
+    a[2] -= v0 * h1 - v1 * h0;
 }
 
-template <typename R, typename G>
-__device__ __forceinline__ void green_rank1(const G *Kq, const G *nd,
-                                            const R (&sr)[6], const R (&si)[6],
-                                            R (&ur)[6], R (&ui)[6], R (&ar)[3], R (&ai)[3],
-                                            R wgt)
+template <typename R>
+__device__ __forceinline__ void green_update(const R (&w)[6], const R (&n)[3], R wgt, const R (&br)[6], const R (&bi)[6],
+                                             R (&ur)[6], R (&ui)[6], R (&ar)[3], R (&ai)[3])
 {
-    G w[6];
-    green_omega<G>(Kq, nd, w);
-    green_update<R, G>(w, nd, sr, si, ur, ui, ar, ai, wgt);
+    const R m[3] = {R(RSQ2) * n[0], R(RSQ2) * n[1], R(RSQ2) * n[2]};
+    green_part<R>(w, n, m, wgt, br, ur, ar);
+    green_part<R>(w, n, m, wgt, bi, ui, ai);
 }
 
 __device__ __forceinline__ const double *green_kq(const RveDesc &d, double *) { return d.Kq; }
@@ -747,41 +740,39 @@ template <typename R>
 __device__ __forceinline__ void green_apply(const RveDesc &d, int ix, int iy, int iz, long long o,
                                             R (&br)[6], R (&bi)[6], R (&ar)[3], R (&ai)[3])
 {
-    R sr[6], si[6], ur[6], ui[6];
-    b_to_t6<R>(br, sr);
-    b_to_t6<R>(bi, si);
+    R ur[6], ui[6];
 #pragma unroll
     for (int a = 0; a < 6; ++a) { ur[a] = R(0); ui[a] = R(0); }
 #pragma unroll
     for (int a = 0; a < 3; ++a) { ar[a] = R(0); ai[a] = R(0); }
     if ((ix | iy | iz) != 0) {
-        typedef typename GreenT<R>::T G;
-        const G *kq = green_kq(d, (G *)nullptr);
-        G n[3], w[6];
-        if (sizeof(G) == 8 && d.gstore) {
+        R n[3], w[6];
+        if (sizeof(R) == 8 && d.gstore) {
             const double *gs = d.gstore + o;
             const long long ns = d.nspec;
 #pragma unroll
-            for (int q = 0; q < 3; ++q) n[q] = (G)__ldg(gs + q * ns);
+            for (int q = 0; q < 3; ++q) n[q] = (R)__ldg(gs + q * ns);
 #pragma unroll
-            for (int q = 0; q < 6; ++q) w[q] = (G)__ldg(gs + (3 + q) * ns);
+            for (int q = 0; q < 6; ++q) w[q] = (R)__ldg(gs + (3 + q) * ns);
         } else {
             unit_freq(d, ix, iy, iz, n);
-            green_omega<G>(kq, n, w);
+            green_omega<R>(green_kq(d, (R *)nullptr), n, w);
         }
-        bool nyq = ((d.nx % 2 == 0) && ix == d.nx / 2) || ((d.ny % 2 == 0) && iy == d.ny / 2) ||
-                   ((d.nz % 2 == 0) && iz == d.nz / 2);
-        if (!nyq) {
-            green_update<R, G>(w, n, sr, si, ur, ui, ar, ai, R(1));
-        } else {
-            G n2[3];
-            unit_freq(d, (d.nx - ix) % d.nx, (d.ny - iy) % d.ny, (d.nz - iz) % d.nz, n2);
-            green_update<R, G>(w, n, sr, si, ur, ui, ar, ai, R(0.5));
-            green_rank1<R, G>(kq, n2, sr, si, ur, ui, ar, ai, R(0.5));
+        const bool nx2 = 2 * ix == d.nx, ny2 = 2 * iy == d.ny, nz2 = 2 * iz == d.nz;
+        const bool nyq = nx2 || ny2 || nz2;
+        green_update<R>(w, n, nyq ? R(0.5) : R(1), br, bi, ur, ui, ar, ai);
+        if (nyq) {
+            // n(-k) is -n(k) but for the Nyquist components, which the
+            // reference leaves at -pi: up to its sign, n with those reversed
+            if (nx2) n[0] = -n[0];
+            if (ny2) n[1] = -n[1];
+            if (nz2) n[2] = -n[2];
+            green_omega<R>(green_kq(d, (R *)nullptr), n, w);
+            green_update<R>(w, n, R(0.5), br, bi, ur, ui, ar, ai);
         }
     }
-    t6_to_b<R>(ur, br);
-    t6_to_b<R>(ui, bi);
+#pragma unroll
+    for (int a = 0; a < 6; ++a) { br[a] = ur[a]; bi[a] = ui[a]; }
 }
 
 // ---------------------------------------------------------------------------
@@ -803,7 +794,7 @@ __device__ __forceinline__ typename Cx<R>::T cmul(typename Cx<R>::T a, typename 
 }
 
 // ---------------------------------------------------------------------------
-// Register FFT of the single-precision spectrum.  A line of length
+// Register FFT.  A line of length
 // L = N1 N2 runs as two passes of small DFTs held in registers (the
 // four-step Cooley-Tukey split).  Pass 1: for each t < N2, the N1 elements
 // t + N2 j are transformed over j and output k1 is multiplied by W_L^(t k1),
@@ -858,25 +849,38 @@ __device__ __forceinline__ void sfor(F &&f)
     }
 }
 
-// v W_N^E, W_N = exp(S 2 pi i / N)
-template <int N, int E, int S>
-__device__ __forceinline__ float2 rot(float2 v)
+template <typename C> struct RealOf;
+template <> struct RealOf<float2> { typedef float T; };
+template <> struct RealOf<double2> { typedef double T; };
+template <typename C>
+__device__ __forceinline__ C mkc(typename RealOf<C>::T x, typename RealOf<C>::T y)
 {
+    C c;
+    c.x = x;
+    c.y = y;
+    return c;
+}
+
+// v W_N^E, W_N = exp(S 2 pi i / N)
+template <int N, int E, int S, typename C>
+__device__ __forceinline__ C rot(C v)
+{
+    typedef typename RealOf<C>::T R;
     static_assert(48 % N == 0, "small DFT lengths divide 48");
     constexpr int a = (48 / N * E) % 48;
     static_assert(a % 3 == 0 || a % 4 == 0, "angle without a constant");
     if constexpr (a == 0) {
         return v;
     } else if constexpr (a == 24) {
-        return make_float2(-v.x, -v.y);
+        return mkc<C>(-v.x, -v.y);
     } else if constexpr (a == 12 || a == 36) {
         // W = g i, g = +-1
         constexpr int g = (a == 12 ? 1 : -1) * S;
-        if constexpr (g > 0) return make_float2(-v.y, v.x);
-        else return make_float2(v.y, -v.x);
+        if constexpr (g > 0) return mkc<C>(-v.y, v.x);
+        else return mkc<C>(v.y, -v.x);
     } else {
-        constexpr float c = (float)cos48(a), s = (float)(S * sin48(a));
-        return make_float2(c * v.x - s * v.y, c * v.y + s * v.x);
+        constexpr R c = (R)cos48(a), s = (R)(S * sin48(a));
+        return mkc<C>(c * v.x - s * v.y, c * v.y + s * v.x);
     }
 }
 
@@ -895,36 +899,37 @@ __host__ __device__ constexpr int dft_pos(int N, int q)
 // X[q] = sum_n x[n] exp(S 2 pi i n q / N) over the view, X[q] left in view
 // element dft_pos(N, q); N = A B composes radix 2, 3 and 4: A-point DFTs
 // over n = t + B j for each t, twiddles W_N^(t k), B-point DFTs over t
-template <int N, int S, int O, int T, int M>
-__device__ __forceinline__ void sdft(float2 (&x)[M])
+template <int N, int S, int O, int T, int M, typename C>
+__device__ __forceinline__ void sdft(C (&x)[M])
 {
+    typedef typename RealOf<C>::T R;
     if constexpr (N == 2) {
-        const float2 a = x[O], b = x[O + T];
-        x[O] = make_float2(a.x + b.x, a.y + b.y);
-        x[O + T] = make_float2(a.x - b.x, a.y - b.y);
+        const C a = x[O], b = x[O + T];
+        x[O] = mkc<C>(a.x + b.x, a.y + b.y);
+        x[O + T] = mkc<C>(a.x - b.x, a.y - b.y);
     } else if constexpr (N == 3) {
-        constexpr float s3 = (float)(S * 0.86602540378443864676);
-        const float2 x0 = x[O], x1 = x[O + T], x2 = x[O + 2 * T];
-        const float2 u = make_float2(x1.x + x2.x, x1.y + x2.y);
-        const float2 w = make_float2(x1.x - x2.x, x1.y - x2.y);
-        const float2 m = make_float2(x0.x - 0.5f * u.x, x0.y - 0.5f * u.y);
-        x[O] = make_float2(x0.x + u.x, x0.y + u.y);
-        x[O + T] = make_float2(m.x - s3 * w.y, m.y + s3 * w.x);
-        x[O + 2 * T] = make_float2(m.x + s3 * w.y, m.y - s3 * w.x);
+        constexpr R s3 = (R)(S * 0.86602540378443864676);
+        const C x0 = x[O], x1 = x[O + T], x2 = x[O + 2 * T];
+        const C u = mkc<C>(x1.x + x2.x, x1.y + x2.y);
+        const C w = mkc<C>(x1.x - x2.x, x1.y - x2.y);
+        const C m = mkc<C>(x0.x - R(0.5) * u.x, x0.y - R(0.5) * u.y);
+        x[O] = mkc<C>(x0.x + u.x, x0.y + u.y);
+        x[O + T] = mkc<C>(m.x - s3 * w.y, m.y + s3 * w.x);
+        x[O + 2 * T] = mkc<C>(m.x + s3 * w.y, m.y - s3 * w.x);
     } else if constexpr (N == 4) {
-        const float2 x0 = x[O], x1 = x[O + T], x2 = x[O + 2 * T], x3 = x[O + 3 * T];
-        const float2 t0 = make_float2(x0.x + x2.x, x0.y + x2.y);
-        const float2 t1 = make_float2(x0.x - x2.x, x0.y - x2.y);
-        const float2 t2 = make_float2(x1.x + x3.x, x1.y + x3.y);
-        const float2 t3 = make_float2(x1.x - x3.x, x1.y - x3.y);
-        x[O] = make_float2(t0.x + t2.x, t0.y + t2.y);
-        x[O + 2 * T] = make_float2(t0.x - t2.x, t0.y - t2.y);
+        const C x0 = x[O], x1 = x[O + T], x2 = x[O + 2 * T], x3 = x[O + 3 * T];
+        const C t0 = mkc<C>(x0.x + x2.x, x0.y + x2.y);
+        const C t1 = mkc<C>(x0.x - x2.x, x0.y - x2.y);
+        const C t2 = mkc<C>(x1.x + x3.x, x1.y + x3.y);
+        const C t3 = mkc<C>(x1.x - x3.x, x1.y - x3.y);
+        x[O] = mkc<C>(t0.x + t2.x, t0.y + t2.y);
+        x[O + 2 * T] = mkc<C>(t0.x - t2.x, t0.y - t2.y);
         if constexpr (S < 0) {   // t1 -/+ i t3
-            x[O + T] = make_float2(t1.x + t3.y, t1.y - t3.x);
-            x[O + 3 * T] = make_float2(t1.x - t3.y, t1.y + t3.x);
+            x[O + T] = mkc<C>(t1.x + t3.y, t1.y - t3.x);
+            x[O + 3 * T] = mkc<C>(t1.x - t3.y, t1.y + t3.x);
         } else {
-            x[O + T] = make_float2(t1.x - t3.y, t1.y + t3.x);
-            x[O + 3 * T] = make_float2(t1.x + t3.y, t1.y - t3.x);
+            x[O + T] = mkc<C>(t1.x - t3.y, t1.y + t3.x);
+            x[O + 3 * T] = mkc<C>(t1.x + t3.y, t1.y - t3.x);
         }
     } else {
         constexpr int A = N % 4 == 0 ? 4 : 2, B = N / A;
@@ -945,27 +950,28 @@ __device__ __forceinline__ void sdft(float2 (&x)[M])
 // tw[L + k N2 + t] = exp(-2 pi i t k / L) (conjugated for S = +1).  Pass 1's tasks are
 // (l, t), pass 2's (l, k1), l fastest: consecutive threads read consecutive
 // words of shared memory.
-template <int N1, int N2, int S>
-__device__ float2 *fft_reg(float2 *a, float2 *b, int NL, int ldl, const float2 *__restrict__ tw)
+template <int N1, int N2, int S, typename C>
+__device__ C *fft_reg(C *a, C *b, int NL, int ldl, const C *__restrict__ tw)
 {
-    const int tid = threadIdx.x, nthr = blockDim.x;
+    const int nthr = blockDim.x;
     const int dl = nthr % NL, dq = nthr / NL;
     {
+        const int tid = threadIdx.x;
         const int st = N2 * ldl;
         int l = tid % NL, t = tid / NL;
         for (int task = tid; task < NL * N2; task += nthr) {
-            float2 *p = a + t * ldl + l;
-            float2 x[N1];
+            C *p = a + t * ldl + l;
+            C x[N1];
 #pragma unroll
             for (int j = 0; j < N1; ++j) x[j] = p[j * st];
             sdft<N1, S, 0, 1>(x);
             if (t != 0) {
-                const float2 *wm = tw + N1 * N2 + t;   // the pass-1 twiddle matrix
+                const C *wm = tw + N1 * N2 + t;   // the pass-1 twiddle matrix
                 sfor<1, N1>([&](auto kc) {
                     constexpr int k = decltype(kc)::v, r = dft_pos(N1, k);
-                    float2 w = __ldg(wm + k * N2);
+                    C w = __ldg(wm + k * N2);
                     if (S > 0) w.y = -w.y;
-                    x[r] = cmul<float>(x[r], w);
+                    x[r] = cmul<typename RealOf<C>::T>(x[r], w);
                 });
             }
             sfor<0, N1>([&](auto kc) { p[decltype(kc)::v * st] = x[dft_pos(N1, decltype(kc)::v)]; });
@@ -976,15 +982,16 @@ __device__ float2 *fft_reg(float2 *a, float2 *b, int NL, int ldl, const float2 *
     }
     __syncthreads();
     {
+        const int tid = threadIdx.x;
         const int sb = N1 * ldl;
         int l = tid % NL, k1 = tid / NL;
         for (int task = tid; task < NL * N1; task += nthr) {
-            const float2 *p = a + N2 * k1 * ldl + l;
-            float2 x[N2];
+            const C *p = a + N2 * k1 * ldl + l;
+            C x[N2];
 #pragma unroll
             for (int t = 0; t < N2; ++t) x[t] = p[t * ldl];
             sdft<N2, S, 0, 1>(x);
-            float2 *q = b + k1 * ldl + l;
+            C *q = b + k1 * ldl + l;
             sfor<0, N2>([&](auto kc) { q[decltype(kc)::v * sb] = x[dft_pos(N2, decltype(kc)::v)]; });
             l += dl;
             k1 += dq;
@@ -995,11 +1002,12 @@ __device__ float2 *fft_reg(float2 *a, float2 *b, int NL, int ldl, const float2 *
     return b;
 }
 
-__device__ __forceinline__ float2 *fft_reg_lines(float2 *a, float2 *b, int NL, int ldl, int L,
-                                                 const float2 *__restrict__ tw, int sign)
+template <typename C>
+__device__ __forceinline__ C *fft_reg_lines(C *a, C *b, int NL, int ldl, int L,
+                                                 const C *__restrict__ tw, int sign)
 {
 #define VOCE_REG_FFT(L_, N1_) \
-    case L_: return sign < 0 ? fft_reg<N1_, L_ / N1_, -1>(a, b, NL, ldl, tw) : fft_reg<N1_, L_ / N1_, 1>(a, b, NL, ldl, tw);
+    case L_: return sign < 0 ? fft_reg<N1_, L_ / N1_, -1, C>(a, b, NL, ldl, tw) : fft_reg<N1_, L_ / N1_, 1, C>(a, b, NL, ldl, tw);
     switch (L) {
     VOCE_REG_FFT(16, 4)
     VOCE_REG_FFT(24, 4)
@@ -1021,14 +1029,12 @@ __device__ typename Cx<R>::T *fft_lines(typename Cx<R>::T *a, typename Cx<R>::T 
                                         const typename Cx<R>::T *__restrict__ tw, int sign)
 {
     typedef typename Cx<R>::T C;
-    if constexpr (sizeof(R) == 4) {
-        // the plan's split always matches reg_fft_split (the host sets both);
-        // an unknown length falls through to the Stockham stages, which the
-        // plan also holds
-        if (pl.n1 && reg_fft_split(pl.L) == pl.n1) {
-            C *res = fft_reg_lines(a, b, NL, ldl, pl.L, tw, sign);
-            if (res) return res;
-        }
+    // the plan's split always matches reg_fft_split (the host sets both); an
+    // unknown length falls through to the Stockham stages, which the plan
+    // also holds
+    if (pl.n1 && reg_fft_split(pl.L) == pl.n1) {
+        C *res = fft_reg_lines<C>(a, b, NL, ldl, pl.L, tw, sign);
+        if (res) return res;
     }
     const int L = pl.L;
     const int tid = threadIdx.x, nthr = blockDim.x;

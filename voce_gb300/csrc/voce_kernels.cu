@@ -2649,11 +2649,24 @@ __device__ __forceinline__ bool unit_on(const RveDesc &d, int mask)
 // resident blocks per SM the single-precision z passes are compiled for
 // (256^3, mixed forms, us per launch: z forward / inverse 461 / 946 at 2,
 // 524 / 1239 at 3, 586 / 1319 at 4, 461 / 1098 at 1)
+// The FP64 passes run blocks of 128 threads, six per SM (five for the Green
+// pass): they are bound by the FP64 pipe, and a block that loads or stores
+// leaves it to the others.  64^3, us per launch of z forward / y / x + Green /
+// z inverse, with the register FFT: 256 threads, 2 blocks 56 / 41 / 149 / 67,
+// 3 blocks 52 / 41 / 146 / 60; 128 threads, 4 blocks 53 / 40 / 137 / 63, 5
+// blocks 47 / 38 / 131 / 57; 64 threads, 8 blocks 52 / 40 / 141 / 64.  The
+// Stockham stages, 256 threads: 53 / 51 / 157 / 66.
+template <typename R> struct FftThreads { static constexpr int v = 256; };
+template <> struct FftThreads<double> { static constexpr int v = 128; };
+constexpr int kFft64Blocks = 6, kFftXg64Blocks = 5;
+// most blocks of a pass's grid, per SM
+template <typename R> struct FftGrid { static constexpr int v = 4; };
+template <> struct FftGrid<double> { static constexpr int v = 2 * kFft64Blocks; };
 #ifndef VOCE_FFTZ32_BLOCKS
 #define VOCE_FFTZ32_BLOCKS 2
 #endif
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? VOCE_FFTZ32_BLOCKS : 1)
+__global__ void __launch_bounds__(FftThreads<R>::v, sizeof(R) == 4 ? VOCE_FFTZ32_BLOCKS : kFft64Blocks)
 kb_fft_z_fwd(const RveDesc *descs, const int2 *map, int total)
 {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
@@ -2773,7 +2786,7 @@ __device__ void fft_y_stream_f32(const RveDesc *descs, const int2 *map, int tota
 #define VOCE_FFTXG32_BLOCKS 2
 #endif
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? VOCE_FFTY32_BLOCKS : 1)
+__global__ void __launch_bounds__(FftThreads<R>::v, sizeof(R) == 4 ? VOCE_FFTY32_BLOCKS : kFft64Blocks)
 kb_fft_y(const RveDesc *descs, const int2 *map, int total, int which, int stream)
 {
     if constexpr (sizeof(R) == 4) {
@@ -2791,12 +2804,11 @@ kb_fft_y(const RveDesc *descs, const int2 *map, int total, int which, int stream
     }
 }
 
-// resident blocks per SM the Green pass is compiled for (registers): 3 with
-// the FP64 spectrum (measured faster despite some spilling), 2 with FP32
-// (256^3 FP32, us per launch: 641 at 2, 1095 at 3, 1227 at 4: the register
+// resident blocks per SM the Green pass is compiled for (registers) with the
+// FP32 spectrum (256^3, us per launch: 641 at 2, 1095 at 3, 1227 at 4: the register
 // FFT spills below 128 registers)
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 3 : VOCE_FFTXG32_BLOCKS)
+__global__ void __launch_bounds__(FftThreads<R>::v, sizeof(R) == 8 ? kFftXg64Blocks : VOCE_FFTXG32_BLOCKS)
 kb_fft_x_green(const RveDesc *descs, const int2 *map, int total)
 {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
@@ -2827,7 +2839,7 @@ kb_fft_x_green(const RveDesc *descs, const int2 *map, int total)
 }
 
 template <typename R>
-__global__ void __launch_bounds__(256) kb_fft_x_aacc(const RveDesc *descs, const int2 *map, int total)
+__global__ void __launch_bounds__(FftThreads<R>::v) kb_fft_x_aacc(const RveDesc *descs, const int2 *map, int total)
 {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int2 e = map[w];
@@ -2840,7 +2852,7 @@ __global__ void __launch_bounds__(256) kb_fft_x_aacc(const RveDesc *descs, const
 
 // mode 0: spectrum -> displacement gradient; 1: accumulator -> rotl
 template <typename R>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? VOCE_FFTZ32_BLOCKS : 1)
+__global__ void __launch_bounds__(FftThreads<R>::v, sizeof(R) == 4 ? VOCE_FFTZ32_BLOCKS : kFft64Blocks)
 kb_fft_z_inv(const RveDesc *descs, const int2 *map, int total, int mode)
 {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
@@ -3118,22 +3130,22 @@ template <typename R>
 static void plan_iteration_t(const BatchPlan &bp, cudaStream_t s, Prof &pf, cudaGraphConditionalHandle cond,
                              int use_cond)
 {
-    const int FG = 152 * 4;
+    const int FG = 152 * FftGrid<R>::v;
     const RveDesc *D = bp.descs;
     pf.begin(K_FFT_Z_FWD, s);
-    kb_fft_z_fwd<R><<<grid_for(bp.total[BP_ZF], FG), 256, bp.smem[BP_ZF], s>>>(D, bp.map[BP_ZF], bp.total[BP_ZF]);
+    kb_fft_z_fwd<R><<<grid_for(bp.total[BP_ZF], FG), FftThreads<R>::v, bp.smem[BP_ZF], s>>>(D, bp.map[BP_ZF], bp.total[BP_ZF]);
     pf.end(K_FFT_Z_FWD, s);
     pf.begin(K_FFT_Y_FWD, s);
-    kb_fft_y<R><<<grid_for(bp.total[BP_Y6], FG), 256, bp.smem[BP_Y6], s>>>(D, bp.map[BP_Y6], bp.total[BP_Y6], 0, bp.ystream);
+    kb_fft_y<R><<<grid_for(bp.total[BP_Y6], FG), FftThreads<R>::v, bp.smem[BP_Y6], s>>>(D, bp.map[BP_Y6], bp.total[BP_Y6], 0, bp.ystream);
     pf.end(K_FFT_Y_FWD, s);
     pf.begin(K_FFT_X_GREEN, s);
-    kb_fft_x_green<R><<<grid_for(bp.total[BP_XG], FG), 256, bp.smem[BP_XG], s>>>(D, bp.map[BP_XG], bp.total[BP_XG]);
+    kb_fft_x_green<R><<<grid_for(bp.total[BP_XG], FG), FftThreads<R>::v, bp.smem[BP_XG], s>>>(D, bp.map[BP_XG], bp.total[BP_XG]);
     pf.end(K_FFT_X_GREEN, s);
     pf.begin(K_FFT_Y_INV, s);
-    kb_fft_y<R><<<grid_for(bp.total[BP_Y6], FG), 256, bp.smem[BP_Y6], s>>>(D, bp.map[BP_Y6], bp.total[BP_Y6], 1, bp.ystream);
+    kb_fft_y<R><<<grid_for(bp.total[BP_Y6], FG), FftThreads<R>::v, bp.smem[BP_Y6], s>>>(D, bp.map[BP_Y6], bp.total[BP_Y6], 1, bp.ystream);
     pf.end(K_FFT_Y_INV, s);
     pf.begin(K_FFT_Z_INV, s);
-    kb_fft_z_inv<R><<<grid_for(bp.total[BP_ZI], FG), 256, bp.smem[BP_ZI], s>>>(D, bp.map[BP_ZI], bp.total[BP_ZI], 0);
+    kb_fft_z_inv<R><<<grid_for(bp.total[BP_ZI], FG), FftThreads<R>::v, bp.smem[BP_ZI], s>>>(D, bp.map[BP_ZI], bp.total[BP_ZI], 0);
     pf.end(K_FFT_Z_INV, s);
     // a plan's RVEs of the {111}<110> family and the others: one launch each,
     // where there are any
@@ -3164,12 +3176,12 @@ static void plan_iteration_t(const BatchPlan &bp, cudaStream_t s, Prof &pf, cuda
 template <typename R>
 static void plan_incr_end_t(const BatchPlan &bp, cudaStream_t s, Prof &pf)
 {
-    const int FG = 152 * 4, NG = 152 * 2;
+    const int FG = 152 * FftGrid<R>::v, NG = 152 * 2;
     const RveDesc *D = bp.descs;
     pf.begin(K_INC_FFT, s);
-    kb_fft_x_aacc<R><<<grid_for(bp.total[BP_X3], FG), 256, bp.smem[BP_X3], s>>>(D, bp.map[BP_X3], bp.total[BP_X3]);
-    kb_fft_y<R><<<grid_for(bp.total[BP_Y3], FG), 256, bp.smem[BP_Y3], s>>>(D, bp.map[BP_Y3], bp.total[BP_Y3], 2, bp.ystream);
-    kb_fft_z_inv<R><<<grid_for(bp.total[BP_Z3], FG), 256, bp.smem[BP_Z3], s>>>(D, bp.map[BP_Z3], bp.total[BP_Z3], 1);
+    kb_fft_x_aacc<R><<<grid_for(bp.total[BP_X3], FG), FftThreads<R>::v, bp.smem[BP_X3], s>>>(D, bp.map[BP_X3], bp.total[BP_X3]);
+    kb_fft_y<R><<<grid_for(bp.total[BP_Y3], FG), FftThreads<R>::v, bp.smem[BP_Y3], s>>>(D, bp.map[BP_Y3], bp.total[BP_Y3], 2, bp.ystream);
+    kb_fft_z_inv<R><<<grid_for(bp.total[BP_Z3], FG), FftThreads<R>::v, bp.smem[BP_Z3], s>>>(D, bp.map[BP_Z3], bp.total[BP_Z3], 1);
     pf.end(K_INC_FFT, s, 3);
     pf.begin(K_INCR_END, s);
     kb_incr_end<<<grid_for(bp.total[BP_NP], NG), 128, 0, s>>>(D, bp.map[BP_NP], bp.total[BP_NP]);
@@ -3204,20 +3216,20 @@ cudaError_t launch_plan_incr_end(const BatchPlan &bp, cudaStream_t s, Prof &pf)
 template <typename R>
 static void plan_phase_t(const BatchPlan &bp, int phase, cudaStream_t s)
 {
-    const int FG = 152 * 4;
+    const int FG = 152 * FftGrid<R>::v;
     const RveDesc *D = bp.descs;
     switch (phase) {
     case BP_ZF:
-        kb_fft_z_fwd<R><<<grid_for(bp.total[BP_ZF], FG), 256, bp.smem[BP_ZF], s>>>(D, bp.map[BP_ZF], bp.total[BP_ZF]);
+        kb_fft_z_fwd<R><<<grid_for(bp.total[BP_ZF], FG), FftThreads<R>::v, bp.smem[BP_ZF], s>>>(D, bp.map[BP_ZF], bp.total[BP_ZF]);
         break;
     case BP_Y6:
-        kb_fft_y<R><<<grid_for(bp.total[BP_Y6], FG), 256, bp.smem[BP_Y6], s>>>(D, bp.map[BP_Y6], bp.total[BP_Y6], 0, bp.ystream);
+        kb_fft_y<R><<<grid_for(bp.total[BP_Y6], FG), FftThreads<R>::v, bp.smem[BP_Y6], s>>>(D, bp.map[BP_Y6], bp.total[BP_Y6], 0, bp.ystream);
         break;
     case BP_XG:
-        kb_fft_x_green<R><<<grid_for(bp.total[BP_XG], FG), 256, bp.smem[BP_XG], s>>>(D, bp.map[BP_XG], bp.total[BP_XG]);
+        kb_fft_x_green<R><<<grid_for(bp.total[BP_XG], FG), FftThreads<R>::v, bp.smem[BP_XG], s>>>(D, bp.map[BP_XG], bp.total[BP_XG]);
         break;
     case BP_ZI:
-        kb_fft_z_inv<R><<<grid_for(bp.total[BP_ZI], FG), 256, bp.smem[BP_ZI], s>>>(D, bp.map[BP_ZI], bp.total[BP_ZI], 0);
+        kb_fft_z_inv<R><<<grid_for(bp.total[BP_ZI], FG), FftThreads<R>::v, bp.smem[BP_ZI], s>>>(D, bp.map[BP_ZI], bp.total[BP_ZI], 0);
         break;
     default: break;
     }
@@ -3230,6 +3242,16 @@ cudaError_t launch_plan_phase(const BatchPlan &bp, int phase, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// units of a phase with tile t
+static int tile_units(const RveDesc &d, int phase, int t)
+{
+    switch (phase) {
+    case BP_Y6: return 6 * d.nzh * (d.nx / t);
+    case BP_XG: return d.nzh * (d.ny / t);
+    default: return d.nx * (d.ny / t);
+    }
+}
+
 int tile_candidates(const RveDesc &d, int phase, int *out, int max)
 {
     const bool f = d.mixed != 0;
@@ -3237,8 +3259,14 @@ int tile_candidates(const RveDesc &d, int phase, int *out, int max)
     const size_t cs = f ? sizeof(float2) : sizeof(double2);
     const size_t smem_max = 200 * 1024;
     int n = 0;
-    for (int k = -2; k <= 2 && n < max; ++k) {
+    // from the largest down, and below a quarter of the budget only while a
+    // tile gives the phase fewer units than two blocks per SM: a small grid
+    // fills the GPU with small tiles (16^3 FP64: x + Green 28 -> 24 us, the
+    // Green iteration 113 -> 102 us; 32^3 163 -> 157 us), a large one does
+    // not need them
+    for (int k = 2; k >= -5 && n < max; --k) {
         const int budget = k < 0 ? (B >> -k) : (B << k);
+        if (k < -2 && n > 0 && tile_units(d, phase, out[n - 1]) >= 2 * 152) break;
         int t = 0;
         size_t sm = 0;
         switch (phase) {
@@ -3644,7 +3672,7 @@ __global__ void __launch_bounds__(256) k_disp_z_inv(RveDesc d, void *work, doubl
 template <typename R>
 static cudaError_t disp_fluct_t(const RveDesc &d, void *work, double *out, cudaStream_t s)
 {
-    const int FG = 152 * 4;
+    const int FG = 152 * FftGrid<R>::v;
     const int budget = (sizeof(R) == 8) ? 2048 : 4096;
     const int kc9 = pick_div<R>(d.ny, (budget * 3 / 2) / (9 * d.nx));
     const int xt = d.nx / d.yxt, nzh = d.nzh;
