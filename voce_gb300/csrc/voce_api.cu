@@ -621,6 +621,12 @@ bool fcc_table(RveDesc &d)
         used[found] = true;
         d.canon[k] = found;
         d.flip[k] = flip;
+        d.file[found] = k;
+        const double *n = d.bn + 3 * k, *b = d.bb + 3 * k, h = flip ? -0.5 : 0.5;
+        for (int q = 0; q < 3; ++q) {
+            const int p = (q + 1) % 3, r = (q + 2) % 3;
+            d.skew[3 * found + q] = h * (n[p] * b[r] - n[r] * b[p]);
+        }
     }
     return true;
 }
@@ -1764,7 +1770,8 @@ const char *snapshot_desc_problem(const SnapHead &h, const RveDesc &d, const voc
     if (d.fcc != 0) {
         unsigned seen = 0;
         for (int k = 0; k < VOCE_NS; ++k) {
-            if (d.canon[k] < 0 || d.canon[k] >= VOCE_NS || d.flip[k] < 0 || d.flip[k] > 1) return "slip table";
+            if (d.canon[k] < 0 || d.canon[k] >= VOCE_NS || d.flip[k] < 0 || d.flip[k] > 1 || d.file[d.canon[k]] != k)
+                return "slip table";
             seen |= 1u << d.canon[k];
         }
         if (d.fcc != 1 || d.nsys != VOCE_NS || d.ipow_n < 1 || seen != (1u << VOCE_NS) - 1)

@@ -91,6 +91,8 @@ struct RveDesc {
     int fcc;             // the slip table is the {111}<110> family: Newton in crystal axes (voce_fcc.cuh)
     int canon[VOCE_NS];  // fcc: canonical index of each system, and whether its
     int flip[VOCE_NS];   // direction is the canonical one reversed
+    int file[VOCE_NS];   // fcc: the system at each canonical index
+    double skew[VOCE_NS * 3];   // fcc: axial vector of the spin of each canonical system, n x b / 2
     int update_flag, hard_flag, creep, iter_max;
     int mixed;           // spectrum precision: 0 double, 1 float
     int chord;           // FP64 Newton: reuse the last Jacobian once the update is below 1e-4

@@ -345,7 +345,7 @@ __device__ __forceinline__ double f2d(float f)
     return __hiloint2double(a < 0x00800000u ? 0 : (int)hi, a < 0x00800000u ? 0 : (int)(u << 29));
 }
 
-// x = h + l to about 2^-47: h = d2f(x), l from the 29 significand bits below h
+// x = h + l to about 2^-47 (h truncated): l from the 29 significand bits below h
 __device__ __forceinline__ ff32 d2ff(double x)
 {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);

@@ -147,6 +147,14 @@ __device__ void schmid_from_tm(const RveDesc &d, long long v, const double (&T)[
         }
 }
 
+// put_pair through the integer pipe
+__device__ __forceinline__ void put_ff(float *hi, float *lo, long long i, double x)
+{
+    const ff32 p = d2ff(x);
+    hi[i] = p.h;
+    lo[i] = p.l;
+}
+
 // The crystal-axes columns of voxel v (voce_fcc.cuh) for the orientation T
 // (crystal -> sample): U, P_y, S0_y, and y of the stress the voxel has.
 // Column c of the rotation's deviatoric block is the basis tensor B_c turned
@@ -204,7 +212,7 @@ __device__ __forceinline__ void fcc_frame(const RveDesc &d, long long v, const d
             }
             fx[(FCC_S0 + sym5(c, k)) * nv] = a0;
             fx[(FCC_P + sym5(c, k)) * nv] = a0 + a1;
-            if (d.sgp32) put_pair(d.sgp32, d.sgp_lo, sym5(c, k) * nv + v, a0 + a1);
+            if (d.sgp32) put_ff(d.sgp32, d.sgp_lo, sym5(c, k) * nv + v, a0 + a1);
             if (d.nr32) d.sch32[sym5(c, k) * nv + v] = (float)a0;
         }
     }
@@ -2289,46 +2297,6 @@ __device__ void orientation(double (&tran)[3][3], double (&rot)[3][3])
         for (int b = 0; b < 3; ++b) tran[a][b] = tn[a][b];
 }
 
-// The flow rule of the increment's end for the crystal-axes form: the stress
-// sp = (y, s5) in, its sample 6-vector out; shear rates gd and tx = |r|^(n-1)
-// n gam0 / tau of every system in file order, strain rate ed in sample axes
-__device__ void fcc_flow_out(const RveDesc &d, long long v, double (&sp)[6], double (&ed)[5], double (&gd)[VOCE_NS],
-                             double (&tx)[VOCE_NS])
-{
-    const long long nv = d.nv;
-    double y[5], E[5];
-    for (int c = 0; c < 5; ++c) y[c] = sp[c];
-    sfor<0, 3>([&](auto zc) {
-        constexpr int Z = decltype(zc)::v;
-        double c[4], g[4];
-        fcc_rss<Z, double>(y, c);
-        for (int k = 0; k < 4; ++k) {
-            const int neg = __double2hiint(c[k]) < 0;
-            const double it = d.itau[(long long)(2 * (4 * Z + k) + neg) * nv + v];
-            const double r = c[k] * it;
-            const double q = d.gam0[0] * pow_abs_e(fabs(r), d.ipow_n - 1);
-            g[k] = q * r;
-            for (int s = 0; s < VOCE_NS; ++s)
-                if (d.canon[s] == 4 * Z + k) {
-                    gd[s] = d.flip[s] ? -g[k] : g[k];
-                    tx[s] = (q * it) * d.nrs[s];
-                }
-        }
-        fcc_edot<Z, double>(g, E);
-    });
-    const double *fx = d.sch + v;
-    for (int i = 0; i < 5; ++i) {
-        double s = 0.0, e = 0.0;
-        for (int c = 0; c < 5; ++c) {
-            const double u = fx[(FCC_U + 5 * i + c) * nv];
-            s += u * y[c];
-            e += u * (E[c] / fcc_w2(c));
-        }
-        sp[i] = s;
-        ed[i] = e;
-    }
-}
-
 // increment epilogue (evolution.c:433-530; update_orient constitutive.c:171-248; harden :250-310;
 // update_schmid kinematics.c:426-459)
 __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
@@ -2366,8 +2334,7 @@ __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
         if (d.solid[ph]) {
             double sp[6], gd[VOCE_NS], tx[VOCE_NS];
             for (int c = 0; c < 6; ++c) sp[c] = d.sigp[c * nv + v];
-            if (d.fcc) fcc_flow_out(d, v, sp, ed, gd, tx);
-            else flow_rule<false, true, double>(d, v, sp, ed, (double *)nullptr, gd, tx);
+            flow_rule<false, true, double>(d, v, sp, ed, (double *)nullptr, gd, tx);
             for (int k = 0; k < d.nsys; ++k) {
                 d.gamdot[k * nv + v] = gd[k];
                 d.taux[k * nv + v] = tx[k];
@@ -2410,16 +2377,7 @@ __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
             // resolved shear stresses for the diagnostics, with the Schmid
             // tensors of this increment (the reorientation below replaces them)
             double rss[VOCE_NS];
-            if (hrd && d.fcc) {
-                double y[5], c[4];
-                for (int q = 0; q < 5; ++q) y[q] = d.sch[(FCC_Y + q) * nv + v];
-                sfor<0, 3>([&](auto zc) {
-                    constexpr int Z = decltype(zc)::v;
-                    fcc_rss<Z, double>(y, c);
-                    for (int k = 0; k < d.nsys; ++k)
-                        if (d.canon[k] / 4 == Z) rss[k] = d.flip[k] ? -c[d.canon[k] % 4] : c[d.canon[k] % 4];
-                });
-            } else if (hrd)
+            if (hrd)
                 for (int k = 0; k < d.nsys; ++k) {
                     const double *sc = d.sch + (long long)(5 * k) * nv + v;
                     rss[k] = sc[0] * s6[0] + sc[nv] * s6[1] + sc[2 * nv] * s6[2] + sc[3 * nv] * s6[3] +
@@ -2458,8 +2416,7 @@ __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
                 orientation(T, Rot);
                 for (int a = 0; a < 3; ++a)
                     for (int b = 0; b < 3; ++b) d.tm[(3 * a + b) * nv + v] = T[a][b];
-                if (d.fcc) fcc_frame(d, v, T);
-                else schmid_from_tm(d, v, T);
+                schmid_from_tm(d, v, T);
             }
             if (hrd) {
                 harden_voxel(d, v, gd);
@@ -2481,6 +2438,243 @@ __device__ void incr_end_unit(const RveDesc &d, int unit, int nunits)
         }
         for (int c = 0; c < 5; ++c) { acc[c] += e5[c]; acc[6 + c] += ed[c]; }
     }
+    block_partials(acc, d.part + (long long)unit * VOCE_NPART);
+}
+
+
+// tan x to rounding for the small half angles of a reorientation (the Taylor
+// series through x^9; the next term is below 1e-20 of x for |x| < 2^-6)
+__device__ __forceinline__ double tan_small(double x)
+{
+    if (fabs(x) >= 0.015625) return tan(x);
+    const double q = x * x;
+    double p = fma(62.0 / 2835.0, q, 17.0 / 315.0);
+    p = fma(p, q, 2.0 / 15.0);
+    p = fma(p, q, 1.0 / 3.0);
+    return fma(x * q, p, x);
+}
+
+// ---------------------------------------------------------------------------
+// The increment epilogue of an RVE of the {111}<110> family: incr_end_unit in
+// crystal axes, every per-system quantity in canonical order and in registers
+// (d.file gives the system's place in the arrays that keep file order).
+// Against incr_end_unit, which is bound by the FP64 pipe and by local memory:
+// the plastic spin is summed as the 3 components of its axial vector in
+// crystal axes and turned once (it was 12 products of 3 x 3 matrices), the
+// reorientation works on axial vectors, and the Voce factor, the same for all
+// systems of a slip mode, is computed once instead of twelve times.
+// Third increment (reorientation and hardening): 37 ms at 256^3 (mixed_ir),
+// 4.4 ms at 128^3 (FP64); the whole 256^3 increment of eight Green iterations
+// went from 298 to 202 ms.
+// ---------------------------------------------------------------------------
+__device__ void incr_end_fcc_unit(const RveDesc &d, int unit, int nunits)
+{
+    __shared__ double s_acc[VOCE_NPART][VOCE_NR_THREADS];
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int q = 0; q < VOCE_NPART; ++q) s_acc[q][tid] = 0.0;
+    const MacroDev *m = d.macro;
+    const long long nv = d.nv;
+    const double dt = d.dt, idt = 1.0 / dt, wgt = d.wgt;
+    const int istep = m->istep;
+    const bool upd = d.update_flag == 1 && istep > 1;
+    const bool hrd = d.hard_flag == 1 && istep > 2;
+    // under creep the prelude set DisGrad to the previous DisGradAvg_actual
+    const double *pg = m->DGA_prev;
+    const double dga0[3] = {0.5 * (pg[5] - pg[7]), 0.5 * (pg[2] - pg[6]), 0.5 * (pg[1] - pg[3])};
+    for (long long v = (long long)unit * blockDim.x + threadIdx.x; v < nv;
+         v += (long long)nunits * blockDim.x) {
+        // antisymmetric displacement gradient bookkeeping
+        double rl[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double prev = d.dga[c * nv + v];
+            const double st = d.creep ? dga0[c] : prev + d.ua[c] * dt;
+            const double en = st + m->acum_a[c] + d.rotl[c * nv + v];
+            rl[c] = (en - prev) * idt;
+            d.dga[c * nv + v] = en;
+        }
+        double e5[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) e5[c] = d.eps[c * nv + v];
+        if (!d.solid[d.phase[v]]) {
+#pragma unroll
+            for (int c = 0; c < 5; ++c) {
+                d.edot[c * nv + v] = 0.0;
+                s_acc[c][tid] += e5[c];
+            }
+            continue;
+        }
+        double *fx = d.sch + v;
+        double gd[VOCE_NS];
+        {
+            double y[5], E[5], it[VOCE_NS], p[VOCE_NS];
+#pragma unroll
+            for (int c = 0; c < 5; ++c) y[c] = d.sigp[c * nv + v];
+            fcc_rss12<double>(y, gd);
+#pragma unroll
+            for (int k = 0; k < VOCE_NS; ++k) {
+                it[k] = d.itau[(long long)(2 * k + (__double2hiint(gd[k]) < 0)) * nv + v];
+                gd[k] *= it[k];
+            }
+            fcc_pow<VOCE_NS, double>(gd, d.ipow_n - 1, p);
+            const double g0 = d.gam0[0], n0 = d.nrs[0];
+#pragma unroll
+            for (int k = 0; k < VOCE_NS; ++k) {
+                const double q = g0 * p[k];
+                gd[k] *= q;
+                const long long o = d.file[k] * nv + v;
+                d.gamdot[o] = d.flip[d.file[k]] ? -gd[k] : gd[k];
+                d.taux[o] = (q * it[k]) * n0;
+            }
+            fcc_edot12<double>(gd, E);
+            // strain rate and penultimate stress in sample axes, the total
+            // strain there (EVM: evolution.c:134-155)
+            double sp[5], te[5];
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                double s = 0.0, e = 0.0;
+#pragma unroll
+                for (int c = 0; c < 5; ++c) {
+                    const double u = fx[(FCC_U + 5 * i + c) * nv];
+                    s = fma(u, y[c], s);
+                    e = fma(u, E[c] * (1.0 / fcc_w2(c)), e);
+                }
+                sp[i] = s;
+                d.edot[i * nv + v] = e;
+                s_acc[6 + i][tid] += e;
+                e5[i] = fma(e, dt, e5[i]);   // Eps += Edot dt (evolution.c:464-468)
+                d.eps[i * nv + v] = e5[i];
+                s_acc[i][tid] += e5[i];
+                te[i] = e5[i];
+            }
+#pragma unroll
+            for (int i = 0; i < 5; ++i)
+#pragma unroll
+                for (int j = i; j < 5; ++j) {
+                    const double q = d.sg[(long long)sym6(i, j) * nv + v];
+                    te[i] = fma(q, sp[j], te[i]);
+                    if (i != j) te[j] = fma(q, sp[i], te[j]);
+                }
+            double t2 = 0.0;
+#pragma unroll
+            for (int i = 0; i < 5; ++i) t2 = fma(te[i], te[i], t2);
+            d.evm[v] = sqrt(2. / 3. * t2);
+        }
+        double rss[VOCE_NS];   // resolved shears of the new stress, for the diagnostics
+        {
+            double y[5];
+#pragma unroll
+            for (int c = 0; c < 5; ++c) y[c] = fx[(FCC_Y + c) * nv];
+            d.svm[v] = sqrt(3. / 2. * fcc_norm2<double>(y));
+            fcc_rss12<double>(y, rss);
+        }
+        if (upd) {
+            // update_orient (constitutive.c:171-248) with axial vectors
+            // (w0, w1, w2) = (W21, W02, W10)
+            double T[3][3], wc[3] = {0.0, 0.0, 0.0}, w[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) T[a][b] = d.tm[(3 * a + b) * nv + v];
+#pragma unroll
+            for (int k = 0; k < VOCE_NS; ++k)
+#pragma unroll
+                for (int a = 0; a < 3; ++a) wc[a] = fma(d.skew[3 * k + a], gd[k], wc[a]);
+            const double lw[3] = {-rl[0], rl[1], -rl[2]}, uw[3] = {-d.ua[0], d.ua[1], -d.ua[2]};
+            double n2 = 0.0, l2 = 0.0, r2 = 0.0;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                const double ws = T[a][0] * wc[0] + T[a][1] * wc[1] + T[a][2] * wc[2];
+                n2 = fma(ws, ws, n2);
+                l2 = fma(lw[a], lw[a], l2);
+                w[a] = ((uw[a] + lw[a]) - ws) * dt;
+                r2 = fma(w[a], w[a], r2);
+            }
+            s_acc[12][tid] += sqrt(n2) * wgt;
+            s_acc[13][tid] += sqrt(l2) * wgt;
+            // Orientation (constitutive.c:117-169): T := (I + 2 (om + om^2) / (1 + t^2)) T
+            const double wn = sqrt(r2), wt = tan_small(0.5 * wn);
+            const double f = wn < 1E-6 ? wt : wt / wn, h = 2.0 / fma(wt, wt, 1.0);
+#pragma unroll
+            for (int a = 0; a < 3; ++a) w[a] *= f;
+            const double w2 = w[0] * w[0] + w[1] * w[1] + w[2] * w[2];
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                // om x = w x x, om^2 x = w (w.x) - x |w|^2
+                const double x0 = T[0][b], x1 = T[1][b], x2 = T[2][b];
+                const double dot = w[0] * x0 + w[1] * x1 + w[2] * x2;
+                T[0][b] = fma(h, (w[1] * x2 - w[2] * x1) + (w[0] * dot - x0 * w2), x0);
+                T[1][b] = fma(h, (w[2] * x0 - w[0] * x2) + (w[1] * dot - x1 * w2), x1);
+                T[2][b] = fma(h, (w[0] * x1 - w[1] * x0) + (w[2] * dot - x2 * w2), x2);
+            }
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int b = 0; b < 3; ++b) d.tm[(3 * a + b) * nv + v] = T[a][b];
+            fcc_frame(d, v, T);
+        }
+        if (hrd) {
+            // harden (constitutive.c:261-305) and rho_rss, rho_crss, work_p
+            // (evolution.c:509-529)
+            const double gamtot = d.gamacum[v];
+            double deltgam = 0.0, rr = 0.0, rc = 0.0, wp = 0.0;
+#pragma unroll
+            for (int k = 0; k < VOCE_NS; ++k) {
+                const int fk = d.file[k];
+                const double sg = d.flip[fk] ? -1.0 : 1.0;
+                const double gt = fma(sg * gd[k], dt, d.gtot[fk * nv + v]);
+                d.gtot[fk * nv + v] = gt;
+                gd[k] = fabs(gd[k]) * dt;
+                deltgam += gd[k];
+                rr = fma(rss[k], rss[k], rr);
+                wp += fabs(gt * rss[k]);
+            }
+            const double tau1 = d.tau1[0], th0 = d.thet0[0], th1 = d.thet1[0];
+            const double tiny = 1.E-4 * d.tau0[0];
+            double voce = 0.0;
+            if (fabs(th0) > tiny) {
+                voce = th1 * deltgam;
+                if (fabs(tau1) > tiny) {
+                    const double fact = fabs(th0 / tau1);
+                    const double exp_ini = exp(-1.0 * gamtot * fact);
+                    const double exp_del = exp(-1.0 * deltgam * fact);
+                    voce += -1. * (fact * tau1 - th1) / fact * exp_ini * (exp_del - 1.0) -
+                            th1 / fact * exp_ini * (exp_del * ((gamtot + deltgam) * fact + 1.0) - (gamtot * fact + 1.0));
+                }
+            }
+            const double rate = voce / deltgam;
+#pragma unroll
+            for (int i = 0; i < VOCE_NS; ++i) {
+                const int fi = d.file[i];
+                double dtau = 0.0;
+#pragma unroll
+                for (int j = 0; j < VOCE_NS; ++j) dtau = fma(d.hard[fi * VOCE_NS + d.file[j]], gd[j], dtau);
+                const double inc = dtau * rate;
+                const double c0 = d.crss[(2 * fi) * nv + v] + inc, c1 = d.crss[(2 * fi + 1) * nv + v] + inc;
+                d.crss[(2 * fi) * nv + v] = c0;
+                d.crss[(2 * fi + 1) * nv + v] = c1;
+                // the two directions' CRSS are mostly one value
+                const double i0 = 1.0 / c0, i1 = c1 == c0 ? i0 : 1.0 / c1;
+                const int f0 = 2 * i + d.flip[fi], f1 = 2 * i + 1 - d.flip[fi];   // itau_col(fi, 0), (fi, 1)
+                d.itau[f0 * nv + v] = i0;
+                d.itau[f1 * nv + v] = i1;
+                if (d.itau32) {
+                    put_ff(d.itau32, d.itau_lo, f0 * nv + v, i0);
+                    put_ff(d.itau32, d.itau_lo, f1 * nv + v, i1);
+                }
+                rc = fma(c0, c0, rc);
+            }
+            d.gamacum[v] = gamtot + deltgam;
+            const double ref = 0.35 * 47.565 * 0.256;
+            d.diag[v] = rr * (1.0 / (ref * ref));
+            d.diag[nv + v] = rc * (1.0 / (ref * ref));
+            d.diag[2 * nv + v] = wp;
+        }
+    }
+    double acc[VOCE_NPART];
+#pragma unroll
+    for (int q = 0; q < VOCE_NPART; ++q) acc[q] = s_acc[q][tid];
     block_partials(acc, d.part + (long long)unit * VOCE_NPART);
 }
 
@@ -2893,6 +3087,9 @@ kb_nr(const RveDesc *descs, const int2 *map, int total)
     }
 }
 
+// blocks of 128 threads per SM (256^3 mixed_ir, third increment: 48 ms at 2, 37 at
+// 3, 38 at 4)
+constexpr int kIncrEndBlocks = 3;
 #ifndef VOCE_NR_FCC_BLOCKS
 #define VOCE_NR_FCC_BLOCKS 3
 #endif
@@ -2917,6 +3114,16 @@ __global__ void __launch_bounds__(128) kb_incr_end(const RveDesc *descs, const i
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, MASK_CONVERGED)) continue;
         incr_end_unit(d, e.y, d.npart);
+    }
+}
+
+__global__ void __launch_bounds__(128, kIncrEndBlocks) kb_incr_end_fcc(const RveDesc *descs, const int2 *map, int total)
+{
+    for (int w = blockIdx.x; w < total; w += gridDim.x) {
+        const int2 e = map[w];
+        const RveDesc &d = descs[e.x];
+        if (!unit_on(d, MASK_CONVERGED)) continue;
+        incr_end_fcc_unit(d, e.y, d.npart);
     }
 }
 
@@ -3184,8 +3391,9 @@ static void plan_incr_end_t(const BatchPlan &bp, cudaStream_t s, Prof &pf)
     kb_fft_z_inv<R><<<grid_for(bp.total[BP_Z3], FG), FftThreads<R>::v, bp.smem[BP_Z3], s>>>(D, bp.map[BP_Z3], bp.total[BP_Z3], 1);
     pf.end(K_INC_FFT, s, 3);
     pf.begin(K_INCR_END, s);
-    kb_incr_end<<<grid_for(bp.total[BP_NP], NG), 128, 0, s>>>(D, bp.map[BP_NP], bp.total[BP_NP]);
-    pf.end(K_INCR_END, s);
+    if (const int n = bp.total[BP_NF]) kb_incr_end_fcc<<<grid_for(n, 152 * kIncrEndBlocks), 128, 0, s>>>(D, bp.map[BP_NF], n);
+    if (const int n = bp.total[BP_NG]) kb_incr_end<<<grid_for(n, NG), 128, 0, s>>>(D, bp.map[BP_NG], n);
+    pf.end(K_INCR_END, s, (bp.total[BP_NF] ? 1 : 0) + (bp.total[BP_NG] ? 1 : 0));
     pf.begin(K_FIN_INCR, s);
     kb_finalize<<<grid_for(bp.nrve, 152 * 4), 256, 0, s>>>(D, bp.nrve, 1, 0, 0);
     pf.end(K_FIN_INCR, s);
