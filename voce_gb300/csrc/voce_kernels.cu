@@ -43,45 +43,54 @@ __device__ void block_partials(double (&acc)[VOCE_NPART], double *out)
     __syncthreads();
 }
 
-// sum the per-block partials of one kernel in a fixed order (one block of
-// 256 threads): thread t takes quantity t % 16 over stripe t / 16, a run of
-// consecutive blocks, with up to 32 loads in flight and a pairwise tree over
-// them; the 16 stripe sums are then added pairwise too.  Entry 15 is a max
-// (of non-negative counts, so 0 is its identity as for the sums).
-__device__ void reduce_partials(const double *part, int npart, double (&tot)[VOCE_NPART])
+// Sum the per-block partials of one kernel in a fixed order (one block of 256
+// threads) into tot, in shared memory.  A thread takes one quantity over one
+// stripe, a run of consecutive blocks, with up to 32 loads in flight and a
+// pairwise tree over them; the stripe sums are then added pairwise too.  Entry
+// 15 is a max (of non-negative counts, so 0 is its identity as for the sums).
+// With one phase (all1) the phase-1 sums 8..13 are those of 2..7, and the
+// threads are shared out over the ten others (25 stripes instead of 16).
+__device__ void reduce_partials(const double *part, int npart, int all1, double (&tot)[VOCE_NPART])
 {
-    __shared__ double red[16][VOCE_NPART];
+    __shared__ double red[25][VOCE_NPART];
     const int t = threadIdx.x;  // blockDim.x == 256
-    const int q = t % VOCE_NPART, stripe = t / VOCE_NPART;
+    const int nq = all1 ? 10 : VOCE_NPART, ns = all1 ? 25 : 16;
+    const int stripe = t / nq, k0 = t - stripe * nq;
+    const int q = all1 && k0 >= 8 ? k0 + 6 : k0;
     const bool mx = q == VOCE_NPART - 1;
-    const int chunk = (npart + 15) / 16;
-    const int b0 = stripe * chunk, b1 = min(npart, b0 + chunk);
+    const int chunk = (npart + ns - 1) / ns;
+    const int b0 = stripe * chunk, b1 = stripe < ns ? min(npart, b0 + chunk) : 0;
     double s = 0.0;
     for (int b = b0; b < b1; b += 32) {
         double x[32];
 #pragma unroll
         for (int k = 0; k < 32; ++k) x[k] = (b + k < b1) ? part[(long long)(b + k) * VOCE_NPART + q] : 0.0;
 #pragma unroll
-        for (int w = 16; w >= 1; w >>= 1)
+        for (int w = 16; w >= 1; w >>= 1) {
+            if (w >= b1 - b) continue;   // (nothing but zeros beyond)
 #pragma unroll
             for (int k = 0; k < w; ++k) x[k] = mx ? fmax(x[k], x[k + w]) : x[k] + x[k + w];
+        }
         s = mx ? fmax(s, x[0]) : s + x[0];
     }
-    red[stripe][q] = s;
+    if (stripe < ns) red[stripe][q] = s;
     __syncthreads();
-    if (t < VOCE_NPART) {
-        double v[16];
+    // quantity q by the lanes of one warp's half: 16 lanes, then 8, 4, 2, 1
+    {
+        const int lane16 = t & 15, q2 = t >> 4;
+        const bool on = !(all1 && q2 >= 8 && q2 < 14), mx2 = q2 == VOCE_NPART - 1;
+        double v = on ? red[lane16][q2] : 0.0;
+        if (on && lane16 + 16 < ns) v = mx2 ? fmax(v, red[lane16 + 16][q2]) : v + red[lane16 + 16][q2];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) v[k] = red[k][t];
-#pragma unroll
-        for (int w = 8; w >= 1; w >>= 1)
-#pragma unroll
-            for (int k = 0; k < w; ++k) v[k] = mx ? fmax(v[k], v[k + w]) : v[k] + v[k + w];
-        red[0][t] = v[0];
+        for (int o = 8; o >= 1; o >>= 1) {
+            const double y = __shfl_down_sync(0xffffffffu, v, o, 16);
+            v = mx2 ? fmax(v, y) : v + y;
+        }
+        if (lane16 == 0 && on) {
+            tot[q2] = v;
+            if (all1 && q2 >= 2 && q2 < 8) tot[q2 + 6] = v;
+        }
     }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < VOCE_NPART; ++k) tot[k] = red[0][k];
     __syncthreads();
 }
 
@@ -2072,127 +2081,114 @@ __device__ void sym9_from_b(const double *b6, double *t9)
     t9[1] = t9[3] = t[5];
 }
 
-// s_vm of a symmetric tensor through the deviatoric 5-vector (get_smacro,
-// evolution.c:218-238)
-__device__ double svm_of(const double *t9)
+// Component p of (00, 11, 22, 12, 02, 01) of a 6-vector b: b_to_t6 with the
+// lane's coefficients, three products whatever p is
+__device__ __forceinline__ double t6_component(int p, const double *b)
 {
-    double t6[6] = {t9[0], t9[4], t9[8], t9[5], t9[2], t9[1]}, b6[6];
-    t6_to_b<double>(t6, b6);
-    b6[5] = 0.0;
-    double dev[9];
-    sym9_from_b(b6, dev);
-    double s = 0.0;
-    for (int q = 0; q < 9; ++q) s += dev[q] * dev[q];
-    return sqrt(3. / 2. * s);
+    const double ca = p == 0 ? -RSQ2 : p == 2 ? 0.0 : RSQ2;
+    const double cb = p < 2 ? -RSQ6 : p == 2 ? 2.0 * RSQ6 : 0.0, cc = p < 3 ? RSQ3 : 0.0;
+    return fma(cc, b[5], fma(cb, b[1], ca * b[p < 3 ? 0 : p - 1]));
 }
 
 // Errors, volume averages, mixed-BC macro correction and the convergence
-// decision (evolution.c:401-431, get_smacro :170-241), after the block's
-// reduction of the partial sums, by the block's first warp.  Every value is
-// computed by one lane with the operations, in the order, a single thread
-// would use, so the results do not depend on the split; the lanes compute
-// independent values side by side (the 9 + 9 stress averages, the 6 mixed-BC
-// corrections, the two von Mises norms, the two error normalisations, the
-// epilogue's 9 velocity-gradient divisions and its two norms), each step as
-// one instruction stream for the warp.  That cuts the dependent chain of
-// slow FP64 operations (~60-cycle DADD/DFMA latency, ~1500-cycle divisions)
-// that bounds this kernel.  m is the block's shared-memory copy.
-__device__ void finalize_iter_body(const RveDesc &d, MacroDev *m, int npart)
+// decision (evolution.c:401-431, get_smacro :170-241), from the reduced
+// partial sums tot.  One SM runs this and waits for its slow FP64 operations
+// (64 cycles of a quarter's pipe each, at any number of lanes), so what counts
+// is the number of instructions on the longest chain: warp 0 takes the error
+// norms (the von Mises norm straight from the 6-vector, one reciprocal square
+// root for it and for the strain normalisation, no division), warp 1 the
+// averages and the mixed-BC correction, a value per lane with lane-wise
+// coefficients.  Measured by events at 16^3 / 64^3 (32 / 456 partial sums):
+// 18.4 / 20.5 -> 8.9 / 14.3 us.  m is the block's shared-memory copy.
+__device__ void finalize_iter_body(const RveDesc &d, MacroDev *m, const double *tot)
 {
-    double tot[VOCE_NPART];
-    reduce_partials(d.part, npart, tot);
-    const int lane = threadIdx.x;
-    if (lane >= 32) return;
-    __shared__ double s_dg[9], s_vm2[2], s_act[2][9];
-    const int IJV0[6] = {0, 1, 2, 1, 0, 0}, IJV1[6] = {0, 1, 2, 2, 2, 1};
-    const int first_iter = m->first_iter, it = m->iter, istep = m->istep;
-    const double Err_e0 = m->Err_e, Err_s0 = m->Err_s, e_vm = m->e_vm;
-    // the mixed form's Newton ran in single precision alone this iteration
-    // (the predicate nr_unit used): it may not end the increment
-    const bool fp32_only = d.nr32 && (first_iter || fmax(fabs(Err_e0), fabs(Err_s0)) > VOCE_POLISH_ERR);
-    // lane q < 9: SigAvg[q]; lane 9 + q: SigAvg1[q] (phase 1)
-    if (lane < 18) {
-        double s9[9];
-        sym9_from_b(tot + (lane < 9 ? 2 : 8), s9);
-        const int q = lane < 9 ? lane : lane - 9;
-        const double v = s9[q] * (lane < 9 ? d.wgt : d.wgt_ratio);
-        if (lane < 9) m->SigAvg[q] = v;
-        else m->SigAvg1[q] = v;
-    }
-    // entries get_smacro leaves alone keep their value
-    if (lane < 9) s_dg[lane] = m->dDisGradAvg[lane];
-    __syncwarp();
-    // lane i < 6: dDisGradAvg at IJV(i) (get_smacro)
-    if (lane < 6) {
-        const int ii = IJV0[lane], jj = IJV1[lane];
-        double s = 0.0;
-        if (d.vflag[lane] == 0)
-#pragma unroll
-            for (int k = 0; k < 6; ++k) {
-                const int kk = IJV0[k], ll = IJV1[k];
-                s += d.S0t[((ii * 3 + jj) * 3 + kk) * 3 + ll] * d.sflag[k] *
-                     (d.Scauchy[kk * 3 + ll] - m->SigAvg[kk * 3 + ll]);
-            }
-        s_dg[ii * 3 + jj] = s;
-    }
-    __syncwarp();
-    if (lane < 9) {
-        const double dg = s_dg[lane];
-        m->dDisGradAvg[lane] = dg;
-        m->dDisGradAvg_acum[lane] += dg;
-    }
-    // lane 0: s_vm, lane 1: s_vm1
-    if (lane < 2) {
-        const double v = svm_of(lane == 0 ? m->SigAvg : m->SigAvg1);
-        if (lane == 0) m->s_vm = v;
-        else m->s_vm1 = v;
-        s_vm2[lane] = v;
-    }
-    __syncwarp();
-    // lane 0: Err_s = sum / s_vm; lane 1: Err_e = sum / e_vm when e_vm > 1e-5
-    // (x / 1.0 is x exactly, so the untaken division is a division by one)
-    double err = 0.0;
-    if (lane < 2) {
-        const double num = tot[lane == 0 ? 0 : 1] * d.wgt;
-        const double den = lane == 0 ? s_vm2[0] : (fabs(e_vm) > 1E-5 ? e_vm : 1.0);
-        err = num / den;
-    }
-    const double Err_s = __shfl_sync(0xffffffffu, err, 0), Err_e = __shfl_sync(0xffffffffu, err, 1);
-    if (lane == 0) {
-        m->Err_e = Err_e;
-        m->Err_s = Err_s;
-    }
-    if (it < d.iter_max && lane < VOCE_ITLOG) {
-        const int slot = (istep - 1) % d.incr_cap;
-        double *lg = d.itlog + ((long long)slot * d.iter_max + it) * VOCE_ITLOG;
-        double v;
-        switch (lane) {
-        case 0: v = Err_e; break;
-        case 1: v = Err_s; break;
-        case 2: v = s_vm2[0]; break;
-        case 3: v = tot[14]; break;
-        case 4: v = tot[1]; break;   // raw sum of the strain-compatibility norms
-        case 5: v = tot[0]; break;   // raw sum of the stress-change norms
-        default: v = tot[2 + lane - 6]; break;   // sum of sigma (basis)
+    __shared__ double s_dg[9], s_t6[6], s_act[2][9];
+    __shared__ int s_more;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int it = m->iter, istep = m->istep;
+    if (warp == 0) {
+        // lane 0: s_vm and Err_s, lane 1: s_vm1, lane 2: Err_e
+        const double e_vm = m->e_vm;
+        // the mixed form's Newton ran in single precision alone this iteration
+        // (the predicate nr_unit used): it may not end the increment
+        const bool fp32_only = d.nr32 && (m->first_iter || fmax(fabs(m->Err_e), fabs(m->Err_s)) > VOCE_POLISH_ERR);
+        const double *b = tot + (lane == 1 ? 8 : 2);
+        double x = lane == 2 ? (fabs(e_vm) > 1E-5 ? e_vm * e_vm : 1.0)
+                             : 1.5 * (((b[0] * b[0] + b[1] * b[1]) + (b[2] * b[2] + b[3] * b[3])) + b[4] * b[4]);
+        const double r = rsqrt(x);
+        // sum wgt / (wgt sqrt(x)), and sum wgt / e_vm
+        const double err = lane == 2 ? (tot[1] * d.wgt) * r : tot[0] * r;
+        const double svm = x > 0.0 ? (x * r) * (lane == 1 ? d.wgt_ratio : d.wgt) : 0.0;
+        const double Err_s = __shfl_sync(0xffffffffu, err, 0), Err_e = __shfl_sync(0xffffffffu, err, 2);
+        const double s_vm = __shfl_sync(0xffffffffu, svm, 0);
+        const bool more = (it + 1 < d.iter_max) &&
+                          (fp32_only || fmax(fabs(Err_s), fabs(Err_e)) > fabs(d.err_tol));
+        if (lane == 1) m->s_vm1 = svm;
+        if (lane == 0) {
+            m->s_vm = svm;
+            m->Err_e = Err_e;
+            m->Err_s = Err_s;
+            m->iter = it + 1;
+            m->iter_total += 1;
+            m->nr_total += tot[14];
+            m->nr_max = max(m->nr_max, (int)tot[15]);
+            m->first_iter = 0;
+            m->pending_prelude = 0;
+            m->converged = more ? 0 : 1;
+            s_more = more;
         }
-        lg[lane] = v;
+        if (it < d.iter_max && lane < VOCE_ITLOG) {
+            const int slot = (istep - 1) % d.incr_cap;
+            double *lg = d.itlog + ((long long)slot * d.iter_max + it) * VOCE_ITLOG;
+            // Err_e, Err_s, s_vm, Newton steps, the raw sums of the strain-compatibility and
+            // stress-change norms, the sum of sigma (basis)
+            const int from[VOCE_ITLOG] = {0, 0, 0, 14, 1, 0, 2, 3, 4, 5, 6, 7};
+            lg[lane] = lane == 0 ? Err_e : lane == 1 ? Err_s : lane == 2 ? s_vm : tot[from[lane]];
+        }
+    } else if (warp == 1) {
+        // lane q < 9: SigAvg[q]; lane 9 + q: SigAvg1[q] (phase 1)
+        if (lane < 18) {
+            const int q = lane < 9 ? lane : lane - 9;
+            const int p6[9] = {0, 5, 4, 5, 1, 3, 4, 3, 2};
+            const double v = t6_component(p6[q], tot + (lane < 9 ? 2 : 8)) * (lane < 9 ? d.wgt : d.wgt_ratio);
+            if (lane < 9) m->SigAvg[q] = v;
+            else m->SigAvg1[q] = v;
+        }
+        // entries get_smacro leaves alone keep their value
+        if (lane < 9) s_dg[lane] = m->dDisGradAvg[lane];
+        __syncwarp();
+        const int I6[6] = {0, 1, 2, 1, 0, 0}, J6[6] = {0, 1, 2, 2, 2, 1};
+        // lane i < 6: dDisGradAvg at component i (get_smacro); the stress flags are 0 or 1
+        if (lane < 6) {
+            const int ii = I6[lane], jj = J6[lane];
+            double s = 0.0;
+            if (d.vflag[lane] == 0)
+#pragma unroll
+                for (int k = 0; k < 6; ++k) {
+                    const int kk = I6[k], ll = J6[k];
+                    if (d.sflag[k])
+                        s = fma(d.S0t[((ii * 3 + jj) * 3 + kk) * 3 + ll], d.Scauchy[kk * 3 + ll] - m->SigAvg[kk * 3 + ll], s);
+                }
+            s_dg[ii * 3 + jj] = s;
+        }
+        __syncwarp();
+        if (lane < 9) {
+            const double dg = s_dg[lane];
+            m->dDisGradAvg[lane] = dg;
+            m->dDisGradAvg_acum[lane] += dg;
+        }
+        // its symmetric part in the 6-vector basis, for the next update
+        if (lane < 6) s_t6[lane] = 0.5 * (s_dg[I6[lane] * 3 + J6[lane]] + s_dg[J6[lane] * 3 + I6[lane]]);
+        __syncwarp();
+        if (lane < 6) {
+            const double k0 = lane == 0 ? -RSQ2 : lane == 1 ? -RSQ6 : lane == 5 ? RSQ3 : 0.0;
+            const double k1 = lane == 0 ? RSQ2 : k0, k2 = lane == 1 ? 2.0 * RSQ6 : lane == 5 ? RSQ3 : 0.0;
+            const bool shear = lane >= 2 && lane < 5;
+            m->ddg6[lane] = shear ? 2.0 * RSQ2 * s_t6[lane + 1] : fma(k2, s_t6[2], fma(k1, s_t6[1], k0 * s_t6[0]));
+        }
     }
-    __syncwarp();
-    const bool more = (it + 1 < d.iter_max) &&
-                      (fp32_only || fmax(fabs(Err_s), fabs(Err_e)) > fabs(d.err_tol));
-    if (lane == 0) {
-        m->iter = it + 1;
-        m->iter_total += 1;
-        m->nr_total += tot[14];
-        m->nr_max = max(m->nr_max, (int)tot[15]);
-        const double *dg = s_dg;
-        double t6[6] = {dg[0], dg[4], dg[8], 0.5 * (dg[5] + dg[7]), 0.5 * (dg[2] + dg[6]), 0.5 * (dg[1] + dg[3])};
-        t6_to_b<double>(t6, m->ddg6);
-        m->first_iter = 0;
-        m->pending_prelude = 0;
-        m->converged = more ? 0 : 1;
-    }
-    if (more) return;
+    __syncthreads();
+    if (s_more || warp != 0) return;
     // epilogue macro bookkeeping (evolution.c:438-461); lane q < 9 entry q
     if (lane < 9) {
         const int q = lane;
@@ -2700,10 +2696,8 @@ __device__ void prelude_unit(const RveDesc &d, int unit, int nunits)
 }
 
 
-__device__ void finalize_incr_body(const RveDesc &d, MacroDev *m, int npart)
+__device__ void finalize_incr_body(const RveDesc &d, MacroDev *m, const double *tot)
 {
-    double tot[VOCE_NPART];
-    reduce_partials(d.part, npart, tot);
     if (threadIdx.x != 0) return;
     double e6[6] = {tot[0], tot[1], tot[2], tot[3], tot[4], 0.0};
     double d6[6] = {tot[6], tot[7], tot[8], tot[9], tot[10], 0.0};
@@ -3140,11 +3134,11 @@ __global__ void __launch_bounds__(128) kb_prelude(const RveDesc *descs, const in
 // one block per RVE.  With use_cond (a plan of one RVE), the iteration
 // finaliser also sets the condition of the graph's WHILE node: continue
 // while the RVE has not converged (evolution.c:342).
-// The RVE's descriptor and macro state are first copied into shared memory
-// by the whole block, so that the finaliser's single thread reads and
-// updates them at shared-memory latency instead of in a chain of dependent
-// global round trips; the macro state is written back once at the end.  The
-// arithmetic is unchanged.
+// The RVE's descriptor and macro state are copied into shared memory by the
+// whole block while the partial sums are reduced, so that the finaliser reads
+// and updates them at shared-memory latency; the macro state is written back
+// once at the end.  The iteration finaliser starts its loads before it knows
+// whether the RVE is active (most are), the increment's waits for the flag.
 __global__ void __launch_bounds__(256) kb_finalize(const RveDesc *descs, int nrve, int incr_end,
                                                    cudaGraphConditionalHandle cond, int use_cond)
 {
@@ -3152,21 +3146,28 @@ __global__ void __launch_bounds__(256) kb_finalize(const RveDesc *descs, int nrv
     constexpr int kDescWords = (int)(sizeof(RveDesc) / 8), kMacroWords = (int)(sizeof(MacroDev) / 8);
     __shared__ unsigned long long s_desc[kDescWords];
     __shared__ unsigned long long s_macro[kMacroWords];
+    __shared__ double s_tot[VOCE_NPART];
     for (int r = blockIdx.x; r < nrve; r += gridDim.x) {
         const RveDesc &dg = descs[r];
-        if (!unit_on(dg, incr_end ? MASK_CONVERGED : MASK_ACTIVE)) continue;
+        if (incr_end && !unit_on(dg, MASK_CONVERGED)) continue;
         unsigned long long *gm = reinterpret_cast<unsigned long long *>(dg.macro);
         const unsigned long long *gd = reinterpret_cast<const unsigned long long *>(&dg);
-        for (int i = threadIdx.x; i < kDescWords; i += blockDim.x) s_desc[i] = gd[i];
+        const double *part = dg.part;
+        const int npart = dg.npart, all1 = !incr_end && dg.all_ph1;
         for (int i = threadIdx.x; i < kMacroWords; i += blockDim.x) s_macro[i] = gm[i];
-        __syncthreads();
+        for (int i = threadIdx.x; i < kDescWords; i += blockDim.x) s_desc[i] = gd[i];
+        reduce_partials(part, npart, all1, s_tot);   // (synchronises the block)
         const RveDesc &d = *reinterpret_cast<const RveDesc *>(s_desc);
         MacroDev *m = reinterpret_cast<MacroDev *>(s_macro);
-        if (incr_end) finalize_incr_body(d, m, d.npart);
-        else finalize_iter_body(d, m, d.npart);
+        if (!m->active) {
+            __syncthreads();
+            continue;
+        }
+        if (incr_end) finalize_incr_body(d, m, s_tot);
+        else finalize_iter_body(d, m, s_tot);
         __syncthreads();
-        for (int i = threadIdx.x; i < kMacroWords; i += blockDim.x) gm[i] = s_macro[i];
         if (use_cond && threadIdx.x == 0) cudaGraphSetConditional(cond, m->converged ? 0u : 1u);
+        for (int i = threadIdx.x; i < kMacroWords; i += blockDim.x) gm[i] = s_macro[i];
         __syncthreads();
     }
 }
