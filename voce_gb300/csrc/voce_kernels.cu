@@ -1712,18 +1712,18 @@ __device__ void nr_unit(const RveDesc &d, int unit, int nunits)
 // 72 for the powers, 25 for P y (the pressure decouples); the tangent and the
 // 5x5 solve, 240 + 125 there, run in float pairs on the FP32 pipe beside it.
 // Measured per launch against kb_nr (FP64 form, first increment): 64^3 879 ->
-// 358 us (477 with the solve in FP64), 16^3 (a grain per voxel) 86 -> 48 us.
+// 359 us (477 with the solve in FP64), 16^3 (a grain per voxel) 86 -> 45 us.
 // With the solve off the FP64 pipe a chord step saves nothing, so d.chord is
 // not looked at here.
 //
 // FCC_IR (VOCE_PREC_MIXED_IR): newton_ir in the same variables: the start in
 // single precision and float pairs, then steps whose residual, flow rule and
 // stop test are FP64 and whose correction is solved in FP32 with the start's
-// last matrix; 64^3 363 -> 221 us, 256^3 29.9 -> 15.6 ms.  FCC_NR32
-// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 309 us.  Nothing is staged
+// last matrix; 64^3 363 -> 216 us, 256^3 29.9 -> 15.4 ms.  FCC_NR32
+// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 295 us.  Nothing is staged
 // in shared memory: the single-precision steps read 15 + 12 floats per voxel
 // instead of 21 + 72.  Conversions go through the integer pipe (d2f, f2d:
-// with the hardware's, 239 and 342 us).
+// with the hardware's, 239 and 331 us).
 //
 // kb_nr stays for every other slip table and for non-integral exponents.
 // ---------------------------------------------------------------------------
@@ -1985,9 +1985,9 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
             // in single precision: they only steer the Green iteration's stop
             // test at 1e-5
             float dy[5], te[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            float d5 = (float)(s5 - s5l), r5 = 0.0f;
+            float d5 = d2f(s5 - s5l), r5 = 0.0f;
 #pragma unroll
-            for (int c = 0; c < 5; ++c) dy[c] = (float)(y[c] - yl[c]);
+            for (int c = 0; c < 5; ++c) dy[c] = d2f(y[c] - yl[c]);
             ncs = (double)sqrtf(fmaf(d5, d5, fcc_norm2<float>(dy)));
             if (!converged) {   // (a point taken as converged: yp = y, no residual)
 #pragma unroll
@@ -2047,16 +2047,26 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
         s_it[0][tid] += it;
         s_it[1][tid] = max(s_it[1][tid], it);
     }
-    double acc[VOCE_NPART];
+    // the block's partial sums: a warp takes every fourth quantity over the 128
+    // thread sums (eight additions a quantity; a shuffle tree per thread over
+    // all sixteen took eighty).  With one phase the phase-1 sums are the full
+    // ones again and are left out.
+    __syncthreads();
+    const int lane = tid & 31, nq = d.all_ph1 ? 8 : 14;
+    double *out = d.part + (long long)unit * VOCE_NPART;
+    for (int q = tid >> 5; q < nq; q += VOCE_NR_THREADS / 32) {
+        double s = (s_acc[q][lane] + s_acc[q][lane + 32]) + (s_acc[q][lane + 64] + s_acc[q][lane + 96]);
 #pragma unroll
-    for (int q = 0; q < VOCE_NPART; ++q) acc[q] = s_acc[q][tid];
-    if (d.all_ph1) {
-#pragma unroll
-        for (int c = 0; c < 6; ++c) acc[8 + c] = acc[2 + c];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (lane == 0) out[q] = s;
     }
-    acc[14] = (double)s_it[0][tid];
-    acc[15] = (double)s_it[1][tid];
-    block_partials(acc, d.part + (long long)unit * VOCE_NPART);
+    if (tid < 32) {
+        const int n = s_it[0][lane] + s_it[0][lane + 32] + s_it[0][lane + 64] + s_it[0][lane + 96];
+        const int m = max(max(s_it[1][lane], s_it[1][lane + 32]), max(s_it[1][lane + 64], s_it[1][lane + 96]));
+        const int sn = __reduce_add_sync(0xffffffffu, n), sm = __reduce_max_sync(0xffffffffu, m);
+        if (lane < 2) out[14 + lane] = (double)(lane ? sm : sn);
+    }
+    __syncthreads();
 }
 
 
