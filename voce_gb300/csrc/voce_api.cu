@@ -862,7 +862,7 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
     d.all_ph1 = nph1 == nv ? 1 : 0;
 
     CUDA_TRY(launch_setup(d, sc, d_eul, r->npart, r->stream));
-    std::vector<double> part((size_t)3 * r->npart * VOCE_NPART);
+    std::vector<double> part((size_t)2 * r->npart * VOCE_NPART);
     CUDA_TRY(cudaMemcpyAsync(part.data(), d.part, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, r->stream));
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     // the Euler angles live on as the orientation matrices: their staging
@@ -872,14 +872,16 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
     CUDA_TRY(cudaFree(d_eul));
     d_eul = nullptr;
     // C066 = WGT * sum over voxels of C_gr (init.c:450-456), block partials
-    // summed in block order
-    double sums[48] = {0};
-    for (int pass = 0; pass < 3; ++pass)
+    // summed in block order: the deviatoric block and the pressure entry
+    double sums[30] = {0};
+    for (int pass = 0; pass < 2; ++pass)
         for (int b = 0; b < r->npart; ++b)
             for (int q = 0; q < VOCE_NPART - 1; ++q)
                 sums[pass * (VOCE_NPART - 1) + q] += part[((size_t)pass * r->npart + b) * VOCE_NPART + q];
-    double C066[6][6], S066[6][6];
-    for (int q = 0; q < 36; ++q) C066[q / 6][q % 6] = sums[1 + q] * d.wgt;
+    double C066[6][6] = {{0.0}}, S066[6][6];
+    for (int i = 0, q = 0; i < 5; ++i)
+        for (int j = i; j < 5; ++j, ++q) C066[i][j] = C066[j][i] = sums[1 + q] * d.wgt;
+    C066[5][5] = sums[16] * d.wgt;
     std::memcpy(S066, C066, sizeof(S066));
     if (!lu_inv66(S066)) return fail(VOCE_ERR_SINGULAR, "singular reference stiffness C066");
     std::memcpy(d.S0, S066, sizeof(S066));
