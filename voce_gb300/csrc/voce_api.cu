@@ -1030,7 +1030,7 @@ int make_plan(const std::vector<RveDesc> &descs, int precision, RveDesc *&d_desc
             p.smem[ph] = std::max(p.smem[ph], batch_smem(descs[i], ph));
         }
     }
-    if (p.mixed) {   // the streamed y pass: all RVEs on the register FFT along y
+    {   // the streamed y pass: all RVEs on the register FFT along y
         long long S = 0;
         bool all = true;
         for (const RveDesc &d : descs) {
@@ -1039,7 +1039,7 @@ int make_plan(const std::vector<RveDesc> &descs, int precision, RveDesc *&d_desc
         }
         if (all) {
             p.ystream = (int)((S + 1) & ~1LL);
-            const size_t sm = 2 * (size_t)p.ystream * sizeof(float2);
+            const size_t sm = 2 * (size_t)p.ystream * (p.mixed ? sizeof(float2) : sizeof(double2));
             p.smem[BP_Y6] = std::max(p.smem[BP_Y6], sm);
             p.smem[BP_Y3] = std::max(p.smem[BP_Y3], sm);
         }

@@ -179,6 +179,38 @@ __host__ __device__ __forceinline__ int sym6(int i, int j)
     return a * 6 - (a * (a - 1)) / 2 + (b - a);
 }
 
+// ---------------------------------------------------------------------------
+// Conversions between double and float with integer operations, which keeps
+// them off the FP64 pipe (a hardware conversion holds it as long as an FP64
+// product).  d2f truncates; values below the smallest normal float become
+// zero, and the caller keeps |x| < 2^127 (finite).  f2d is exact for normal
+// floats and zero; subnormal floats become zero, infinities and NaN are the
+// caller's to exclude.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float d2f(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    // exponent bias 1023 -> 127: the low eight exponent bits with the top one
+    // of them flipped
+    const unsigned m = ((__funnelshift_l(lo, hi, 3) & 0x7fffffffu) ^ 0x40000000u) | (hi & 0x80000000u);
+    return __uint_as_float((hi & 0x7fffffffu) < 0x38100000u ? 0u : m);
+}
+
+// d2f rounded to nearest (ties away from zero)
+__device__ __forceinline__ float d2f_rn(double x)
+{
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned l2 = lo + 0x10000000u, h2 = hi + (l2 < lo ? 1u : 0u);
+    return d2f(__hiloint2double((int)h2, (int)l2));
+}
+
+__device__ __forceinline__ double f2d(float f)
+{
+    const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+    const unsigned hi = ((a >> 3) + 0x38000000u) | (u & 0x80000000u);
+    return __hiloint2double(a < 0x00800000u ? 0 : (int)hi, a < 0x00800000u ? 0 : (int)(u << 29));
+}
+
 // Newton-Raphson reciprocal: the hardware's approximate double reciprocal
 // (rcp.approx.ftz.f64, about 20 correct bits) refined by two steps of
 // r <- r + r(1 - x r), each of which squares the relative error (down to
@@ -786,12 +818,16 @@ template <typename R> struct Cx;
 template <> struct Cx<double> { typedef double2 T; };
 template <> struct Cx<float> { typedef float2 T; };
 
+// (the fused operations are written out: the y pass has two kernels for one
+// transform, which must round alike)
+__device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return fma(a, b, c); }
 template <typename R>
 __device__ __forceinline__ typename Cx<R>::T cmul(typename Cx<R>::T a, typename Cx<R>::T b)
 {
     typename Cx<R>::T c;
-    c.x = a.x * b.x - a.y * b.y;
-    c.y = a.x * b.y + a.y * b.x;
+    c.x = fma_(-a.y, b.y, a.x * b.x);
+    c.y = fma_(a.y, b.x, a.x * b.y);
     return c;
 }
 
@@ -882,7 +918,7 @@ __device__ __forceinline__ C rot(C v)
         else return mkc<C>(v.y, -v.x);
     } else {
         constexpr R c = (R)cos48(a), s = (R)(S * sin48(a));
-        return mkc<C>(c * v.x - s * v.y, c * v.y + s * v.x);
+        return mkc<C>(fma_(-s, v.y, c * v.x), fma_(s, v.x, c * v.y));
     }
 }
 

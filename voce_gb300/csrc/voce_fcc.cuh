@@ -321,30 +321,6 @@ __device__ __forceinline__ int itau_col(const RveDesc &d, int k, int f)
     return d.fcc ? 2 * d.canon[k] + (f ^ d.flip[k]) : 2 * k + f;
 }
 
-// ---------------------------------------------------------------------------
-// Conversions between double and float with integer operations, which keeps
-// them off the FP64 pipe (a hardware conversion holds it as long as an FP64
-// product).  d2f truncates; values below the smallest normal float become
-// zero, and the caller keeps |x| < 2^127 (finite).  f2d is exact for normal
-// floats and zero; subnormal floats become zero, infinities and NaN are the
-// caller's to exclude.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float d2f(double x)
-{
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    // exponent bias 1023 -> 127: the low eight exponent bits with the top one
-    // of them flipped
-    const unsigned m = ((__funnelshift_l(lo, hi, 3) & 0x7fffffffu) ^ 0x40000000u) | (hi & 0x80000000u);
-    return __uint_as_float((hi & 0x7fffffffu) < 0x38100000u ? 0u : m);
-}
-
-__device__ __forceinline__ double f2d(float f)
-{
-    const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
-    const unsigned hi = ((a >> 3) + 0x38000000u) | (u & 0x80000000u);
-    return __hiloint2double(a < 0x00800000u ? 0 : (int)hi, a < 0x00800000u ? 0 : (int)(u << 29));
-}
-
 // x = h + l to about 2^-47 (h truncated): l from the 29 significand bits below h
 __device__ __forceinline__ ff32 d2ff(double x)
 {

@@ -381,6 +381,10 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(__cvta_generic_to_global(gmem)) : "memory");
 }
 
+// one complex number
+__device__ __forceinline__ void cp_asyncc(float2 *smem, const float2 *gmem) { cp_async8(smem, gmem); }
+__device__ __forceinline__ void cp_asyncc(double2 *smem, const double2 *gmem) { cp_async16(smem, gmem); }
+
 __device__ __forceinline__ void cp_async_wait_all()
 {
     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -482,7 +486,7 @@ __device__ void fft_z_fwd_unit(const RveDesc &d, int rows, int unit)
         Idx3 ix(threadIdx.x, blockDim.x, nz, rows);
         for (int i = threadIdx.x; i < 3 * run; i += blockDim.x, ix.next()) {
             const int z = ix.a0, r = ix.a1, p = ix.a2, q = r * nz + z;
-            bufA[z * ldl + p * rows + r] = make_float2((float)stage[2 * p * run + q], (float)stage[(2 * p + 1) * run + q]);
+            bufA[z * ldl + p * rows + r] = make_float2(d2f_rn(stage[2 * p * run + q]), d2f_rn(stage[(2 * p + 1) * run + q]));
         }
     } else {
         // element (z, r, c) is sig[c][vb + r * nz + z]
@@ -595,7 +599,7 @@ __device__ void fft_y_unit(const RveDesc &d, void *specp, int sign, int xt, int 
 
 
 // ---------------------------------------------------------------------------
-// The y pass of the single-precision spectrum as a stream over a block's
+// The y pass as a stream over a block's
 // units, for plans whose RVEs all run the register FFT along y.  A unit's
 // tile (NL = yxt lines of L = ny contiguous coefficients) is held line by
 // line at pos(l, i) = l LP + i + i / N2, LP = L + N1 + 1: pass 1 (tasks
@@ -603,26 +607,26 @@ __device__ void fft_y_unit(const RveDesc &d, void *specp, int sign, int xt, int 
 // of consecutive words, and pass 2 writes X[k1 + N1 k2] of line l straight
 // to the spectrum, consecutive threads to consecutive coefficients.  The
 // next unit's tile is staged by cp.async while this one transforms (two
-// tile buffers of S complex floats, S >= NL LP of every RVE of the plan).
+// tile buffers of S complex numbers, S >= NL LP of every RVE of the plan).
 // ---------------------------------------------------------------------------
-template <int N1, int N2, int S>
-__device__ __forceinline__ void ystream_tile(float2 *A, int NL, float2 *g, const float2 *__restrict__ tw)
+template <typename C, int N1, int N2, int S>
+__device__ __forceinline__ void ystream_tile(C *A, int NL, C *g, const C *__restrict__ tw)
 {
     constexpr int L = N1 * N2, LP = L + N1 + 1;
     const int tid = threadIdx.x, nthr = blockDim.x;
     for (int task = tid; task < NL * N2; task += nthr) {
         const int l = task / N2, t = task - l * N2;
-        float2 *p = A + l * LP + t;
-        float2 x[N1];
+        C *p = A + l * LP + t;
+        C x[N1];
         sfor<0, N1>([&](auto jc) { x[decltype(jc)::v] = p[(N2 + 1) * decltype(jc)::v]; });
         sdft<N1, S, 0, 1>(x);
         if (t != 0) {
-            const float2 *wm = tw + L + t;   // the pass-1 twiddle matrix
+            const C *wm = tw + L + t;   // the pass-1 twiddle matrix
             sfor<1, N1>([&](auto kc) {
                 constexpr int k = decltype(kc)::v, r = dft_pos(N1, k);
-                float2 w = __ldg(wm + k * N2);
+                C w = __ldg(wm + k * N2);
                 if (S > 0) w.y = -w.y;
-                x[r] = cmul<float>(x[r], w);
+                x[r] = cmul<typename RealOf<C>::T>(x[r], w);
             });
         }
         sfor<0, N1>([&](auto kc) { p[(N2 + 1) * decltype(kc)::v] = x[dft_pos(N1, decltype(kc)::v)]; });
@@ -630,12 +634,12 @@ __device__ __forceinline__ void ystream_tile(float2 *A, int NL, float2 *g, const
     __syncthreads();
     for (int task = tid; task < NL * N1; task += nthr) {
         const int l = task / N1, k1 = task - l * N1;
-        const float2 *p = A + l * LP + (N2 + 1) * k1;
-        float2 x[N2];
+        const C *p = A + l * LP + (N2 + 1) * k1;
+        C x[N2];
 #pragma unroll
         for (int t = 0; t < N2; ++t) x[t] = p[t];
         sdft<N2, S, 0, 1>(x);
-        float2 *q = g + l * L + k1;
+        C *q = g + l * L + k1;
         sfor<0, N2>([&](auto kc) { q[N1 * decltype(kc)::v] = x[dft_pos(N2, decltype(kc)::v)]; });
     }
 }
@@ -727,8 +731,8 @@ __device__ void fft_x_green_unit(const RveDesc &d, int kc, int unit)
 
 
 // ---------------------------------------------------------------------------
-// The x pass with the Green operator for an RVE on the register FFT along x
-// (single precision).  The tile's NL = 6 kc lines (line l = c kc + yl:
+// The x pass with the Green operator for an RVE on the register FFT along x.
+// The tile's NL = 6 kc lines (line l = c kc + yl:
 // component c, column y0 + yl) are held line by line at pos(l, i) = l LP +
 // i + i / N2, LP = L + N1 + 1 (odd): the forward transform runs in place on
 // A and leaves X[k] at pos(l, k) of B, the Green operator works on B, the
@@ -736,64 +740,65 @@ __device__ void fft_x_green_unit(const RveDesc &d, int kc, int unit)
 // to the spectrum.  Every shared-memory index inside the transforms is a
 // compile-time offset from one base per task.
 // ---------------------------------------------------------------------------
-template <int N1, int N2, int S>
-__device__ __forceinline__ void xg_pass1(float2 *A, int NL, const float2 *__restrict__ tw)
+template <typename C, int N1, int N2, int S>
+__device__ __forceinline__ void xg_pass1(C *A, int NL, const C *__restrict__ tw)
 {
     constexpr int L = N1 * N2, LP = L + N1 + 1;
     for (int task = threadIdx.x; task < NL * N2; task += blockDim.x) {
         const int l = task / N2, t = task - l * N2;
-        float2 *p = A + l * LP + t;
-        float2 x[N1];
+        C *p = A + l * LP + t;
+        C x[N1];
         sfor<0, N1>([&](auto jc) { x[decltype(jc)::v] = p[(N2 + 1) * decltype(jc)::v]; });
         sdft<N1, S, 0, 1>(x);
         if (t != 0) {
-            const float2 *wm = tw + L + t;   // the pass-1 twiddle matrix
+            const C *wm = tw + L + t;   // the pass-1 twiddle matrix
             sfor<1, N1>([&](auto kc) {
                 constexpr int k = decltype(kc)::v, r = dft_pos(N1, k);
-                float2 w = __ldg(wm + k * N2);
+                C w = __ldg(wm + k * N2);
                 if (S > 0) w.y = -w.y;
-                x[r] = cmul<float>(x[r], w);
+                x[r] = cmul<typename RealOf<C>::T>(x[r], w);
             });
         }
         sfor<0, N1>([&](auto kc) { p[(N2 + 1) * decltype(kc)::v] = x[dft_pos(N1, decltype(kc)::v)]; });
     }
 }
 
-template <int N1, int N2>
-__device__ void xg_unit_f32(const RveDesc &d, int kc, int unit)
+template <typename C, int N1, int N2>
+__device__ void xg_unit(const RveDesc &d, int kc, int unit)
 {
+    typedef typename RealOf<C>::T R;
     constexpr int L = N1 * N2, LP = L + N1 + 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2 *A = reinterpret_cast<float2 *>(smem_raw);
+    C *A = reinterpret_cast<C *>(smem_raw);
     const int NL = 6 * kc;
-    float2 *B = A + NL * LP;
+    C *B = A + NL * LP;
     const int ny = d.ny, nzh = d.nzh;
     const int ytiles = ny / kc;
     const int kz = unit / ytiles, y0 = (unit % ytiles) * kc;
-    float2 *spec = (float2 *)d.spec, *aacc = (float2 *)d.aacc;
+    C *spec = (C *)d.spec, *aacc = (C *)d.aacc;
     const long long plane = (long long)L * ny, cstride = (long long)nzh * plane;
     const long long kb = (long long)kz * plane + y0;
-    const float2 *tw = (const float2 *)d.twx;
+    const C *tw = (const C *)d.twx;
     const int tid = threadIdx.x, nthr = blockDim.x;
     {   // element (yl, x, c), yl fastest
         Idx3 il(tid, nthr, kc, L);
         for (int i = tid; i < NL * L; i += nthr, il.next()) {
             const int yl = il.a0, x = il.a1, c = il.a2;
-            cp_async8(A + (c * kc + yl) * LP + x + x / N2, spec + c * cstride + kb + (long long)x * ny + yl);
+            cp_asyncc(A + (c * kc + yl) * LP + x + x / N2, spec + c * cstride + kb + (long long)x * ny + yl);
         }
         cp_async_wait_all();
     }
     __syncthreads();
-    xg_pass1<N1, N2, -1>(A, NL, tw);
+    xg_pass1<C, N1, N2, -1>(A, NL, tw);
     __syncthreads();
     for (int task = tid; task < NL * N1; task += nthr) {
         const int l = task / N1, k1 = task - l * N1;
-        const float2 *p = A + l * LP + (N2 + 1) * k1;
-        float2 x[N2];
+        const C *p = A + l * LP + (N2 + 1) * k1;
+        C x[N2];
 #pragma unroll
         for (int t = 0; t < N2; ++t) x[t] = p[t];
         sdft<N2, -1, 0, 1>(x);
-        float2 *q = B + l * LP;
+        C *q = B + l * LP;
         sfor<0, N2>([&](auto mc) {
             const int k = k1 + N1 * decltype(mc)::v;
             q[k + k / N2] = x[dft_pos(N2, decltype(mc)::v)];
@@ -805,7 +810,7 @@ __device__ void xg_unit_f32(const RveDesc &d, int kc, int unit)
     if (!first) {
         Idx3 il(tid, nthr, kc, L);
         for (int i = tid; i < 3 * L * kc; i += nthr, il.next())
-            cp_async8(A + i, aacc + il.a2 * cstride + kb + (long long)il.a1 * ny + il.a0);
+            cp_asyncc(A + i, aacc + il.a2 * cstride + kb + (long long)il.a1 * ny + il.a0);
         cp_async_wait_all();
         __syncthreads();
     }
@@ -813,22 +818,22 @@ __device__ void xg_unit_f32(const RveDesc &d, int kc, int unit)
     Idx3 ig(tid, nthr, kc, kIdxUnbounded);
     for (int idx = tid; idx < L * kc; idx += nthr, ig.next()) {
         const int yl = ig.a0, x = ig.a1, px = x + x / N2;
-        float br[6], bi[6], ar[3], ai[3];
+        R br[6], bi[6], ar[3], ai[3];
 #pragma unroll
         for (int c = 0; c < 6; ++c) {
-            const float2 e = B[(c * kc + yl) * LP + px];
+            const C e = B[(c * kc + yl) * LP + px];
             br[c] = e.x;
             bi[c] = e.y;
         }
         const long long o = kb + (long long)x * ny + yl;
-        green_apply<float>(d, x, y0 + yl, kz, o, br, bi, ar, ai);
+        green_apply<R>(d, x, y0 + yl, kz, o, br, bi, ar, ai);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) B[(c * kc + yl) * LP + px] = make_float2(br[c], bi[c]);
+        for (int c = 0; c < 6; ++c) B[(c * kc + yl) * LP + px] = mkc<C>(br[c], bi[c]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            float2 e = make_float2(ar[c], ai[c]);
+            C e = mkc<C>(ar[c], ai[c]);
             if (!first) {
-                const float2 a = A[(c * L + x) * kc + yl];
+                const C a = A[(c * L + x) * kc + yl];
                 e.x += a.x;
                 e.y += a.y;
             }
@@ -836,7 +841,7 @@ __device__ void xg_unit_f32(const RveDesc &d, int kc, int unit)
         }
     }
     __syncthreads();
-    xg_pass1<N1, N2, 1>(B, NL, tw);
+    xg_pass1<C, N1, N2, 1>(B, NL, tw);
     __syncthreads();
     // inverse pass 2: tasks (l, k1), l fastest, written to spectrum line l
     {
@@ -844,13 +849,13 @@ __device__ void xg_unit_f32(const RveDesc &d, int kc, int unit)
         const int dl = nthr % NL, dk = nthr / NL;
         int l = tid % NL, k1 = tid / NL;
         for (int task = tid; task < NL * N1; task += nthr) {
-            const float2 *p = B + l * LP + (N2 + 1) * k1;
-            float2 x[N2];
+            const C *p = B + l * LP + (N2 + 1) * k1;
+            C x[N2];
 #pragma unroll
             for (int t = 0; t < N2; ++t) x[t] = p[t];
             sdft<N2, 1, 0, 1>(x);
             const int c = l / kc, yl = l - c * kc;
-            float2 *g = spec + c * cstride + kb + yl + (long long)k1 * ny;
+            C *g = spec + c * cstride + kb + yl + (long long)k1 * ny;
             sfor<0, N2>([&](auto mc) { g[decltype(mc)::v * sN] = x[dft_pos(N2, decltype(mc)::v)]; });
             l += dl;
             k1 += dk;
@@ -859,10 +864,11 @@ __device__ void xg_unit_f32(const RveDesc &d, int kc, int unit)
     }
 }
 
-// smem of xg_unit_f32, bytes
-__host__ __device__ inline size_t xg32_smem(int nx, int n1, int kc)
+// smem of xg_unit, bytes
+template <typename C>
+__host__ __device__ inline size_t xg_smem(int nx, int n1, int kc)
 {
-    return 2 * sizeof(float2) * (size_t)(6 * kc) * (size_t)(nx + n1 + 1);
+    return 2 * sizeof(C) * (size_t)(6 * kc) * (size_t)(nx + n1 + 1);
 }
 
 template <typename R>
@@ -975,14 +981,232 @@ __device__ void fft_z_inv_dgs_f32(const RveDesc &d, int rows, int unit)
     // the update val/N as a float product (exact for a power-of-two N):
     // one FP64-pipe operation fewer per value than a product in FP64
     const float inv = (float)d.inv_nv;
+    // no mean correction (a load given by its velocity gradient alone): one
+    // FP64 addition per value instead of two
+    bool mean = false;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) mean = mean || m->ddg6[c] != 0.0;
     // element (z, r, c) is dgs[c][vb + r * nz + z] = D[i]
     Idx3 iz(threadIdx.x, blockDim.x, nz, rows);
     for (int i = threadIdx.x; i < 6 * run; i += blockDim.x, iz.next()) {
         const int z = iz.a0, r = iz.a1, c = iz.a2;
         const float2 e = res[z * ldl + (c >> 1) * rows + r];
-        const double val = (double)(((c & 1) ? e.y : e.x) * inv);
-        d.dgs[(long long)c * nv + vb + (long long)r * nz + z] = D[i] + (m->ddg6[c] + val);
+        double val = f2d(((c & 1) ? e.y : e.x) * inv);
+        if (mean) val += m->ddg6[c];
+        d.dgs[(long long)c * nv + vb + (long long)r * nz + z] = D[i] + val;
     }
+}
+
+// ---------------------------------------------------------------------------
+// The z passes of an RVE on the register FFT along z.  A tile is rows lines of
+// y at one x; its 3 rows complex lines (two components each, line l = p rows +
+// r) are transformed in the layout of the y stream, element (l, i) at l LP +
+// i + i / N2.  Pass 1 takes its inputs straight from the staged data -- the
+// stress runs, converted on the way, or the half-spectrum columns, unpacked on
+// the way -- and the inverse pass 2 adds its outputs straight to the
+// displacement gradient, so that a line crosses shared memory once less in
+// each direction than through fft_lines and a tile needs two block barriers
+// fewer.  Everything is staged by asynchronous copies.
+// us per launch, forward / inverse, against the passes through fft_lines:
+// single precision 256^3 461 / 950 -> 376 / 645, 96^3 34 / 64 -> 28 / 42; FP64
+// 128^3 359 / 408 -> 321 / 329.  Those passes stay for the Stockham stages.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float from_double(double x, float) { return d2f_rn(x); }
+__device__ __forceinline__ double from_double(double x, double) { return x; }
+
+template <typename C, int N1, int N2>
+__device__ void zf_unit(const RveDesc &d, int rows, int unit)
+{
+    typedef typename RealOf<C>::T R;
+    constexpr int L = N1 * N2, LP = L + N1 + 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int NL = 3 * rows, run = rows * L, half_run = run / 2;
+    C *W = reinterpret_cast<C *>(smem_raw);
+    double *stage = reinterpret_cast<double *>(W + ((NL * LP + 1) & ~1));   // the six runs (z fastest)
+    C *res = reinterpret_cast<C *>(stage);                                  // then the transformed lines, at l (L + 1) + k
+    const int ny = d.ny, nzh = d.nzh, ytiles = ny / rows;
+    const int x = unit / ytiles, y0 = (unit - x * ytiles) * rows;
+    const long long nv = d.nv, vb = ((long long)x * ny + y0) * L;
+    const C *tw = (const C *)d.twz;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    {
+        Idx3 ic(tid, nthr, half_run, kIdxUnbounded);
+        for (int i = tid; i < 6 * half_run; i += nthr, ic.next())
+            cp_async16(stage + 2 * i, d.sig + ic.a1 * nv + vb + 2 * ic.a0);
+        cp_async_wait_all();
+    }
+    __syncthreads();
+    for (int task = tid; task < NL * N2; task += nthr) {
+        const int l = task / N2, t = task - l * N2, p = l / rows, r = l - p * rows;
+        const double *a = stage + 2 * p * run + r * L + t;
+        C v[N1];
+        sfor<0, N1>([&](auto jc) {
+            constexpr int j = decltype(jc)::v;
+            v[j] = mkc<C>(from_double(a[j * N2], R(0)), from_double(a[run + j * N2], R(0)));
+        });
+        sdft<N1, -1, 0, 1>(v);
+        if (t != 0) {
+            const C *wm = tw + L + t;   // the pass-1 twiddle matrix
+            sfor<1, N1>([&](auto kc) {
+                constexpr int k = decltype(kc)::v, q = dft_pos(N1, k);
+                v[q] = cmul<R>(v[q], __ldg(wm + k * N2));
+            });
+        }
+        C *w = W + l * LP + t;
+        sfor<0, N1>([&](auto kc) { w[(N2 + 1) * decltype(kc)::v] = v[dft_pos(N1, decltype(kc)::v)]; });
+    }
+    __syncthreads();
+    for (int task = tid; task < NL * N1; task += nthr) {
+        const int l = task / N1, k1 = task - l * N1;
+        const C *w = W + l * LP + (N2 + 1) * k1;
+        C v[N2];
+#pragma unroll
+        for (int t = 0; t < N2; ++t) v[t] = w[t];
+        sdft<N2, -1, 0, 1>(v);
+        C *q = res + l * (L + 1) + k1;
+        sfor<0, N2>([&](auto mc) { q[N1 * decltype(mc)::v] = v[dft_pos(N2, decltype(mc)::v)]; });
+    }
+    __syncthreads();
+    C *spec = (C *)d.spec;
+    const long long plane = (long long)d.nx * ny;
+    Idx3 ix(tid, nthr, rows, nzh);
+    for (int i = tid; i < 3 * rows * nzh; i += nthr, ix.next()) {
+        const int r = ix.a0, k = ix.a1, p = ix.a2;
+        const C *q = res + (p * rows + r) * (L + 1);
+        const C zk = q[k], zm = q[k ? L - k : 0];
+        const long long o = (long long)k * plane + (long long)x * ny + y0 + r;
+        spec[(long long)(2 * p) * nzh * plane + o] = mkc<C>(R(0.5) * (zk.x + zm.x), R(0.5) * (zk.y - zm.y));
+        spec[(long long)(2 * p + 1) * nzh * plane + o] = mkc<C>(R(0.5) * (zk.y + zm.y), R(-0.5) * (zk.x - zm.x));
+    }
+}
+
+template <typename C>
+__host__ __device__ inline size_t zf_smem(int nz, int n1, int rows)
+{
+    const size_t w = (((size_t)(3 * rows) * (nz + n1 + 1) + 1) & ~(size_t)1) * sizeof(C);
+    const size_t st = sizeof(double) * 6 * (size_t)rows * nz, res = sizeof(C) * (size_t)(3 * rows) * (nz + 1);
+    return w + (st > res ? st : res);
+}
+
+// the inverse pass into the symmetric displacement gradient (evolution.c:383-394)
+template <bool MEAN>
+__device__ __forceinline__ double add_update(double old, float v, float inv, double m)
+{
+    const double x = f2d(v * inv);   // (the product exact for a power-of-two number of voxels)
+    return MEAN ? old + (x + m) : old + x;
+}
+template <bool MEAN>
+__device__ __forceinline__ double add_update(double old, double v, double inv, double m)
+{
+    return MEAN ? old + fma(v, inv, m) : fma(v, inv, old);
+}
+
+// pass 2 of zi_unit; MEAN: the update has a mean part (MacroDev::ddg6)
+template <typename C, int N1, int N2, bool MEAN>
+__device__ __forceinline__ void zi_pass2(const RveDesc &d, const C *W, const double *D, int rows, long long vb)
+{
+    typedef typename RealOf<C>::T R;
+    constexpr int L = N1 * N2, LP = L + N1 + 1;
+    const int run = rows * L;
+    const long long nv = d.nv;
+    const MacroDev *m = d.macro;
+    const R inv = (R)d.inv_nv;
+    for (int task = threadIdx.x; task < 3 * rows * N1; task += blockDim.x) {
+        const int l = task / N1, k1 = task - l * N1, p = l / rows, r = l - p * rows;
+        const C *w = W + l * LP + (N2 + 1) * k1;
+        C v[N2];
+#pragma unroll
+        for (int t = 0; t < N2; ++t) v[t] = w[t];
+        sdft<N2, 1, 0, 1>(v);
+        const double *o = D + 2 * p * run + r * L + k1;
+        double *g = d.dgs + 2 * p * nv + vb + r * L + k1;
+        const double m0 = MEAN ? m->ddg6[2 * p] : 0.0, m1 = MEAN ? m->ddg6[2 * p + 1] : 0.0;
+        sfor<0, N2>([&](auto mc) {
+            constexpr int q = N1 * decltype(mc)::v, e = dft_pos(N2, decltype(mc)::v);
+            g[q] = add_update<MEAN>(o[q], v[e].x, inv, m0);
+            g[nv + q] = add_update<MEAN>(o[run + q], v[e].y, inv, m1);
+        });
+    }
+}
+
+template <typename C, int N1, int N2>
+__device__ void zi_unit(const RveDesc &d, int rows, int unit)
+{
+    typedef typename RealOf<C>::T R;
+    constexpr int L = N1 * N2, LP = L + N1 + 1, nzh = L / 2 + 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int NL = 3 * rows, run = rows * L, half_run = run / 2;
+    C *W = reinterpret_cast<C *>(smem_raw);
+    double *D = reinterpret_cast<double *>(W + ((NL * LP + 1) & ~1));   // the old gradient: six runs (z fastest)
+    C *S = reinterpret_cast<C *>(D + 6 * run);                          // columns: S[(c nzh + k) rows + r]
+    const int ny = d.ny, ytiles = ny / rows;
+    const int x = unit / ytiles, y0 = (unit - x * ytiles) * rows;
+    const long long nv = d.nv, xy = (long long)x * ny + y0, vb = xy * L;
+    const long long plane = (long long)d.nx * ny, cstride = (long long)nzh * plane;
+    const C *spec = (const C *)d.spec, *tw = (const C *)d.twz;
+    const int tid = threadIdx.x, nthr = blockDim.x;
+    {
+        Idx3 is(tid, nthr, rows, nzh);   // (r, k, c)
+        for (int i = tid; i < 6 * nzh * rows; i += nthr, is.next())
+            cp_asyncc(S + i, spec + is.a2 * cstride + (long long)is.a1 * plane + xy + is.a0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        Idx3 ic(tid, nthr, half_run, kIdxUnbounded);
+        for (int i = tid; i < 6 * half_run; i += nthr, ic.next())
+            cp_async16(D + 2 * i, d.dgs + ic.a1 * nv + vb + 2 * ic.a0);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+    }
+    __syncthreads();
+    {
+        const int dl = nthr % NL, dt = nthr / NL;
+        int l = tid % NL, t = tid / NL;
+        for (int task = tid; task < NL * N2; task += nthr) {
+            const int p = l / rows, r = l - p * rows;
+            const C *a = S + (long long)2 * p * nzh * rows + r, *b = a + nzh * rows;
+            C v[N1];
+            sfor<0, N1>([&](auto jc) {
+                constexpr int j = decltype(jc)::v;
+                constexpr bool hi = j >= N1 / 2;   // coefficient k = t + N2 j: k >= L / 2
+                const int k = hi ? L - t - N2 * j : t + N2 * j;
+                C A = a[k * rows], B = b[k * rows];
+                if (hi) { A.y = -A.y; B.y = -B.y; }
+                if ((j == 0 || j == N1 / 2) && t == 0) { A.y = R(0); B.y = R(0); }
+                v[j] = mkc<C>(A.x - B.y, A.y + B.x);
+            });
+            sdft<N1, 1, 0, 1>(v);
+            if (t != 0) {
+                const C *wm = tw + L + t;
+                sfor<1, N1>([&](auto kc) {
+                    constexpr int k = decltype(kc)::v, q = dft_pos(N1, k);
+                    C w = __ldg(wm + k * N2);
+                    w.y = -w.y;
+                    v[q] = cmul<R>(v[q], w);
+                });
+            }
+            C *w = W + l * LP + t;
+            sfor<0, N1>([&](auto kc) { w[(N2 + 1) * decltype(kc)::v] = v[dft_pos(N1, decltype(kc)::v)]; });
+            l += dl;
+            t += dt;
+            if (l >= NL) { l -= NL; ++t; }
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    // no mean correction (a load given by its velocity gradient alone): one
+    // FP64 operation per value fewer
+    const double *g6 = d.macro->ddg6;
+    long long any = 0;
+#pragma unroll
+    for (int c = 0; c < 6; ++c) any |= __double_as_longlong(g6[c]) << 1;   // (but for the sign)
+    if (any) zi_pass2<C, N1, N2, true>(d, W, D, rows, vb);
+    else zi_pass2<C, N1, N2, false>(d, W, D, rows, vb);
+}
+
+template <typename C>
+__host__ __device__ inline size_t zi_smem(int nz, int n1, int rows)
+{
+    return (((size_t)(3 * rows) * (nz + n1 + 1) + 1) & ~(size_t)1) * sizeof(C) + sizeof(double) * 6 * (size_t)rows * nz +
+           sizeof(C) * 6 * (size_t)(nz / 2 + 1) * rows;
 }
 
 // inverse z transform (Hermitian half spectrum -> real); mode 0 adds the
@@ -2884,6 +3108,21 @@ template <> struct FftGrid<double> { static constexpr int v = 2 * kFft64Blocks; 
 #ifndef VOCE_FFTZ32_BLOCKS
 #define VOCE_FFTZ32_BLOCKS 2
 #endif
+// CALL(N1, N2) for the register FFT's split of length L
+#define VOCE_REG_SPLITS(L, CALL) \
+    switch (L) { \
+    case 16: CALL(4, 4); break; \
+    case 24: CALL(4, 6); break; \
+    case 32: CALL(4, 8); break; \
+    case 48: CALL(6, 8); break; \
+    case 64: CALL(8, 8); break; \
+    case 96: CALL(8, 12); break; \
+    case 128: CALL(8, 16); break; \
+    case 192: CALL(12, 16); break; \
+    case 256: CALL(16, 16); break; \
+    default: break; \
+    }
+
 template <typename R>
 __global__ void __launch_bounds__(FftThreads<R>::v, sizeof(R) == 4 ? VOCE_FFTZ32_BLOCKS : kFft64Blocks)
 kb_fft_z_fwd(const RveDesc *descs, const int2 *map, int total)
@@ -2892,37 +3131,46 @@ kb_fft_z_fwd(const RveDesc *descs, const int2 *map, int total)
         const int2 e = map[w];
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, MASK_ACTIVE)) continue;
-        fft_z_fwd_unit<R>(d, d.zrows, e.y);
+        typedef typename Cx<R>::T C;
+        if (d.plz.n1 > 0) {
+#define VOCE_CALL(N1, N2) zf_unit<C, N1, N2>(d, d.zrows, e.y)
+            VOCE_REG_SPLITS(d.nz, VOCE_CALL)
+#undef VOCE_CALL
+        } else {
+            fft_z_fwd_unit<R>(d, d.zrows, e.y);
+        }
         __syncthreads();
     }
 }
 
 // which: 0 spectrum forward, 1 spectrum inverse, 2 antisymmetric accumulator inverse
 // cp.async of a y tile (NL lines of L contiguous coefficients at g) into the
-// stream layout; with 256 threads and L dividing 256 a thread keeps its
+// stream layout; where L divides the number of threads a thread keeps its
 // coefficient index and steps by whole lines
-template <int N1, int N2>
-__device__ __forceinline__ void ystream_issue(float2 *A, const float2 *g, int NL)
+template <typename C, int N1, int N2, int NT>
+__device__ __forceinline__ void ystream_issue(C *A, const C *g, int NL)
 {
     constexpr int L = N1 * N2, LP = L + N1 + 1;
-    if (256 % L == 0 && blockDim.x == 256) {
-        constexpr int dl = 256 % L == 0 ? 256 / L : 1;
+    if constexpr (NT % L == 0) {   // (NT threads)
+        constexpr int dl = NT / L;
         const int i = threadIdx.x % L;
-        float2 *s = A + (threadIdx.x / L) * LP + i + i / N2;
-        const float2 *src = g + threadIdx.x;
-        for (int l = threadIdx.x / L; l < NL; l += dl, s += dl * LP, src += 256) cp_async8(s, src);
+        C *s = A + (threadIdx.x / L) * LP + i + i / N2;
+        const C *src = g + threadIdx.x;
+        for (int l = threadIdx.x / L; l < NL; l += dl, s += dl * LP, src += NT) cp_asyncc(s, src);
     } else {
         for (int e = threadIdx.x; e < NL * L; e += blockDim.x) {
             const int l = e / L, i = e - l * L;
-            cp_async8(A + l * LP + i + i / N2, g + e);
+            cp_asyncc(A + l * LP + i + i / N2, g + e);
         }
     }
 }
 
-__device__ void fft_y_stream_f32(const RveDesc *descs, const int2 *map, int total, int which, int S)
+template <typename R>
+__device__ void fft_y_stream(const RveDesc *descs, const int2 *map, int total, int which, int S)
 {
+    typedef typename Cx<R>::T C;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2 *cur = reinterpret_cast<float2 *>(smem_raw), *nxt = cur + S;
+    C *cur = reinterpret_cast<C *>(smem_raw), *nxt = cur + S;
     const int mask = which == 2 ? MASK_CONVERGED : MASK_ACTIVE;
     const int sign = which == 0 ? -1 : +1;
     auto next_on = [&](int w) {
@@ -2930,30 +3178,21 @@ __device__ void fft_y_stream_f32(const RveDesc *descs, const int2 *map, int tota
         return w;
     };
     // the unit's RVE, its spectrum (y lines: contiguous) and tile base
-    auto tile = [&](int w, const RveDesc *&dp, float2 *&g) {
+    auto tile = [&](int w, const RveDesc *&dp, C *&g) {
         const int2 e = map[w];
         dp = &descs[e.x];
         const RveDesc &d = *dp;
         const int xtiles = d.nx / d.yxt;
         const int line = e.y / xtiles, x0 = (e.y % xtiles) * d.yxt;
-        g = (float2 *)(which == 2 ? d.aacc : d.spec) + ((long long)line * d.nx + x0) * d.ny;
+        g = (C *)(which == 2 ? d.aacc : d.spec) + ((long long)line * d.nx + x0) * d.ny;
     };
-    auto issue = [&](int w, float2 *A) {
+    auto issue = [&](int w, C *A) {
         const RveDesc *dp;
-        float2 *g;
+        C *g;
         tile(w, dp, g);
-        switch (dp->ny) {
-        case 16: ystream_issue<4, 4>(A, g, dp->yxt); break;
-        case 24: ystream_issue<4, 6>(A, g, dp->yxt); break;
-        case 32: ystream_issue<4, 8>(A, g, dp->yxt); break;
-        case 48: ystream_issue<6, 8>(A, g, dp->yxt); break;
-        case 64: ystream_issue<8, 8>(A, g, dp->yxt); break;
-        case 96: ystream_issue<8, 12>(A, g, dp->yxt); break;
-        case 128: ystream_issue<8, 16>(A, g, dp->yxt); break;
-        case 192: ystream_issue<12, 16>(A, g, dp->yxt); break;
-        case 256: ystream_issue<16, 16>(A, g, dp->yxt); break;
-        default: break;
-        }
+#define VOCE_CALL(N1, N2) ystream_issue<C, N1, N2, FftThreads<R>::v>(A, g, dp->yxt)
+        VOCE_REG_SPLITS(dp->ny, VOCE_CALL)
+#undef VOCE_CALL
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     int w = next_on(blockIdx.x);
@@ -2968,30 +3207,21 @@ __device__ void fft_y_stream_f32(const RveDesc *descs, const int2 *map, int tota
         }
         __syncthreads();
         const RveDesc *dp;
-        float2 *g;
+        C *g;
         tile(w, dp, g);
-        const float2 *tw = (const float2 *)dp->twy;
+        const C *tw = (const C *)dp->twy;
         const int NL = dp->yxt;
-#define VOCE_YSTREAM(L_, N1_) \
-    case L_: \
-        if (sign < 0) ystream_tile<N1_, L_ / N1_, -1>(cur, NL, g, tw); \
-        else ystream_tile<N1_, L_ / N1_, 1>(cur, NL, g, tw); \
-        break;
-        switch (dp->ny) {
-        VOCE_YSTREAM(16, 4)
-        VOCE_YSTREAM(24, 4)
-        VOCE_YSTREAM(32, 4)
-        VOCE_YSTREAM(48, 6)
-        VOCE_YSTREAM(64, 8)
-        VOCE_YSTREAM(96, 8)
-        VOCE_YSTREAM(128, 8)
-        VOCE_YSTREAM(192, 12)
-        VOCE_YSTREAM(256, 16)
-        default: break;
+        if (sign < 0) {
+#define VOCE_CALL(N1, N2) ystream_tile<C, N1, N2, -1>(cur, NL, g, tw)
+            VOCE_REG_SPLITS(dp->ny, VOCE_CALL)
+#undef VOCE_CALL
+        } else {
+#define VOCE_CALL(N1, N2) ystream_tile<C, N1, N2, 1>(cur, NL, g, tw)
+            VOCE_REG_SPLITS(dp->ny, VOCE_CALL)
+#undef VOCE_CALL
         }
-#undef VOCE_YSTREAM
         __syncthreads();
-        float2 *t = cur; cur = nxt; nxt = t;
+        C *t = cur; cur = nxt; nxt = t;
         w = nw;
     }
 }
@@ -3008,11 +3238,9 @@ template <typename R>
 __global__ void __launch_bounds__(FftThreads<R>::v, sizeof(R) == 4 ? VOCE_FFTY32_BLOCKS : kFft64Blocks)
 kb_fft_y(const RveDesc *descs, const int2 *map, int total, int which, int stream)
 {
-    if constexpr (sizeof(R) == 4) {
-        if (stream > 0) {
-            fft_y_stream_f32(descs, map, total, which, stream);
-            return;
-        }
+    if (stream > 0) {
+        fft_y_stream<R>(descs, map, total, which, stream);
+        return;
     }
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int2 e = map[w];
@@ -3034,25 +3262,14 @@ kb_fft_x_green(const RveDesc *descs, const int2 *map, int total)
         const int2 e = map[w];
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, MASK_ACTIVE)) continue;
-        bool done = false;
-        if constexpr (sizeof(R) == 4) {
-            if (d.plx.n1 > 0) {
-                done = true;
-                switch (d.nx) {
-                case 16: xg_unit_f32<4, 4>(d, d.xkc, e.y); break;
-                case 24: xg_unit_f32<4, 6>(d, d.xkc, e.y); break;
-                case 32: xg_unit_f32<4, 8>(d, d.xkc, e.y); break;
-                case 48: xg_unit_f32<6, 8>(d, d.xkc, e.y); break;
-                case 64: xg_unit_f32<8, 8>(d, d.xkc, e.y); break;
-                case 96: xg_unit_f32<8, 12>(d, d.xkc, e.y); break;
-                case 128: xg_unit_f32<8, 16>(d, d.xkc, e.y); break;
-                case 192: xg_unit_f32<12, 16>(d, d.xkc, e.y); break;
-                case 256: xg_unit_f32<16, 16>(d, d.xkc, e.y); break;
-                default: done = false; break;
-                }
-            }
+        typedef typename Cx<R>::T C;
+        if (d.plx.n1 > 0) {
+#define VOCE_CALL(N1, N2) xg_unit<C, N1, N2>(d, d.xkc, e.y)
+            VOCE_REG_SPLITS(d.nx, VOCE_CALL)
+#undef VOCE_CALL
+        } else {
+            fft_x_green_unit<R>(d, d.xkc, e.y);
         }
-        if (!done) fft_x_green_unit<R>(d, d.xkc, e.y);
         __syncthreads();
     }
 }
@@ -3078,7 +3295,12 @@ kb_fft_z_inv(const RveDesc *descs, const int2 *map, int total, int mode)
         const int2 e = map[w];
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, mode == 0 ? MASK_ACTIVE : MASK_CONVERGED)) continue;
-        if (mode == 0) {
+        typedef typename Cx<R>::T C;
+        if (mode == 0 && d.plz.n1 > 0) {
+#define VOCE_CALL(N1, N2) zi_unit<C, N1, N2>(d, d.zirows, e.y)
+            VOCE_REG_SPLITS(d.nz, VOCE_CALL)
+#undef VOCE_CALL
+        } else if (mode == 0) {
             if constexpr (sizeof(R) == 4) fft_z_inv_dgs_f32(d, d.zirows, e.y);
             else fft_z_inv_unit<R>(d, d.spec, 6, d.zirows, 0, e.y);
         } else {
@@ -3273,10 +3495,14 @@ void batch_units(const RveDesc &d, int u[BP_COUNT])
 template <typename R>
 static size_t batch_smem_t(const RveDesc &d, int ph)
 {
-    if (sizeof(R) == 4) {   // the staged single-precision z passes, the register-FFT Green pass
+    typedef typename Cx<R>::T C;
+    // the register-FFT z and Green passes, the staged single-precision z passes
+    if (ph == BP_ZF && d.plz.n1 > 0) return zf_smem<C>(d.nz, d.plz.n1, d.zrows);
+    if (ph == BP_ZI && d.plz.n1 > 0) return zi_smem<C>(d.nz, d.plz.n1, d.zirows);
+    if (ph == BP_XG && d.plx.n1 > 0) return xg_smem<C>(d.nx, d.plx.n1, d.xkc);
+    if (sizeof(R) == 4) {
         if (ph == BP_ZF) return sizeof(float2) * (size_t)zf32_fwd_size(d.nz, d.zrows);
         if (ph == BP_ZI) return sizeof(float2) * (size_t)zi32_size(d.nz, d.nzh, d.zirows);
-        if (ph == BP_XG && d.plx.n1 > 0) return xg32_smem(d.nx, d.plx.n1, d.xkc);
     }
     switch (ph) {
     case BP_ZF: return smem_lines<R>(d.nz, 3 * d.zrows);
@@ -3496,7 +3722,6 @@ int tile_candidates(const RveDesc &d, int phase, int *out, int max)
 {
     const bool f = d.mixed != 0;
     const int B = f ? 4096 : 2048;
-    const size_t cs = f ? sizeof(float2) : sizeof(double2);
     const size_t smem_max = 200 * 1024;
     int n = 0;
     // from the largest down, and below a quarter of the budget only while a
@@ -3508,23 +3733,15 @@ int tile_candidates(const RveDesc &d, int phase, int *out, int max)
         const int budget = k < 0 ? (B >> -k) : (B << k);
         if (k < -2 && n > 0 && tile_units(d, phase, out[n - 1]) >= 2 * 152) break;
         int t = 0;
-        size_t sm = 0;
+        RveDesc dt = d;
         switch (phase) {
-        case BP_ZF:
-            t = pick_div<double>(d.ny, budget / (3 * d.nz));
-            sm = f ? cs * (size_t)zf32_fwd_size(d.nz, t) : 2 * (size_t)d.nz * ((3 * t) | 1) * cs;
-            break;
-        case BP_Y6: t = pick_div<double>(d.nx, budget / d.ny); sm = 2 * (size_t)d.ny * (t | 1) * cs; break;
-        case BP_XG:
-            t = pick_div<double>(d.ny, (budget * 3 / 2) / (6 * d.nx));
-            sm = (f && d.plx.n1 > 0) ? xg32_smem(d.nx, d.plx.n1, t) : 2 * (size_t)d.nx * ((6 * t) | 1) * cs;
-            break;
-        case BP_ZI:
-            t = pick_div<double>(d.ny, budget / (3 * d.nz));
-            sm = f ? cs * (size_t)zi32_size(d.nz, d.nzh, t) : 2 * (size_t)d.nz * ((3 * t) | 1) * cs;
-            break;
+        case BP_ZF: t = dt.zrows = pick_div<double>(d.ny, budget / (3 * d.nz)); break;
+        case BP_Y6: t = dt.yxt = pick_div<double>(d.nx, budget / d.ny); break;
+        case BP_XG: t = dt.xkc = pick_div<double>(d.ny, (budget * 3 / 2) / (6 * d.nx)); break;
+        case BP_ZI: t = dt.zirows = pick_div<double>(d.ny, budget / (3 * d.nz)); break;
         default: return 0;
         }
+        const size_t sm = batch_smem(dt, phase);
         if (t < 1 || sm > smem_max) continue;
         bool seen = false;
         for (int i = 0; i < n; ++i) seen = seen || out[i] == t;
