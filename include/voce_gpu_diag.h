@@ -97,9 +97,9 @@ int voce_rve_set_tiles(voce_rve *r, const int tiles[6]);
  * 256 has one more candidate, placed first: the register FFT, two passes of
  * small DFTs of lengths N1 x N2 = L held in registers (4x4, 4x6, 4x8, 6x8,
  * 8x8, 8x12, 8x16, 12x16, 16x16).  Candidate 0 is the default.
- * In the FP64 form candidate 0 of those lengths is computed by the register
- * FFT too (fewer operations in the same two passes); it is counted and
- * reported as the default Stockham order.
+ * In the FP64 form candidate 0 of those lengths, and in every form candidate 0
+ * of 8, 12, 18, 27, 36, 54, 72, 81, 108 and 144, is computed by the register
+ * FFT too; it is counted and reported as the default Stockham order.
  * Unlike the tiles, the schedule changes results in the last bits (a
  * different order of roundings).  So the FP64 form never tunes it: its RVEs
  * run the default schedule of every axis unless the caller sets one, and its

@@ -233,10 +233,10 @@ int fft_schedules(int L, FftPlan1 *out, int max)
 
 // Transform candidates of an axis of an RVE: for the single-precision
 // spectrum forms, the register FFT first where the length has one
-// (reg_fft_split), then the Stockham schedules; for the FP64 form, the
-// Stockham schedules only, of which candidate 0 runs as the register FFT
-// where the length has one (and is still reported by its radices).
-// Candidate 0 is the default.
+// (reg_fft_split), then the Stockham schedules; for the FP64 form and the
+// other lengths, the Stockham schedules only, of which candidate 0 runs as the
+// register FFT where the length has one (reg_fft_any; it is still reported by
+// its radices).  Candidate 0 is the default.
 int axis_schedules(int L, bool mixed, FftPlan1 *out, int max)
 {
     int n = 0;
@@ -245,7 +245,7 @@ int axis_schedules(int L, bool mixed, FftPlan1 *out, int max)
         n = 1;
     }
     const int total = n + fft_schedules(L, out + n, max - n);
-    if (!mixed && total > 0) out[0].n1 = reg_fft_split(L);
+    if (n == 0 && total > 0) out[0].n1 = reg_fft_any(L);
     return total;
 }
 
@@ -339,7 +339,7 @@ void populate(void *p, size_t n)
 template <typename C, typename R>
 std::vector<C> twiddles(int L)
 {
-    const int n1 = reg_fft_split(L);
+    const int n1 = reg_fft_any(L);
     std::vector<C> t(n1 ? 2 * L : L);
     const long double two_pi = 6.283185307179586476925286766559005768L;
     auto w = [&](long long e, C &c) {
@@ -2063,7 +2063,7 @@ int voce_rve_get_fft_schedule(const voce_rve *r, int axis, int *radices, int max
 {
     if (!r || axis < 0 || axis > 2) return -fail(VOCE_ERR_ARG, "bad argument");
     const FftPlan1 &p = axis == 0 ? r->d.plx : axis == 1 ? r->d.ply : r->d.plz;
-    if (p.n1 > 0 && r->d.mixed) {   // the register FFT: its two passes
+    if (p.n1 > 0 && r->d.mixed && reg_fft_split(p.L)) {   // the register FFT: its two passes
         const int rr[2] = {p.n1, p.L / p.n1};
         for (int k = 0; k < 2 && k < max && radices; ++k) radices[k] = rr[k];
         return 2;

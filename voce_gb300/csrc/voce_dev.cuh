@@ -172,6 +172,17 @@ __host__ __device__ __forceinline__ void b_to_t6(const T *b, T *t)
     t[5] = T(RSQ2) * b[4];
 }
 
+// the 3x3 tensor (row-major) of a 6-vector
+__device__ __forceinline__ void sym9_from_b(const double *b6, double *t9)
+{
+    double t[6];
+    b_to_t6<double>(b6, t);
+    t9[0] = t[0]; t9[4] = t[1]; t9[8] = t[2];
+    t9[5] = t9[7] = t[3];
+    t9[2] = t9[6] = t[4];
+    t9[1] = t9[3] = t[5];
+}
+
 // packed upper-triangle index of a symmetric 6x6
 __host__ __device__ __forceinline__ int sym6(int i, int j)
 {
@@ -860,6 +871,27 @@ __host__ __device__ inline int reg_fft_split(int L)
     }
 }
 
+// The split of every length the register FFT can run: the ones above, and the
+// others below 256 whose factors the small DFTs have (2, 3, 4, 6, 8, 9, 12,
+// 16; an even length has an even N1).  Those run it in place of the default
+// Stockham order, under that order's name.
+__host__ __device__ inline int reg_fft_any(int L)
+{
+    switch (L) {
+    case 8: return 4;     // 4 x 2
+    case 12: return 4;    // 4 x 3
+    case 18: return 6;    // 6 x 3
+    case 27: return 3;    // 3 x 9
+    case 36: return 6;    // 6 x 6
+    case 54: return 6;    // 6 x 9
+    case 72: return 8;    // 8 x 9
+    case 81: return 9;    // 9 x 9
+    case 108: return 12;  // 12 x 9
+    case 144: return 12;  // 12 x 12
+    default: return reg_fft_split(L);
+    }
+}
+
 // cos(2 pi a / 48) for 0 <= a <= 12.  The small DFTs (N dividing 48) meet
 // only angles a that are multiples of 3 (N = 16) or 4 (N = 12); the values
 // are cos 0, cos pi/8 = sqrt(2 + sqrt 2) / 2, cos pi/6 = sqrt 3 / 2,
@@ -904,6 +936,13 @@ template <int N, int E, int S, typename C>
 __device__ __forceinline__ C rot(C v)
 {
     typedef typename RealOf<C>::T R;
+    if constexpr (N == 9) {
+        // exp(2 pi i E / 9) for the exponents of its 3 x 3 split
+        static_assert(E == 1 || E == 2 || E == 4, "angle without a constant");
+        constexpr R c = (R)(E == 1 ? 0.76604444311897803520 : E == 2 ? 0.17364817766693034885 : -0.93969262078590838405);
+        constexpr R s = (R)(S * (E == 1 ? 0.64278760968653932632 : E == 2 ? 0.98480775301220805937 : 0.34202014332566873304));
+        return mkc<C>(fma_(-s, v.y, c * v.x), fma_(s, v.x, c * v.y));
+    } else {
     static_assert(48 % N == 0, "small DFT lengths divide 48");
     constexpr int a = (48 / N * E) % 48;
     static_assert(a % 3 == 0 || a % 4 == 0, "angle without a constant");
@@ -920,6 +959,7 @@ __device__ __forceinline__ C rot(C v)
         constexpr R c = (R)cos48(a), s = (R)(S * sin48(a));
         return mkc<C>(fma_(-s, v.y, c * v.x), fma_(s, v.x, c * v.y));
     }
+    }
 }
 
 // The small DFTs run in place on a strided view of a register array, the
@@ -927,11 +967,12 @@ __device__ __forceinline__ C rot(C v)
 // view element dft_pos(N, q) (the four-step split transposes; placing the
 // outputs in the registers the inputs came from needs no temporaries, and
 // the caller indexes the permutation at compile time).
+__host__ __device__ constexpr int dft_first(int N) { return N % 4 == 0 ? 4 : N % 2 == 0 ? 2 : 3; }
 __host__ __device__ constexpr int dft_pos(int N, int q)
 {
     return N <= 4 ? q
-                  : dft_pos(N / (N % 4 == 0 ? 4 : 2), q / (N % 4 == 0 ? 4 : 2)) +
-                        N / (N % 4 == 0 ? 4 : 2) * dft_pos(N % 4 == 0 ? 4 : 2, q % (N % 4 == 0 ? 4 : 2));
+                  : dft_pos(N / dft_first(N), q / dft_first(N)) +
+                        N / dft_first(N) * dft_pos(dft_first(N), q % dft_first(N));
 }
 
 // X[q] = sum_n x[n] exp(S 2 pi i n q / N) over the view, X[q] left in view
@@ -970,7 +1011,7 @@ __device__ __forceinline__ void sdft(C (&x)[M])
             x[O + 3 * T] = mkc<C>(t1.x + t3.y, t1.y - t3.x);
         }
     } else {
-        constexpr int A = N % 4 == 0 ? 4 : 2, B = N / A;
+        constexpr int A = dft_first(N), B = N / A;
         sfor<0, B>([&](auto tc) { sdft<A, S, O + T * decltype(tc)::v, T * B>(x); });
         sfor<1, B>([&](auto tc) {
             constexpr int t = decltype(tc)::v;
@@ -1040,25 +1081,40 @@ __device__ C *fft_reg(C *a, C *b, int NL, int ldl, const C *__restrict__ tw)
     return b;
 }
 
+// CALL(N1, N2) for the register FFT's split of length L (reg_fft_any)
+#define VOCE_REG_SPLITS(L, CALL) \
+    switch (L) { \
+    case 8: CALL(4, 2); break; \
+    case 12: CALL(4, 3); break; \
+    case 16: CALL(4, 4); break; \
+    case 18: CALL(6, 3); break; \
+    case 24: CALL(4, 6); break; \
+    case 27: CALL(3, 9); break; \
+    case 32: CALL(4, 8); break; \
+    case 36: CALL(6, 6); break; \
+    case 48: CALL(6, 8); break; \
+    case 54: CALL(6, 9); break; \
+    case 64: CALL(8, 8); break; \
+    case 72: CALL(8, 9); break; \
+    case 81: CALL(9, 9); break; \
+    case 96: CALL(8, 12); break; \
+    case 108: CALL(12, 9); break; \
+    case 128: CALL(8, 16); break; \
+    case 144: CALL(12, 12); break; \
+    case 192: CALL(12, 16); break; \
+    case 256: CALL(16, 16); break; \
+    default: break; \
+    }
+
 template <typename C>
 __device__ __forceinline__ C *fft_reg_lines(C *a, C *b, int NL, int ldl, int L,
                                                  const C *__restrict__ tw, int sign)
 {
-#define VOCE_REG_FFT(L_, N1_) \
-    case L_: return sign < 0 ? fft_reg<N1_, L_ / N1_, -1, C>(a, b, NL, ldl, tw) : fft_reg<N1_, L_ / N1_, 1, C>(a, b, NL, ldl, tw);
-    switch (L) {
-    VOCE_REG_FFT(16, 4)
-    VOCE_REG_FFT(24, 4)
-    VOCE_REG_FFT(32, 4)
-    VOCE_REG_FFT(48, 6)
-    VOCE_REG_FFT(64, 8)
-    VOCE_REG_FFT(96, 8)
-    VOCE_REG_FFT(128, 8)
-    VOCE_REG_FFT(192, 12)
-    VOCE_REG_FFT(256, 16)
-    default: return nullptr;
-    }
-#undef VOCE_REG_FFT
+#define VOCE_CALL(N1, N2) \
+    return sign < 0 ? fft_reg<N1, N2, -1, C>(a, b, NL, ldl, tw) : fft_reg<N1, N2, 1, C>(a, b, NL, ldl, tw)
+    VOCE_REG_SPLITS(L, VOCE_CALL)
+#undef VOCE_CALL
+    return nullptr;
 }
 
 template <typename R>
@@ -1067,10 +1123,10 @@ __device__ typename Cx<R>::T *fft_lines(typename Cx<R>::T *a, typename Cx<R>::T 
                                         const typename Cx<R>::T *__restrict__ tw, int sign)
 {
     typedef typename Cx<R>::T C;
-    // the plan's split always matches reg_fft_split (the host sets both); an
+    // the plan's split always matches reg_fft_any (the host sets both); an
     // unknown length falls through to the Stockham stages, which the plan
     // also holds
-    if (pl.n1 && reg_fft_split(pl.L) == pl.n1) {
+    if (pl.n1 && reg_fft_any(pl.L) == pl.n1) {
         C *res = fft_reg_lines<C>(a, b, NL, ldl, pl.L, tw, sign);
         if (res) return res;
     }

@@ -11,6 +11,15 @@ struct SetupConst {
     double sc6[6];            // B-basis Scauchy (creep start stress, init.c:523-525)
 };
 
+// the largest divisor of n up to limit
+inline int pick_div(int n, int limit)
+{
+    int best = 1;
+    for (int k = 1; k <= n; ++k)
+        if (n % k == 0 && k <= limit) best = k;
+    return best;
+}
+
 // FFT tile sizes (lines per block) for one grid, and the radix schedule of
 // each axis (an index into fft_schedules' candidates of that axis' length)
 struct Tiles {
@@ -72,6 +81,16 @@ struct BatchPlan {
                           // pass streams its units through two tile buffers of
                           // this many complex floats
 };
+// The spectrum passes of a plan (float: single-precision spectrum): z forward,
+// y forward, x with the Green operator, y inverse, z inverse into DisGrad, and
+// the three inverse passes of the antisymmetric sum.
+enum FftPass { FFT_ZF, FFT_YF, FFT_XG, FFT_YI, FFT_ZI, FFT_X3, FFT_Y3, FFT_Z3 };
+template <typename R> void launch_fft(const BatchPlan &bp, FftPass pass, cudaStream_t s);
+template <> void launch_fft<float>(const BatchPlan &bp, FftPass pass, cudaStream_t s);
+template <> void launch_fft<double>(const BatchPlan &bp, FftPass pass, cudaStream_t s);
+template <typename R> cudaError_t set_fft_smem(const BatchPlan &bp);
+template <> cudaError_t set_fft_smem<float>(const BatchPlan &bp);
+template <> cudaError_t set_fft_smem<double>(const BatchPlan &bp);
 // units of one RVE in each phase
 void batch_units(const RveDesc &d, int units[BP_COUNT]);
 size_t batch_smem(const RveDesc &d, int phase);
