@@ -174,6 +174,22 @@ __device__ __forceinline__ void fcc_tangent12(const T (&h)[12], T (&J)[15])
     fcc_tangent<2, T>({h[8], h[9], h[10], h[11]}, J);
 }
 
+// |r[k]|^e by binary powering, out of line: the exponents other than 19 are
+// rare, and the loops of the twelve systems would sit between the hot
+// instructions
+template <int N, typename T>
+__device__ __noinline__ void fcc_pow_any(const T *r, int e, T *p)
+{
+    for (int k = 0; k < N; ++k) {
+        T b = sizeof(T) == 4 ? (T)fabsf((float)r[k]) : (T)fabs((double)r[k]), q = T(1);
+        for (int x = e; x; x >>= 1) {
+            if (x & 1) q *= b;
+            b *= b;
+        }
+        p[k] = q;
+    }
+}
+
 // p[k] = |r[k]|^e, e = n - 1.  The exponent is tested once for all N, so that
 // their loads and products stay in one straight run of instructions.
 template <int N, typename T>
@@ -186,19 +202,12 @@ __device__ __forceinline__ void fcc_pow(const T (&r)[N], int e, T (&p)[N])
             p[k] = (a16 * a2) * (sizeof(T) == 4 ? (T)fabsf((float)r[k]) : (T)fabs((double)r[k]));
         }
     } else {
-        T b[N];
+        T a[N], q[N];
 #pragma unroll
-        for (int k = 0; k < N; ++k) {
-            p[k] = T(1);
-            b[k] = sizeof(T) == 4 ? (T)fabsf((float)r[k]) : (T)fabs((double)r[k]);
-        }
-        for (; e; e >>= 1) {
+        for (int k = 0; k < N; ++k) a[k] = r[k];
+        fcc_pow_any<N, T>(a, e, q);
 #pragma unroll
-            for (int k = 0; k < N; ++k) {
-                if (e & 1) p[k] *= b[k];
-                b[k] *= b[k];
-            }
-        }
+        for (int k = 0; k < N; ++k) p[k] = q[k];
     }
 }
 
@@ -267,6 +276,45 @@ __device__ __forceinline__ bool fcc_edot_fp64(const RveDesc &d, long long v, con
         for (int k = 0; k < 12; ++k) r[k] *= p[k];
     }
     fcc_edot12<double>(r, E);
+    return big;
+}
+
+// The same family by family in one loop body, for the FP64 form, whose Newton
+// loop is long: fewer instructions to wait for (128^3 3.94 -> 3.79 ms per
+// launch; the mixed_ir form at 64^3 213 -> 218 us, so it keeps the run above)
+__device__ __forceinline__ bool fcc_edot_fp64_loop(const RveDesc &d, long long v, const double (&y)[5], double (&E)[5])
+{
+    bool big = false;
+#pragma unroll
+    for (int c = 0; c < 5; ++c) E[c] = 0.0;
+#pragma unroll 1
+    for (int z = 0; z < 3; ++z) {
+        const double D = (z == 0 ? y[0] : -y[0]) - (z == 2 ? y[0] : y[1]);
+        const double a = z == 2 ? y[3] : y[4], b = z == 0 ? y[3] : y[2], u = a + b, w = a - b;
+        double r[4] = {D + u, D - u, D + w, D - w};
+        const double *tau = d.itau + (long long)(8 * z) * d.nv + v;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] *= __ldg(tau + (long long)(2 * k + (__double2hiint(r[k]) < 0)) * d.nv);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) big = big || (__double2hiint(r[k]) & 0x7fffffff) >= 0x404E0000;
+        if (d.ipow_n == 20) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const double a2 = r[k] * r[k], a4 = a2 * a2, a5 = a4 * fabs(r[k]), a10 = a5 * a5, a20 = a10 * a10;
+                r[k] = __hiloint2double(__double2hiint(a20) | (__double2hiint(r[k]) & (int)0x80000000), __double2loint(a20));
+            }
+        } else {
+            double p[4];
+            fcc_pow<4, double>(r, d.ipow_n - 1, p);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[k] *= p[k];
+        }
+        const double G = (r[0] + r[1]) + (r[2] + r[3]), gu = r[0] - r[1], gw = r[2] - r[3];
+        const double ea = gu + gw, eb = gu - gw;
+        if (z == 0) { E[0] = G; E[1] = -G; E[4] = ea; E[3] = eb; }
+        else if (z == 1) { E[0] -= G; E[1] -= G; E[4] += ea; E[2] = eb; }
+        else { E[0] = fma(-2.0, G, E[0]); E[3] += ea; E[2] += eb; }
+    }
     return big;
 }
 
@@ -405,22 +453,6 @@ __device__ __forceinline__ ff32 ffs_sum(float a, float b)
     return r;
 }
 
-// the resolved shears of family Z as float pairs (y: exact floats)
-template <int Z>
-__device__ __forceinline__ void fcc_rss_ff(const float (&y)[5], ff32 *c)
-{
-    ff32 D;
-    if (Z == 0) D = ffs_sum(y[0], -y[1]);
-    else if (Z == 1) D = ffs_sum(-y[0], -y[1]);
-    else { D.h = -2.0f * y[0]; D.l = 0.0f; }
-    const float a = Z == 2 ? y[3] : y[4], b = Z == 0 ? y[3] : y[2];
-    const ff32 u = ffs_sum(a, b), w = ffs_sum(a, -b);
-    c[0] = ffs_add(D, u);
-    c[1] = ffs_sub(D, u);
-    c[2] = ffs_add(D, w);
-    c[3] = ffs_sub(D, w);
-}
-
 // E += the strain-rate sums of family Z (as fcc_edot)
 template <int Z>
 __device__ __forceinline__ void fcc_edot_ff(const ff32 *g, ff32 (&E)[5])
@@ -448,46 +480,58 @@ __device__ __forceinline__ void fcc_edot_ff(const ff32 *g, ff32 (&E)[5])
     }
 }
 
+// a[k] := |a[k]|^e for n float pairs, out of line like fcc_pow_any
+__device__ __noinline__ void fcc_ipow_any(ff32 *a, int n, int e)
+{
+    for (int k = 0; k < n; ++k) a[k] = ff_ipow(a[k].h < 0.0f ? ffs_neg(a[k]) : a[k], e);
+}
+
 // the strain rate (without gam0) as float pairs at the single-precision point
-// y; false when a ratio leaves the float range
+// y (the families in one loop body, as in fcc_jac_ff); false when a ratio
+// leaves the float range
 __device__ __forceinline__ bool fcc_flow_ff(const RveDesc &d, long long v, const float (&y)[5], ff32 (&E)[5])
 {
-    ff32 r[12];
-    float ih[12], il[12];
-    fcc_rss_ff<0>(y, r);
-    fcc_rss_ff<1>(y, r + 4);
-    fcc_rss_ff<2>(y, r + 8);
     bool ok = true;
+    const ff32 zero = {0.0f, 0.0f};
 #pragma unroll
-    for (int k = 0; k < 12; ++k) {
-        const long long col = (long long)(2 * k + (r[k].h < 0.0f)) * d.nv + v;
-        ih[k] = __ldg(d.itau32 + col);
-        il[k] = __ldg(d.itau_lo + col);
-    }
+    for (int c = 0; c < 5; ++c) E[c] = zero;
+#pragma unroll 1
+    for (int z = 0; z < 3; ++z) {
+        const ff32 D = ffs_sum(z == 0 ? y[0] : -y[0], z == 2 ? -y[0] : -y[1]);
+        const float a = z == 2 ? y[3] : y[4], b = z == 0 ? y[3] : y[2];
+        const ff32 u = ffs_sum(a, b), w = ffs_sum(a, -b);
+        ff32 r[4] = {ffs_add(D, u), ffs_sub(D, u), ffs_add(D, w), ffs_sub(D, w)};
+        float ih[4], il[4];
 #pragma unroll
-    for (int k = 0; k < 12; ++k) {
-        r[k] = ff_mul(ff_norm(r[k].h, r[k].l), ih[k], il[k]);
-        ok = ok && fabsf(r[k].h) < 60.0f;
-    }
-    // |r|^n sign(r)
-    if (d.ipow_n == 20) {
-#pragma unroll
-        for (int k = 0; k < 12; ++k) {
-            const ff32 a2 = ff_mul(r[k], r[k].h, r[k].l), a4 = ff_mul(a2, a2.h, a2.l), a8 = ff_mul(a4, a4.h, a4.l);
-            const ff32 a16 = ff_mul(a8, a8.h, a8.l), a20 = ff_mul(a16, a4.h, a4.l);
-            r[k] = r[k].h < 0.0f ? ffs_neg(a20) : a20;
+        for (int k = 0; k < 4; ++k) {
+            const long long col = (long long)(2 * (4 * z + k) + (r[k].h < 0.0f)) * d.nv + v;
+            ih[k] = __ldg(d.itau32 + col);
+            il[k] = __ldg(d.itau_lo + col);
         }
-    } else {
 #pragma unroll
-        for (int k = 0; k < 12; ++k) {
-            const bool neg = r[k].h < 0.0f;
-            const ff32 p = ff_ipow(neg ? ffs_neg(r[k]) : r[k], d.ipow_n);
-            r[k] = neg ? ffs_neg(p) : p;
+        for (int k = 0; k < 4; ++k) {
+            r[k] = ff_mul(ff_norm(r[k].h, r[k].l), ih[k], il[k]);
+            ok = ok && fabsf(r[k].h) < 60.0f;
         }
+        if (d.ipow_n == 20) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const ff32 a2 = ff_mul(r[k], r[k].h, r[k].l), a4 = ff_mul(a2, a2.h, a2.l), a8 = ff_mul(a4, a4.h, a4.l);
+                const ff32 a16 = ff_mul(a8, a8.h, a8.l), a20 = ff_mul(a16, a4.h, a4.l);
+                r[k] = r[k].h < 0.0f ? ffs_neg(a20) : a20;
+            }
+        } else {
+            ff32 q[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k] = r[k];
+            fcc_ipow_any(q, 4, d.ipow_n);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) r[k] = r[k].h < 0.0f ? ffs_neg(q[k]) : q[k];
+        }
+        if (z == 0) fcc_edot_ff<0>(r, E);
+        else if (z == 1) fcc_edot_ff<1>(r, E);
+        else fcc_edot_ff<2>(r, E);
     }
-    fcc_edot_ff<0>(r, E);
-    fcc_edot_ff<1>(r + 4, E);
-    fcc_edot_ff<2>(r + 8, E);
     return ok;
 }
 
@@ -573,9 +617,8 @@ __device__ __forceinline__ ff32 ff_rcp(ff32 a)
     return ff_norm(r, r * e);
 }
 
-// the tangent of family Z from its four h (see fcc_tangent)
-template <int Z>
-__device__ __forceinline__ void fcc_tangent_ff(const ff32 (&h)[4], ff32 (&J)[15])
+// J += the tangent of family z from its four h (see fcc_tangent)
+__device__ __forceinline__ void fcc_tangent_ff(int z, const ff32 (&h)[4], ff32 (&J)[15])
 {
     const ff32 pu = ffs_add(h[0], h[1]), pw = ffs_add(h[2], h[3]);
     const ff32 mu = ffs_sub(h[0], h[1]), mw = ffs_sub(h[2], h[3]);
@@ -583,7 +626,7 @@ __device__ __forceinline__ void fcc_tangent_ff(const ff32 (&h)[4], ff32 (&J)[15]
     auto twice = [](ff32 x) { x.h *= 2.0f; x.l *= 2.0f; return x; };
     auto add = [&](int i, int j, ff32 x) { J[sym5(i, j)] = ffs_add(J[sym5(i, j)], x); };
     auto sub = [&](int i, int j, ff32 x) { J[sym5(i, j)] = ffs_sub(J[sym5(i, j)], x); };
-    if (Z == 0) {
+    if (z == 0) {
         add(0, 0, s);
         sub(0, 1, s);
         add(1, 1, s);
@@ -594,7 +637,7 @@ __device__ __forceinline__ void fcc_tangent_ff(const ff32 (&h)[4], ff32 (&J)[15]
         add(0, 3, b);
         sub(1, 3, b);
         add(3, 4, dl);
-    } else if (Z == 1) {
+    } else if (z == 1) {
         add(0, 0, s);
         add(0, 1, s);
         add(1, 1, s);
@@ -615,40 +658,45 @@ __device__ __forceinline__ void fcc_tangent_ff(const ff32 (&h)[4], ff32 (&J)[15]
     }
 }
 
-// h = dtgn |r|^(n-1) / tau of family Z at y (float pairs), into the tangent
-template <int Z>
-__device__ __forceinline__ void fcc_jac_family_ff(const RveDesc &d, long long v, const ff32 (&y)[5], ff32 dtgn,
-                                                  ff32 (&J)[15])
+// h = dtgn |r|^(n-1) / tau of every system at y (float pairs), into the
+// tangent.  One loop body serves the three families (their inputs selected by
+// z): unrolled, the instructions of this part alone were three times as many,
+// and the warps, each in another place of the Newton loop, waited for them.
+__device__ __forceinline__ void fcc_jac_ff(const RveDesc &d, long long v, const ff32 (&y)[5], ff32 dtgn, ff32 (&J)[15])
 {
-    const ff32 D = Z == 0 ? ffs_sub(y[0], y[1]) : Z == 1 ? ffs_neg(ffs_add(y[0], y[1])) : ffs_add(ffs_neg(y[0]), ffs_neg(y[0]));
-    const ff32 a = Z == 2 ? y[3] : y[4], b = Z == 0 ? y[3] : y[2];
-    const ff32 u = ffs_add(a, b), w = ffs_sub(a, b);
-    ff32 r[4] = {ffs_add(D, u), ffs_sub(D, u), ffs_add(D, w), ffs_sub(D, w)}, h[4];
     const int e = d.ipow_n - 1;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int neg = r[k].h < 0.0f;
-        const ff32 it = d2ff(__ldg(d.itau + (long long)(2 * (4 * Z + k) + neg) * d.nv + v));
-        r[k] = ffs_mul(ffs_norm(r[k]), it);
-        if (neg) r[k] = ffs_neg(r[k]);
-        h[k] = ffs_mul(it, dtgn);
-    }
-    if (e == 19) {
+#pragma unroll 1
+    for (int z = 0; z < 3; ++z) {
+        // D = y0 - y1, -y0 - y1, -2 y0
+        const ff32 D = ffs_sub(z == 0 ? y[0] : ffs_neg(y[0]), z == 2 ? y[0] : y[1]);
+        const ff32 a = z == 2 ? y[3] : y[4], b = z == 0 ? y[3] : y[2];
+        const ff32 u = ffs_add(a, b), w = ffs_sub(a, b);
+        ff32 r[4] = {ffs_add(D, u), ffs_sub(D, u), ffs_add(D, w), ffs_sub(D, w)}, h[4];
+        const double *tau = d.itau + (long long)(8 * z) * d.nv + v;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const ff32 a2 = ffs_mul(r[k], r[k]), a4 = ffs_mul(a2, a2), a8 = ffs_mul(a4, a4), a16 = ffs_mul(a8, a8);
-            h[k] = ffs_mul(ffs_mul(ffs_mul(a16, a2), r[k]), h[k]);
+            const int neg = r[k].h < 0.0f;
+            const ff32 it = d2ff(__ldg(tau + (long long)(2 * k + neg) * d.nv));
+            r[k] = ffs_mul(ffs_norm(r[k]), it);
+            if (neg) r[k] = ffs_neg(r[k]);
+            h[k] = ffs_mul(it, dtgn);
         }
-    } else {
-        for (int q = e; q; q >>= 1) {
+        if (e == 19) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                if (q & 1) h[k] = ffs_mul(h[k], r[k]);
-                r[k] = ffs_mul(r[k], r[k]);
+                const ff32 a2 = ffs_mul(r[k], r[k]), a4 = ffs_mul(a2, a2), a8 = ffs_mul(a4, a4), a16 = ffs_mul(a8, a8);
+                h[k] = ffs_mul(ffs_mul(ffs_mul(a16, a2), r[k]), h[k]);
             }
+        } else if (e > 0) {
+            ff32 q[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k] = r[k];
+            fcc_ipow_any(q, 4, e);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) h[k] = ffs_mul(q[k], h[k]);
         }
+        fcc_tangent_ff(z, h, J);
     }
-    fcc_tangent_ff<Z>(h, J);
 }
 
 // x := M^-1 x at the stress y.  False when a value left the float range (the
@@ -663,9 +711,7 @@ __device__ __forceinline__ bool fcc_solve_ff(const RveDesc &d, long long v, cons
         for (int c = 0; c < 5; ++c) y[c] = d2ff(yd[c]);
 #pragma unroll
         for (int q = 0; q < 15; ++q) M[q] = d2ff(__ldg(d.sch + (FCC_P + q) * d.nv + v));
-        fcc_jac_family_ff<0>(d, v, y, dtgn, M);
-        fcc_jac_family_ff<1>(d, v, y, dtgn, M);
-        fcc_jac_family_ff<2>(d, v, y, dtgn, M);
+        fcc_jac_ff(d, v, y, dtgn, M);
     }
     auto fms = [](ff32 &acc, ff32 a, ff32 b) { ff_acc2(acc, -a.h, -a.l, b.h, b.l); };
     // LDL^T in place, as fcc_factor

@@ -1023,15 +1023,16 @@ __device__ void nr_unit(const RveDesc &d, int unit, int nunits)
 // 72 for the powers, 25 for P y (the pressure decouples); the tangent and the
 // 5x5 solve, 240 + 125 there, run in float pairs on the FP32 pipe beside it.
 // Measured per launch against kb_nr (FP64 form, first increment): 64^3 879 ->
-// 359 us (477 with the solve in FP64), 16^3 (a grain per voxel) 86 -> 45 us.
+// 343 us (477 with the solve in FP64), 128^3 10.4 -> 3.8 ms, 16^3 (a grain
+// per voxel) 86 -> 44 us.
 // With the solve off the FP64 pipe a chord step saves nothing, so d.chord is
 // not looked at here.
 //
 // FCC_IR (VOCE_PREC_MIXED_IR): newton_ir in the same variables: the start in
 // single precision and float pairs, then steps whose residual, flow rule and
 // stop test are FP64 and whose correction is solved in FP32 with the start's
-// last matrix; 64^3 363 -> 216 us, 256^3 29.9 -> 15.4 ms.  FCC_NR32
-// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 295 us.  Nothing is staged
+// last matrix; 64^3 363 -> 213 us, 256^3 29.9 -> 14.6 ms.  FCC_NR32
+// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 306 us.  Nothing is staged
 // in shared memory: the single-precision steps read 15 + 12 floats per voxel
 // instead of 21 + 72.  Conversions go through the integer pipe (d2f, f2d:
 // with the hardware's, 239 and 331 us).
@@ -1100,7 +1101,7 @@ __device__ __forceinline__ void fcc_newton(const RveDesc &d, long long v, const 
 #pragma unroll
         for (int c = 0; c < 5; ++c) yp[c] = y[c];
         s5p = s5;
-        bool fp64 = fcc_edot_fp64(d, v, y, E) || d.ipow_n > 20;
+        bool fp64 = fcc_edot_fp64_loop(d, v, y, E) || d.ipow_n > 20;
 #pragma unroll
         for (int c = 0; c < 5; ++c) x[c] = fma(dtg, E[c], cc[c]);
         fcc_add_Py(fx, nv, y, x);
