@@ -1999,12 +1999,15 @@ __device__ void prelude_unit(const RveDesc &d, int unit, int nunits)
         t6_to_b<double>(t6, set6);
     }
     const long long nv = d.nv;
-    for (long long v = (long long)unit * blockDim.x + threadIdx.x; v < nv;
-         v += (long long)nunits * blockDim.x)
-        for (int c = 0; c < 6; ++c) {
-            if (d.creep) d.dgs[c * nv + v] = set6[c];
-            else d.dgs[c * nv + v] += d.u6[c] * d.dt;
-        }
+    // component by component, the ones that do not change left out
+    for (int c = 0; c < 6; ++c) {
+        const double add = d.u6[c] * d.dt, set = set6[c];
+        if (!d.creep && add == 0.0) continue;
+        double *g = d.dgs + c * nv;
+#pragma unroll 4
+        for (long long v = (long long)unit * blockDim.x + threadIdx.x; v < nv; v += (long long)nunits * blockDim.x)
+            g[v] = d.creep ? set : g[v] + add;
+    }
 }
 
 
@@ -2193,7 +2196,10 @@ __global__ void __launch_bounds__(128, kIncrEndBlocks) kb_incr_end_fcc(const Rve
     }
 }
 
-__global__ void __launch_bounds__(128) kb_prelude(const RveDesc *descs, const int2 *map, int total)
+// threads per block of the prelude: pure memory traffic over the 456 or fewer
+// units of an RVE, so wide blocks keep enough of it in flight
+constexpr int kPreludeThreads = 512;
+__global__ void __launch_bounds__(kPreludeThreads) kb_prelude(const RveDesc *descs, const int2 *map, int total)
 {
     for (int w = blockIdx.x; w < total; w += gridDim.x) {
         const int2 e = map[w];
@@ -2370,9 +2376,9 @@ int nr_resident_blocks(int kind)
 template <typename R>
 static void plan_prelude_t(const BatchPlan &bp, cudaStream_t s, Prof &pf)
 {
-    const int NG = 152 * 2;
+    const int NG = 152 * 4;
     pf.begin(K_PRELUDE, s);
-    kb_prelude<<<grid_for(bp.total[BP_NP], NG), 128, 0, s>>>(bp.descs, bp.map[BP_NP], bp.total[BP_NP]);
+    kb_prelude<<<grid_for(bp.total[BP_NP], NG), kPreludeThreads, 0, s>>>(bp.descs, bp.map[BP_NP], bp.total[BP_NP]);
     pf.end(K_PRELUDE, s);
 }
 
