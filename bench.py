@@ -63,8 +63,7 @@ DTYPE = {"fp64": "f64", "mixed": "f32 spectrum+f64 newton",
          "mixed_ir": "f32 spectrum+f64 newton residual+f32 newton correction",
          "mixed_ir_strict": "f32 spectrum+f64 newton residual+f32 newton correction",
          "mixed_nr32": "f32 spectrum+f32 newton+f64 acceptance"}
-FORM_DOC = {"mixed": "FP32 spectrum and Green operator; FP64 Newton (exact Jacobian, chord steps "
-                     "near the root), hardening, norms, averages",
+FORM_DOC = {"mixed": "FP32 spectrum and Green operator; FP64 Newton, hardening, norms, averages",
             "mixed_ir": "FP32 spectrum and Green operator; Newton: FP32 steps choose the start, "
                         "then every accepted step evaluates the residual and flow rule in FP64 with "
                         "the FP64 stop test, its Jacobian and LDL^T correction in FP32; hardening, "
@@ -240,23 +239,23 @@ def measured_peaks():
     return 6800.0, "fallback"
 
 
-# From the ncu capture of kb_nr<0> (FP64 form) on this workload, summarised in
-# profiles/kb_nr_fp64_cfg2_64.md: DRAM bytes read + written by one launch over
-# 262144 voxels, and the FP64 flops (FMA = 2) per Newton iteration of a voxel
-# and per voxel per launch (instruction counts fitted against the Newton
-# iterations of each launch; the capture there checks the fit).
-KB_NR_FP64_DRAM_BYTES = 268.9e6
+# From the ncu capture of the Newton kernel (kb_nr_fcc<0>, FP64 form) on this
+# workload, summarised in profiles/kb_nr_fp64_cfg2_64.md: DRAM bytes read +
+# written by one launch over 262144 voxels, and the FP64 flops (FMA = 2) per
+# Newton iteration of a voxel and per voxel per launch (instruction counts of 62
+# launches fitted against their Newton iterations).
+KB_NR_FP64_DRAM_BYTES = 228.1e6
 KB_NR_FP64_VOXELS = 262144
-KB_NR_FP64_FLOPS_PER_NEWTON = 1127
-KB_NR_FP64_FLOPS_PER_VOXEL = 307
+KB_NR_FP64_FLOPS_PER_NEWTON = 212
+KB_NR_FP64_FLOPS_PER_VOXEL = 300.6
 
 
-# The same for kb_nr<1> (mixed_nr32 form, profiles/kb_nr_nr32_cfg2_64.md) and
-# kb_nr<0, 0, 1> (mixed_ir form, profiles/kb_nr_mixed_ir_cfg2_64.md); the mixed
-# form's chord-step instance of the FP64 Newton kernel moves the same bytes as
-# the FP64 one (profiles/kb_nr_mixed_cfg2_64.md).
-KB_NR_NR32_DRAM_BYTES = 280.0e6
-KB_NR_IR_DRAM_BYTES = 545.3e6
+# The same for the mixed_nr32 form's kernel (kb_nr_fcc<2>,
+# profiles/kb_nr_nr32_cfg2_64.md) and the mixed_ir form's (kb_nr_fcc<1>,
+# profiles/kb_nr_mixed_ir_cfg2_64.md); the mixed form runs the FP64 form's
+# kernel (profiles/kb_nr_mixed_cfg2_64.md).
+KB_NR_NR32_DRAM_BYTES = 244.4e6
+KB_NR_IR_DRAM_BYTES = 349.7e6
 
 
 def profiled_traffic(precision="fp64"):
@@ -268,8 +267,9 @@ def profiled_traffic(precision="fp64"):
 
 
 def fp64_flops_per_newton_iteration():
-    """FP64 flops (FMA = 2) that kb_nr<0> executes per Newton iteration of
-    one voxel and per voxel per launch (profiles/kb_nr_fp64_cfg2_64.md)."""
+    """FP64 flops (FMA = 2) that the FP64 form's Newton kernel executes per
+    Newton iteration of one voxel and per voxel per launch
+    (profiles/kb_nr_fp64_cfg2_64.md)."""
     return KB_NR_FP64_FLOPS_PER_NEWTON, KB_NR_FP64_FLOPS_PER_VOXEL
 
 
@@ -501,10 +501,10 @@ def run_voce(args, rank, world, grp):
         "config": conf,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": profiled_traffic(args.precision),
-                     "kernel": "kb_nr", "peak_kind": peak_kind,
+                     "kernel": "kb_nr_fcc", "peak_kind": peak_kind,
                      "algorithmic_bytes_per_voxel": NR_BYTES_PER_VOXEL,
                      "avg_launch_ms": nr_avg_s * 1e3},
-        "fp64_roof": {"bound": "fp64", "kernel": "kb_nr", "achieved": fp64_ach,
+        "fp64_roof": {"bound": "fp64", "kernel": "kb_nr_fcc", "achieved": fp64_ach,
                       "peak": fp64_peak, "unit": "TFLOP/s",
                       "frac": (fp64_ach / fp64_peak) if fp64_ach else None,
                       "peak_kind": "measured by voce_measure_fp64_tflops in this run"},

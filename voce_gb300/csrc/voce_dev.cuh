@@ -21,6 +21,8 @@
 //   spec[6][nzh][nx][ny] half spectrum (kz = 0..nz/2), complex, y fastest
 //   aacc[3][nzh][nx][ny] antisymmetric part of the Green update, summed
 //                 over the iterations of the current increment
+// For the {111}<110> slip family (RveDesc::fcc) sch, sigp, itau and the float
+// arrays hold the crystal-axes quantities that voce_fcc.cuh lists.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

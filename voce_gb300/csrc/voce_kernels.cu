@@ -1,10 +1,12 @@
 // sm_103a kernels of the EVP-FFT solver step.  See voce_dev.cuh for the
 // data layout.  One Green-operator iteration is
-//   k_fft_z_fwd  -> k_fft_y(-1) -> k_fft_x_green -> k_fft_y(+1) ->
-//   k_fft_z_inv(update) -> k_nr -> k_finalize_iter
-// and an increment ends with
-//   k_fft_x(+1,aacc) -> k_fft_y(+1,aacc) -> k_fft_z_inv(rotl) ->
-//   k_incr_end -> k_finalize_incr
+//   kb_fft_z_fwd -> kb_fft_y(-1) -> kb_fft_x_green -> kb_fft_y(+1) ->
+//   kb_fft_z_inv(update) -> kb_nr / kb_nr_fcc -> kb_finalize
+// and an increment, opened by kb_prelude, ends with
+//   kb_fft_x_aacc -> kb_fft_y(+1,aacc) -> kb_fft_z_inv(rotl) ->
+//   kb_incr_end / kb_incr_end_fcc -> kb_finalize
+// The spectrum passes are in voce_fft.cuh; the Newton kernels and the increment
+// epilogue of the {111}<110> slip family use voce_fcc.cuh.
 #include "voce_dev.cuh"
 #include "voce_fcc.cuh"
 #include "voce_fft.cuh"
