@@ -2239,7 +2239,10 @@ __global__ void __launch_bounds__(256) kb_finalize(const RveDesc *descs, int nrv
         reduce_partials(part, npart, all1, s_tot);   // (synchronises the block)
         const RveDesc &d = *reinterpret_cast<const RveDesc *>(s_desc);
         MacroDev *m = reinterpret_cast<MacroDev *>(s_macro);
-        if (!m->active) {
+        // (the increment's finaliser has tested the flag above, and its thread 0
+        // clears it in m below: tested here too, it would be read by the other
+        // threads while it changes.  The iteration's leaves it alone.)
+        if (!incr_end && !m->active) {
             __syncthreads();
             continue;
         }
