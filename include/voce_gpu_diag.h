@@ -87,6 +87,12 @@ int voce_rve_get_tiles(const voce_rve *r, int tiles[6]);
 /* Force the tiles (each divides the dimension it splits: ny, nx, ny, ny, ny,
  * ny; all phases fit in shared memory); between calls, outside a batch. */
 int voce_rve_set_tiles(voce_rve *r, const int tiles[6]);
+/* Shared memory in bytes that the FFT passes of an RVE of dims would ask for
+ * with these tiles (null: the fixed-budget choice) and the default schedules:
+ * z forward, y, x/Green, z inverse, and the antisymmetric back-transform's x,
+ * y, z.  Host arithmetic only.  VOCE_ERR_ARG for tiles that
+ * voce_rve_set_tiles refuses. */
+int voce_fft_smem(const int dims[3], int precision, const int tiles[6], long long bytes[7]);
 
 /* FFT radix schedules (no counterpart in the reference, which leaves its
  * transforms to FFTW).  Each axis of length L = 2^a 3^b can run as Stockham

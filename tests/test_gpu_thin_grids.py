@@ -1,0 +1,64 @@
+"""Grids whose y tile fits the y pass's line buffers but not its two padded
+stream buffers (a long x edge over a short y edge): they are created with the
+default settings, and run as with small tiles, bit for bit."""
+import numpy as np
+import pytest
+
+from voce_gb300 import capi, synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _create(dims, prec, seed):
+    mesh = synth.voronoi_mesh_box(dims, 9, seed)
+    nl, slip = capi.VoceNamelist(), capi.VoceSlip()
+    m, load = synth.CU_LIKE, synth.tension_z()
+    nl.CellDim[:] = mesh.dims
+    nl.N_phases = 1
+    nl.TimeStep, nl.N_steps, nl.IterMax, nl.Err = 0.2, 10, 6, 1e-5
+    nl.Update_Flag = nl.Hard_Flag = 1
+    nl.VelGrad_BC_Flag[:], nl.VelGrad_BC[:] = load.velgrad_flag, load.velgrad
+    nl.Stress_BC_Flag[:], nl.Stress_BC[:] = load.stress_flag, load.stress
+    nl.ElastConst_PhaseI[:] = (168400.0, 121400.0, 75400.0, 0.35)
+    for k in ("self", "coplane", "cross", "glissile", "hirth", "lomer"):
+        getattr(nl, k)[0] = 1.0
+    slip.nsys, slip.nrs, slip.gamd0 = 12, 20.0, m.gamd0
+    slip.tau0f, slip.tau0b, slip.tau1, slip.thet0, slip.thet1 = m.tau0f, m.tau0b, m.tau1, m.thet0, m.thet1
+    for k, (n, b) in enumerate(synth.FCC_111_110):
+        slip.bn[k][:], slip.bb[k][:] = n, b
+    return capi.Rve.create(nl, slip, mesh.euler_deg, mesh.grain, mesh.phase, prec)
+
+
+def _solve(r):
+    r.run(2)
+    return [r.increment(k) for k in range(2)], r.field("sig"), r.field("disgrad")
+
+
+@pytest.mark.parametrize("dims,prec,yxt", [
+    ((256, 24, 4), capi.PREC_FP64, 256),       # register FFT along y, 237568 B for the stream
+    ((384, 16, 2), capi.PREC_FP64, 384),
+    ((324, 18, 2), capi.PREC_FP64, 324),       # a factor 3 along y
+    ((216, 32, 2), capi.PREC_FP64, 216),       # only when asked for
+    ((864, 12, 2), capi.PREC_MIXED, 864),
+    ((512, 24, 2), capi.PREC_MIXED_IR, 512),
+])
+def test_long_x_edges_over_short_y_edges(dims, prec, yxt, voce_lib):
+    with _create(dims, prec, 96) as r:
+        if prec != capi.PREC_FP64:             # the timed schedules aside, which change the rounding
+            for a in range(3):
+                r.set_fft_schedule(a, 0)
+        want = _solve(r)
+        assert np.all(np.isfinite(want[1]))
+    with _create(dims, prec, 96) as r:
+        if prec != capi.PREC_FP64:
+            for a in range(3):
+                r.set_fft_schedule(a, 0)
+        t = r.tiles()
+        for ty in (yxt, 1):                    # past the stream's size, and a small one
+            t[1] = ty
+            r.set_tiles(t)
+            assert r.tiles()[1] == ty
+            with capi.Rve.restore(r.snapshot()) as q:
+                got = _solve(q)
+            assert got[0] == want[0]
+            assert np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2]), ty

@@ -113,6 +113,7 @@ PROTOTYPES = [
     ("voce_rve_get_namelist", C.c_int, [C.c_void_p, C.POINTER(VoceNamelist)]),
     ("voce_rve_destroy", C.c_int, [C.c_void_p]),
     ("voce_rve_footprint", C.c_longlong, [C.POINTER(C.c_int), C.c_int]),
+    ("voce_fft_smem", C.c_int, [C.POINTER(C.c_int), C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_longlong)]),
     # voce_gpu_diag.h
     ("voce_rve_run_timed", C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_double)]),
     ("voce_rve_set_graph", C.c_int, [C.c_void_p, C.c_int]),
@@ -285,6 +286,15 @@ def read_mesh(path: str, dims: Sequence[int]):
 
 def footprint(dims: Sequence[int], precision: int = PREC_FP64) -> int:
     return int(load().voce_rve_footprint((C.c_int * 3)(*dims), precision))
+
+
+def fft_smem(dims: Sequence[int], precision: int = PREC_FP64, tiles=None) -> list:
+    """Shared memory in bytes of the FFT passes (z forward, y, x/Green, z
+    inverse, back-transform x, y, z); VoceError for tiles set_tiles refuses."""
+    b = (C.c_longlong * 7)()
+    t = None if tiles is None else (C.c_int * 6)(*tiles)
+    _check(load().voce_fft_smem((C.c_int * 3)(*dims), precision, t, b))
+    return list(b)
 
 
 def device_memory():

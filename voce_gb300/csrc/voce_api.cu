@@ -472,6 +472,7 @@ namespace {
 int autotune_tiles(voce_rve *r);
 void apply_tiles(voce_rve *r, const Tiles &t);
 Tiles tiles_of(const RveDesc &d);
+int tiles_problem(const RveDesc &d);
 FftPlan1 schedule_of(int L, bool mixed, int k);
 extern int g_autotune;
 extern int g_newton_chord;
@@ -828,7 +829,7 @@ int voce_rve_create(const voce_namelist *nl, const voce_slip *slip[2], const voc
         dt.ply = schedule_of(ny, d.mixed != 0, 0);
         dt.plz = schedule_of(nz, d.mixed != 0, 0);
         for (int ph = BP_ZF; ph < BP_COUNT; ++ph)
-            if (batch_smem(dt, ph) > 227 * 1024)
+            if (batch_smem(dt, ph) > kBlockSmem)
                 return fail(VOCE_ERR_UNSUPPORTED,
                             "grid %dx%dx%d: a line is too long for the FFT passes' shared memory in this precision",
                             nx, ny, nz);
@@ -1025,25 +1026,10 @@ int make_plan(const std::vector<RveDesc> &descs, int precision, RveDesc *&d_desc
     for (int i = 0; i < p.nrve; ++i) {
         int u[BP_COUNT];
         batch_units(descs[i], u);
-        for (int ph = 0; ph < BP_COUNT; ++ph) {
+        for (int ph = 0; ph < BP_COUNT; ++ph)
             for (int k = 0; k < u[ph]; ++k) maps[ph].push_back(make_int2(i, k));
-            p.smem[ph] = std::max(p.smem[ph], batch_smem(descs[i], ph));
-        }
     }
-    {   // the streamed y pass: all RVEs on the register FFT along y
-        long long S = 0;
-        bool all = true;
-        for (const RveDesc &d : descs) {
-            if (d.ply.n1 <= 0) all = false;
-            else S = std::max(S, (long long)d.yxt * (d.ny + d.ply.n1 + 1));
-        }
-        if (all) {
-            p.ystream = (int)((S + 1) & ~1LL);
-            const size_t sm = 2 * (size_t)p.ystream * (p.mixed ? sizeof(float2) : sizeof(double2));
-            p.smem[BP_Y6] = std::max(p.smem[BP_Y6], sm);
-            p.smem[BP_Y3] = std::max(p.smem[BP_Y3], sm);
-        }
-    }
+    p.ystream = plan_smem(descs, p.mixed, p.smem);
     size_t tot = 0;
     for (int ph = 0; ph < BP_COUNT; ++ph) tot += maps[ph].size();
     CUDA_TRY(cudaMalloc(&d_descs, sizeof(RveDesc) * descs.size()));
@@ -1125,6 +1111,20 @@ Tiles tiles_of(const RveDesc &d)
             }
     }
     return t;
+}
+
+// The tile rule: each tile divides the dimension it splits and its phase fits
+// in a block's shared memory.  Returns the first tile that breaks it (its
+// index as in voce_rve_set_tiles, or 6 when a phase does not fit), or -1.
+int tiles_problem(const RveDesc &d)
+{
+    const int dim[6] = {d.ny, d.nx, d.ny, d.ny, d.ny, d.ny};
+    const int tl[6] = {d.zrows, d.yxt, d.xkc, d.zirows, d.xkc3, d.zirows3};
+    for (int k = 0; k < 6; ++k)
+        if (tl[k] < 1 || dim[k] % tl[k] != 0) return k;
+    for (int ph = BP_ZF; ph < BP_COUNT; ++ph)
+        if (batch_smem(d, ph) > kBlockSmem) return 6;
+    return -1;
 }
 
 void apply_tiles(voce_rve *r, const Tiles &t)
@@ -1210,7 +1210,11 @@ int autotune_tiles(voce_rve *r)
         int2 *pm = nullptr;
         BatchPlan bp;
         rc = make_plan(one, r->precision, pd, pm, bp);
-        if (rc) return -1.f;
+        if (rc) {
+            cudaFree(pd);
+            cudaFree(pm);
+            return -1.f;
+        }
         float ms = 1e30f;
         cudaError_t e = launch_plan_phase(bp, ph, r->stream);
         for (int round = 0; round < 2 && e == cudaSuccess; ++round) {
@@ -1760,12 +1764,7 @@ const char *snapshot_desc_problem(const SnapHead &h, const RveDesc &d, const voc
         if (!found) return "FFT schedule";
     }
     // the tiles: the rule voce_rve_set_tiles applies
-    const int dim[6] = {d.ny, d.nx, d.ny, d.ny, d.ny, d.ny};
-    const int tl[6] = {d.zrows, d.yxt, d.xkc, d.zirows, d.xkc3, d.zirows3};
-    for (int k = 0; k < 6; ++k)
-        if (tl[k] < 1 || dim[k] % tl[k] != 0) return "FFT tiles";
-    for (int ph = BP_ZF; ph < BP_COUNT; ++ph)
-        if (batch_smem(d, ph) > 227 * 1024) return "FFT tiles";
+    if (tiles_problem(d) >= 0) return "FFT tiles";
     if (h.npart < 1 || d.npart != h.npart || h.npart > std::max<long long>(1, (d.nv + 127) / 128))
         return "work split";
     if (d.nsys < 1 || d.nsys > VOCE_NS) return "number of slip systems";
@@ -2093,21 +2092,48 @@ int voce_rve_set_tiles(voce_rve *r, const int tiles[6])
     if (!r || !tiles) return fail(VOCE_ERR_ARG, "null argument");
     if (r->batch) return fail(VOCE_ERR_STATE, "the RVE belongs to a batch");
     const RveDesc &d = r->d;
-    // each tile divides the dimension it splits, and its phase fits in shared memory
-    const int dim[6] = {d.ny, d.nx, d.ny, d.ny, d.ny, d.ny};
-    for (int k = 0; k < 6; ++k)
-        if (tiles[k] < 1 || dim[k] % tiles[k] != 0) return fail(VOCE_ERR_ARG, "tile %d = %d", k, tiles[k]);
     Tiles t = r->tiles;   // the radix schedules stay
     t.zrows = tiles[0]; t.yxt = tiles[1]; t.xkc = tiles[2];
     t.zirows = tiles[3]; t.xkc3 = tiles[4]; t.zirows3 = tiles[5];
     RveDesc dt = d;
     dt.zrows = t.zrows; dt.yxt = t.yxt; dt.xkc = t.xkc; dt.xkc3 = t.xkc3; dt.zirows = t.zirows; dt.zirows3 = t.zirows3;
-    for (int ph = BP_ZF; ph < BP_COUNT; ++ph)
-        if (batch_smem(dt, ph) > 227 * 1024) return fail(VOCE_ERR_ARG, "tiles need more shared memory than a block has");
+    const int bad = tiles_problem(dt);
+    if (bad == 6) return fail(VOCE_ERR_ARG, "tiles need more shared memory than a block has");
+    if (bad >= 0) return fail(VOCE_ERR_ARG, "tile %d = %d", bad, tiles[bad]);
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     apply_tiles(r, t);
     if (r->graph_exec) { cudaGraphExecDestroy(r->graph_exec); r->graph_exec = nullptr; }
     if (r->graph) { cudaGraphDestroy(r->graph); r->graph = nullptr; }
+    return VOCE_OK;
+}
+
+int voce_fft_smem(const int dims[3], int precision, const int tiles[6], long long bytes[7])
+{
+    if (!dims || !bytes || precision < VOCE_PREC_FP64 || precision > VOCE_PREC_MIXED_IR)
+        return fail(VOCE_ERR_ARG, "bad argument");
+    RveDesc d;
+    std::memset(&d, 0, sizeof(d));
+    d.nx = dims[0]; d.ny = dims[1]; d.nz = dims[2]; d.nzh = d.nz / 2 + 1;
+    d.mixed = precision != VOCE_PREC_FP64;
+    FftPlan1 p;
+    if (!fft_plan(d.nx, p) || !fft_plan(d.ny, p) || !fft_plan(d.nz, p) || d.nz % 2)
+        return fail(VOCE_ERR_UNSUPPORTED, "grid %dx%dx%d", d.nx, d.ny, d.nz);
+    d.plx = schedule_of(d.nx, d.mixed, 0);
+    d.ply = schedule_of(d.ny, d.mixed, 0);
+    d.plz = schedule_of(d.nz, d.mixed, 0);
+    Tiles t;
+    if (d.mixed) t.choose<float>(d);
+    else t.choose<double>(d);
+    if (tiles) {
+        t.zrows = tiles[0]; t.yxt = tiles[1]; t.xkc = tiles[2];
+        t.zirows = tiles[3]; t.xkc3 = tiles[4]; t.zirows3 = tiles[5];
+    }
+    d.zrows = t.zrows; d.yxt = t.yxt; d.xkc = t.xkc; d.xkc3 = t.xkc3; d.zirows = t.zirows; d.zirows3 = t.zirows3;
+    if (tiles_problem(d) >= 0) return fail(VOCE_ERR_ARG, "tiles");
+    size_t smem[BP_COUNT] = {};
+    plan_smem(std::vector<RveDesc>(1, d), d.mixed != 0, smem);
+    const int ph[7] = {BP_ZF, BP_Y6, BP_XG, BP_ZI, BP_X3, BP_Y3, BP_Z3};
+    for (int k = 0; k < 7; ++k) bytes[k] = (long long)smem[ph[k]];
     return VOCE_OK;
 }
 

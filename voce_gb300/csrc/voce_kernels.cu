@@ -2335,6 +2335,23 @@ size_t batch_smem(const RveDesc &d, int ph)
     return d.mixed ? batch_smem_t<float>(d, ph) : batch_smem_t<double>(d, ph);
 }
 
+int plan_smem(const std::vector<RveDesc> &descs, bool mixed, size_t smem[BP_COUNT])
+{
+    long long S = 0;
+    bool all = !descs.empty();
+    for (const RveDesc &d : descs) {
+        for (int ph = 0; ph < BP_COUNT; ++ph) smem[ph] = std::max(smem[ph], batch_smem(d, ph));
+        if (d.ply.n1 <= 0) all = false;
+        else S = std::max(S, (long long)d.yxt * (d.ny + d.ply.n1 + 1));
+    }
+    S = (S + 1) & ~1LL;
+    const size_t sm = 2 * (size_t)S * (mixed ? sizeof(float2) : sizeof(double2));
+    if (!all || sm > kBlockSmem) return 0;
+    smem[BP_Y6] = std::max(smem[BP_Y6], sm);
+    smem[BP_Y3] = std::max(smem[BP_Y3], sm);
+    return (int)S;
+}
+
 cudaError_t set_batch_smem(const BatchPlan &bp)
 {
     return bp.mixed ? set_fft_smem<float>(bp) : set_fft_smem<double>(bp);

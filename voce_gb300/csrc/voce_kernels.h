@@ -2,6 +2,8 @@
 #pragma once
 #include "voce_dev.cuh"
 
+#include <vector>
+
 namespace voce {
 
 // Constants used only by the setup and increment-end kernels.
@@ -79,7 +81,7 @@ struct BatchPlan {
     bool ir = false;      // FP64-residual Newton with a float Jacobian
     int ystream = 0;      // > 0: every RVE runs the register FFT along y; the y
                           // pass streams its units through two tile buffers of
-                          // this many complex floats
+                          // this many complex numbers
 };
 // The spectrum passes of a plan (float: single-precision spectrum): z forward,
 // y forward, x with the Green operator, y inverse, z inverse into DisGrad, and
@@ -94,6 +96,16 @@ template <> cudaError_t set_fft_smem<double>(const BatchPlan &bp);
 // units of one RVE in each phase
 void batch_units(const RveDesc &d, int units[BP_COUNT]);
 size_t batch_smem(const RveDesc &d, int phase);
+// dynamic shared memory a block can ask for
+constexpr size_t kBlockSmem = 227 * 1024;
+// Shared memory of every FFT phase of a plan of n RVEs whose phases each fit,
+// and the size of the y pass's stream buffers (0: the plan does not stream):
+// the y pass streams where all RVEs run the register FFT along y and the two
+// padded tile buffers fit in a block.  Their tile is larger than the two line
+// buffers a lone phase needs (2 yxt (ny + N1 + 1) against 2 ny (yxt | 1)
+// complex numbers), so a tile that fits the phase need not fit the stream; the
+// y pass then runs a tile at a time, with the same results.
+int plan_smem(const std::vector<RveDesc> &descs, bool mixed, size_t smem[BP_COUNT]);
 cudaError_t set_batch_smem(const BatchPlan &bp);
 // one forward-pass FFT phase (BP_ZF, BP_Y6 forward, BP_XG, BP_ZI) alone, for
 // tile tuning
