@@ -1,6 +1,7 @@
-"""Grids whose y tile fits the y pass's line buffers but not its two padded
-stream buffers (a long x edge over a short y edge): they are created with the
-default settings, and run as with small tiles, bit for bit."""
+"""FFT tiles that fit the passes' line buffers but not the larger layouts of
+the register FFT (a long x edge over a short y edge, whose y tile is past the
+two padded stream buffers, and forced tiles of the x and z passes): such an
+RVE is created, and runs as with small tiles, bit for bit."""
 import numpy as np
 import pytest
 
@@ -9,10 +10,12 @@ from voce_gb300 import capi, synth
 pytestmark = pytest.mark.gpu
 
 
-def _create(dims, prec, seed):
+def _create(dims, prec, seed, mixed_load=True):
     mesh = synth.voronoi_mesh_box(dims, 9, seed)
     nl, slip = capi.VoceNamelist(), capi.VoceSlip()
-    m, load = synth.CU_LIKE, synth.tension_z()
+    m = synth.CU_LIKE
+    load = synth.tension_z() if mixed_load else \
+        synth.random_traceless_load(np.random.Generator(np.random.PCG64(seed)))
     nl.CellDim[:] = mesh.dims
     nl.N_phases = 1
     nl.TimeStep, nl.N_steps, nl.IterMax, nl.Err = 0.2, 10, 6, 1e-5
@@ -62,3 +65,29 @@ def test_long_x_edges_over_short_y_edges(dims, prec, yxt, voce_lib):
                 got = _solve(q)
             assert got[0] == want[0]
             assert np.array_equal(got[1], want[1]) and np.array_equal(got[2], want[2]), ty
+
+
+@pytest.mark.parametrize("dims,prec,tiles", [
+    # z forward, y, x/Green, z inverse tiles, each past the register FFT's own layout
+    ((64, 36, 64), capi.PREC_FP64, [36, 2, 18, 36]),
+    ((144, 24, 144), capi.PREC_FP64, [8, 2, 8, 12]),      # 12 x 12
+    ((8, 96, 32), capi.PREC_MIXED, [96, 2, 8, 48]),
+    ((8, 72, 32), capi.PREC_MIXED_NR32, [72, 2, 8, 72]),
+    ((36, 64, 8), capi.PREC_MIXED, [8, 2, 64, 8]),        # 6 x 6
+])
+@pytest.mark.parametrize("mixed_load", [False, True])     # with and without a mean correction of the gradient
+def test_tiles_beyond_the_register_layout(dims, prec, tiles, mixed_load, voce_lib):
+    with _create(dims, prec, 97, mixed_load) as r:
+        for a in range(3):
+            if prec != capi.PREC_FP64:
+                r.set_fft_schedule(a, 0)
+        t = r.tiles()
+        got = []
+        for use in (tiles, [1, 1, 1, 1]):
+            r.set_tiles(use + t[4:])
+            with capi.Rve.restore(r.snapshot()) as q:
+                assert q.tiles() == use + t[4:]
+                got.append(_solve(q))
+    assert got[0][0] == got[1][0]
+    assert np.all(np.isfinite(got[0][1]))
+    assert np.array_equal(got[0][1], got[1][1]) and np.array_equal(got[0][2], got[1][2])

@@ -525,6 +525,15 @@ __host__ __device__ inline size_t xg_smem(int nx, int n1, int kc)
 {
     return 2 * sizeof(C) * (size_t)(6 * kc) * (size_t)(nx + n1 + 1);
 }
+// whether the RVE's x pass runs xg_unit: an axis on the register FFT whose
+// tile fits in a block in xg_unit's padded layout.  A larger tile, which fits
+// in the two line buffers of fft_lines alone, goes through those
+// (fft_x_green_unit), with the same results.
+template <typename C>
+__host__ __device__ inline bool xg_fits(const RveDesc &d)
+{
+    return d.plx.n1 > 0 && xg_smem<C>(d.nx, d.plx.n1, d.xkc) <= kBlockSmem;
+}
 
 template <typename R>
 __device__ void fft_x_unit(const RveDesc &d, void *specp, int ncomp, int sign, int kc, int unit)
@@ -664,7 +673,8 @@ static __device__ void fft_z_inv_dgs_f32(const RveDesc &d, int rows, int unit)
 // fewer.  Everything is staged by asynchronous copies.
 // us per launch, forward / inverse, against the passes through fft_lines:
 // single precision 256^3 461 / 950 -> 376 / 645, 96^3 34 / 64 -> 28 / 42; FP64
-// 128^3 359 / 408 -> 321 / 329.  Those passes stay for the Stockham stages.
+// 128^3 359 / 408 -> 321 / 329.  Those passes stay for the Stockham stages
+// and for tiles that do not fit in a block in this layout (zf_fits, zi_fits).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float from_double(double x, float) { return d2f_rn(x); }
 __device__ __forceinline__ double from_double(double x, double) { return x; }
@@ -864,6 +874,19 @@ __host__ __device__ inline size_t zi_smem(int nz, int n1, int rows)
            sizeof(C) * 6 * (size_t)(nz / 2 + 1) * rows;
 }
 
+// whether the RVE's z passes run zf_unit, zi_unit (as xg_fits): larger tiles
+// go through fft_lines
+template <typename C>
+__host__ __device__ inline bool zf_fits(const RveDesc &d)
+{
+    return d.plz.n1 > 0 && zf_smem<C>(d.nz, d.plz.n1, d.zrows) <= kBlockSmem;
+}
+template <typename C>
+__host__ __device__ inline bool zi_fits(const RveDesc &d)
+{
+    return d.plz.n1 > 0 && zi_smem<C>(d.nz, d.plz.n1, d.zirows) <= kBlockSmem;
+}
+
 // inverse z transform (Hermitian half spectrum -> real); mode 0 adds the
 // result to the symmetric displacement gradient (evolution.c:383-394),
 // mode 1 writes it (scaled by 1/N) to rotl, mode 2 (scaled by 1/N) to
@@ -916,6 +939,10 @@ __device__ void fft_z_inv_unit(const RveDesc &d, void *specp, int ncomp, int row
     const double inv = d.inv_nv;
     if (mode == 0) {
         const MacroDev *m = d.macro;
+        // on the register FFT, the arithmetic of zi_unit's add_update
+        bool direct = d.plz.n1 > 0;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) direct = direct && m->ddg6[c] == 0.0;
         // element (z, r, c) is dgs[c][vb + r * nz + z]
         staged_copy3<kZCopyDepth, double>(
             ncomp * rows * nz, nz, rows,
@@ -923,7 +950,8 @@ __device__ void fft_z_inv_unit(const RveDesc &d, void *specp, int ncomp, int row
             [&](int z, int r, int c, double old) {
                 const C e = res[z * ldl + (c >> 1) * rows + r];
                 const double val = (double)((c & 1) ? e.y : e.x);
-                d.dgs[(long long)c * nv + vb + (long long)r * nz + z] = old + (m->ddg6[c] + val * inv);
+                d.dgs[(long long)c * nv + vb + (long long)r * nz + z] =
+                    direct ? fma(val, inv, old) : old + fma(val, inv, m->ddg6[c]);
             });
     } else if (mode == 1) {
         Idx3 iz(threadIdx.x, blockDim.x, nz, rows);
@@ -989,7 +1017,7 @@ kb_fft_z_fwd(const RveDesc *descs, const int2 *map, int total)
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, MASK_ACTIVE)) continue;
         typedef typename Cx<R>::T C;
-        if (d.plz.n1 > 0) {
+        if (zf_fits<C>(d)) {
 #define VOCE_CALL(N1, N2) if constexpr (N1 * N2 % 2 == 0) zf_unit<C, N1, N2>(d, d.zrows, e.y)   /* nz is even */
             VOCE_REG_SPLITS(d.nz, VOCE_CALL)
 #undef VOCE_CALL
@@ -1120,7 +1148,7 @@ kb_fft_x_green(const RveDesc *descs, const int2 *map, int total)
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, MASK_ACTIVE)) continue;
         typedef typename Cx<R>::T C;
-        if (d.plx.n1 > 0) {
+        if (xg_fits<C>(d)) {
 #define VOCE_CALL(N1, N2) xg_unit<C, N1, N2>(d, d.xkc, e.y)
             VOCE_REG_SPLITS(d.nx, VOCE_CALL)
 #undef VOCE_CALL
@@ -1153,7 +1181,7 @@ kb_fft_z_inv(const RveDesc *descs, const int2 *map, int total, int mode)
         const RveDesc &d = descs[e.x];
         if (!unit_on(d, mode == 0 ? MASK_ACTIVE : MASK_CONVERGED)) continue;
         typedef typename Cx<R>::T C;
-        if (mode == 0 && d.plz.n1 > 0) {
+        if (mode == 0 && zi_fits<C>(d)) {
 #define VOCE_CALL(N1, N2) if constexpr (N1 * N2 % 2 == 0) zi_unit<C, N1, N2>(d, d.zirows, e.y)
             VOCE_REG_SPLITS(d.nz, VOCE_CALL)
 #undef VOCE_CALL

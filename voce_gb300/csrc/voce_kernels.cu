@@ -2312,9 +2312,13 @@ static size_t batch_smem_t(const RveDesc &d, int ph)
 {
     typedef typename Cx<R>::T C;
     // the register-FFT z and Green passes, the staged single-precision z passes
-    if (ph == BP_ZF && d.plz.n1 > 0) return zf_smem<C>(d.nz, d.plz.n1, d.zrows);
-    if (ph == BP_ZI && d.plz.n1 > 0) return zi_smem<C>(d.nz, d.plz.n1, d.zirows);
-    if (ph == BP_XG && d.plx.n1 > 0) return xg_smem<C>(d.nx, d.plx.n1, d.xkc);
+    // where the tile fits in their layout
+    if (ph == BP_ZF && zf_fits<C>(d)) return zf_smem<C>(d.nz, d.plz.n1, d.zrows);
+    if (ph == BP_ZI && zi_fits<C>(d)) return zi_smem<C>(d.nz, d.plz.n1, d.zirows);
+    if (ph == BP_XG && xg_fits<C>(d)) return xg_smem<C>(d.nx, d.plx.n1, d.xkc);
+    // (the single-precision forms' own lengths always had that layout along x:
+    // a tile too large for it is refused)
+    if (ph == BP_XG && sizeof(R) == 4 && d.plx.n1 > 0 && reg_fft_split(d.nx)) return xg_smem<C>(d.nx, d.plx.n1, d.xkc);
     if (sizeof(R) == 4) {
         if (ph == BP_ZF) return sizeof(float2) * (size_t)zf32_fwd_size(d.nz, d.zrows);
         if (ph == BP_ZI) return sizeof(float2) * (size_t)zi32_size(d.nz, d.nzh, d.zirows);
@@ -2509,6 +2513,18 @@ static int tile_units(const RveDesc &d, int phase, int t)
     }
 }
 
+// an axis on the register FFT whose tile goes through fft_lines all the same
+template <typename C>
+static bool off_layout(const RveDesc &d, int phase)
+{
+    switch (phase) {
+    case BP_ZF: return d.plz.n1 > 0 && !zf_fits<C>(d);
+    case BP_XG: return d.plx.n1 > 0 && !xg_fits<C>(d);
+    case BP_ZI: return d.plz.n1 > 0 && !zi_fits<C>(d);
+    default: return false;
+    }
+}
+
 int tile_candidates(const RveDesc &d, int phase, int *out, int max)
 {
     const bool f = d.mixed != 0;
@@ -2532,8 +2548,10 @@ int tile_candidates(const RveDesc &d, int phase, int *out, int max)
         case BP_ZI: t = dt.zirows = pick_div(d.ny, budget / (3 * d.nz)); break;
         default: return 0;
         }
-        const size_t sm = batch_smem(dt, phase);
-        if (t < 1 || sm > smem_max) continue;
+        if (t < 1 || batch_smem(dt, phase) > smem_max) continue;
+        // only in the register FFT's own layout, where the axis has one
+        const bool off = f ? off_layout<float2>(dt, phase) : off_layout<double2>(dt, phase);
+        if (off) continue;
         bool seen = false;
         for (int i = 0; i < n; ++i) seen = seen || out[i] == t;
         if (!seen) out[n++] = t;
