@@ -129,6 +129,7 @@ PROTOTYPES = [
     ("voce_device_memory", C.c_int, [C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]),
     ("voce_diag_rcp", C.c_int, [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int]),
     ("voce_diag_sqrt", C.c_int, [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int]),
+    ("voce_diag_convert", C.c_int, [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int]),
     ("voce_diag_fft", C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
     # voce_batch.h
     ("voce_batch_create", C.c_int, [C.c_int, C.POINTER(C.c_void_p)]),
@@ -310,6 +311,15 @@ def diag_sqrt(x: np.ndarray) -> np.ndarray:
     out = np.empty_like(x)
     _check(load().voce_diag_sqrt(_dptr(x), _dptr(out), x.size))
     return out
+
+
+def diag_convert(x: np.ndarray):
+    """x truncated to float, x rounded to float, and the double of np.float32(x),
+    by the device's integer conversions (voce_diag_convert)."""
+    x = np.ascontiguousarray(x, dtype=np.float64).ravel()
+    out = np.empty((3, x.size))
+    _check(load().voce_diag_convert(_dptr(x), _dptr(out), x.size))
+    return out[0], out[1], out[2]
 
 
 def diag_rcp(x: np.ndarray) -> np.ndarray:

@@ -369,7 +369,8 @@ __device__ __forceinline__ int itau_col(const RveDesc &d, int k, int f)
     return d.fcc ? 2 * d.canon[k] + (f ^ d.flip[k]) : 2 * k + f;
 }
 
-// x = h + l to about 2^-47 (h truncated): l from the 29 significand bits below h
+// x = h + l to about 2^-47 (h truncated): l from the 29 significand bits below
+// h.  |x| < 2^128 (the callers' residual and ratio tests see to it)
 __device__ __forceinline__ ff32 d2ff(double x)
 {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
@@ -571,7 +572,8 @@ __device__ __forceinline__ bool fcc_newton_f32(const RveDesc &d, long long v, co
 
 // One step on the float-float residual (residual_ff's accuracy, about 48
 // bits) from the single-precision point y with the factors L; x receives the
-// correction.  False when a ratio leaves the float range.
+// correction.  False when a ratio leaves the float range or the correction is
+// not finite.
 __device__ __forceinline__ bool fcc_step_ff(const RveDesc &d, long long v, const float (&y)[5], const double (&cc)[5],
                                             const float (&P)[15], const float (&L)[15], float dtgh, float dtgl,
                                             float (&x)[5])
@@ -594,7 +596,7 @@ __device__ __forceinline__ bool fcc_step_ff(const RveDesc &d, long long v, const
 #pragma unroll
     for (int i = 0; i < 5; ++i) x[i] = t[i].h + t[i].l;
     fcc_solve<float>(L, x);
-    return true;
+    return finite_f((x[0] + x[1]) + (x[2] + x[3]) + x[4]);
 }
 
 // ---------------------------------------------------------------------------
@@ -751,7 +753,7 @@ __device__ __forceinline__ bool fcc_solve_ff(const RveDesc &d, long long v, cons
 #pragma unroll
     for (int c = 0; c < 5; ++c) {
         ok = ok && fabsf(b[c].h) < 1e30f;
-        xd[c] = f2d(b[c].h) + f2d(b[c].l);
+        xd[c] = f2d(b[c].h) + f2d(b[c].l);   // (finite, or not taken)
     }
     return ok;
 }

@@ -655,7 +655,8 @@ static __device__ void fft_z_inv_dgs_f32(const RveDesc &d, int rows, int unit)
     for (int i = threadIdx.x; i < 6 * run; i += blockDim.x, iz.next()) {
         const int z = iz.a0, r = iz.a1, c = iz.a2;
         const float2 e = res[z * ldl + (c >> 1) * rows + r];
-        double val = f2d(((c & 1) ? e.y : e.x) * inv);
+        const float vf = ((c & 1) ? e.y : e.x) * inv;
+        double val = finite_f(vf) ? f2d(vf) : (double)vf;
         if (mean) val += m->ddg6[c];
         d.dgs[(long long)c * nv + vb + (long long)r * nz + z] = D[i] + val;
     }
@@ -754,13 +755,14 @@ __host__ __device__ inline size_t zf_smem(int nz, int n1, int rows)
 }
 
 // the inverse pass into the symmetric displacement gradient (evolution.c:383-394)
-template <bool MEAN>
+template <bool MEAN, bool FINITE>
 __device__ __forceinline__ double add_update(double old, float v, float inv, double m)
 {
-    const double x = f2d(v * inv);   // (the product exact for a power-of-two number of voxels)
+    const float f = v * inv;   // (exact for a power-of-two number of voxels)
+    const double x = FINITE ? f2d(f) : (double)f;
     return MEAN ? old + (x + m) : old + x;
 }
-template <bool MEAN>
+template <bool MEAN, bool FINITE>
 __device__ __forceinline__ double add_update(double old, double v, double inv, double m)
 {
     return MEAN ? old + fma(v, inv, m) : fma(v, inv, old);
@@ -786,11 +788,17 @@ __device__ __forceinline__ void zi_pass2(const RveDesc &d, const C *W, const dou
         const double *o = D + 2 * p * run + r * L + k1;
         double *g = d.dgs + 2 * p * nv + vb + r * L + k1;
         const double m0 = MEAN ? m->ddg6[2 * p] : 0.0, m1 = MEAN ? m->ddg6[2 * p + 1] : 0.0;
-        sfor<0, N2>([&](auto mc) {
-            constexpr int q = N1 * decltype(mc)::v, e = dft_pos(N2, decltype(mc)::v);
-            g[q] = add_update<MEAN>(o[q], v[e].x, inv, m0);
-            g[nv + q] = add_update<MEAN>(o[run + q], v[e].y, inv, m1);
-        });
+        auto put = [&](auto finite) {
+            sfor<0, N2>([&](auto mc) {
+                constexpr int q = N1 * decltype(mc)::v, e = dft_pos(N2, decltype(mc)::v);
+                g[q] = add_update<MEAN, decltype(finite)::v>(o[q], v[e].x, inv, m0);
+                g[nv + q] = add_update<MEAN, decltype(finite)::v>(o[run + q], v[e].y, inv, m1);
+            });
+        };
+        // X[0] is the sum of the inputs: it is finite only if all of them are
+        // (single precision converts finite values alone by their bits)
+        if (sizeof(R) == 8 || finite_f((float)v[0].x + (float)v[0].y)) put(IC<1>());
+        else put(IC<0>());
     }
 }
 

@@ -1172,8 +1172,13 @@ __device__ __forceinline__ void fcc_newton_ir(const RveDesc &d, long long v, boo
 #pragma unroll
                 for (int c = 0; c < 5; ++c) xf[c] = d2f(x[c]);
                 fcc_solve<float>(L, xf);
+                // a correction that is not finite in float (a residual beyond
+                // the floats or broken, or an overflowed Jacobian) is solved
+                // in FP64, where it stays what it is
+                fp64 = !finite_f((xf[0] + xf[1]) + (xf[2] + xf[3]) + xf[4]);
+                if (!fp64)
 #pragma unroll
-                for (int c = 0; c < 5; ++c) x[c] = f2d(xf[c]);
+                    for (int c = 0; c < 5; ++c) x[c] = f2d(xf[c]);
             }
         }
         if (fp64) fcc_rare_step(d, v, y, x);
@@ -1432,7 +1437,11 @@ __device__ void finalize_iter_body(const RveDesc &d, MacroDev *m, const double *
         const double r = rsqrt(x);
         // sum wgt / (wgt sqrt(x)), and sum wgt / e_vm
         const double err = lane == 2 ? (tot[1] * d.wgt) * r : tot[0] * r;
-        const double svm = x > 0.0 ? (x * r) * (lane == 1 ? d.wgt_ratio : d.wgt) : 0.0;
+        // sqrt(x) as x / sqrt(x): 0 and infinity are their own roots (x is never
+        // negative, NaN stays; tested on the integer pipe)
+        const long long xb = __double_as_longlong(x);
+        const double root = xb == 0 || xb == 0x7ff0000000000000LL ? x : x * r;
+        const double svm = root * (lane == 1 ? d.wgt_ratio : d.wgt);
         const double Err_s = __shfl_sync(0xffffffffu, err, 0), Err_e = __shfl_sync(0xffffffffu, err, 2);
         const double s_vm = __shfl_sync(0xffffffffu, svm, 0);
         const bool more = (it + 1 < d.iter_max) &&
@@ -2745,6 +2754,25 @@ __global__ void k_sqrt_probe(const double *__restrict__ x, double *__restrict__ 
 cudaError_t launch_sqrt_probe(const double *x, double *out, int n, cudaStream_t s)
 {
     if (n > 0) k_sqrt_probe<<<(n + 255) / 256, 256, 0, s>>>(x, out, n);
+    return cudaGetLastError();
+}
+
+// out[0..n): d2f, out[n..2n): d2f_rn, out[2n..3n): f2d of (float)x where that
+// is finite, (float)x itself where it is not
+__global__ void k_convert_probe(const double *__restrict__ x, double *__restrict__ out, int n)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        out[i] = (double)d2f(x[i]);
+        out[n + i] = (double)d2f_rn(x[i]);
+        const float f = (float)x[i];
+        out[2 * n + i] = finite_f(f) ? f2d(f) : (double)f;
+    }
+}
+
+cudaError_t launch_convert_probe(const double *x, double *out, int n, cudaStream_t s)
+{
+    if (n > 0) k_convert_probe<<<(n + 255) / 256, 256, 0, s>>>(x, out, n);
     return cudaGetLastError();
 }
 
