@@ -2688,12 +2688,18 @@ cudaError_t launch_fill_p32(const RveDesc &d, cudaStream_t s)
     return cudaGetLastError();
 }
 
-// the crystal-axes columns of every solid voxel, once S0 is known
+// the crystal-axes columns of every solid voxel, once S0 is known; gas voxels,
+// which nothing reads but a snapshot, hold zeros (k_setup writes theirs in the
+// other arrays)
 __global__ void __launch_bounds__(128) k_fill_fcc(RveDesc d)
 {
     for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < d.nv;
          v += (long long)gridDim.x * blockDim.x) {
-        if (!d.solid[d.phase[v]]) continue;
+        if (!d.solid[d.phase[v]]) {
+            if (d.sgp32)
+                for (int q = 0; q < 15; ++q) put_ff(d.sgp32, d.sgp_lo, q * d.nv + v, 0.0);
+            continue;
+        }
         double T[3][3];
         for (int i = 0; i < 3; ++i)
             for (int j = 0; j < 3; ++j) T[i][j] = d.tm[(3 * i + j) * d.nv + v];
