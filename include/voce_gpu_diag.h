@@ -66,11 +66,13 @@ int voce_diag_rcp(const double *x, double *out, int n);
  * reference. */
 int voce_diag_sqrt(const double *x, double *out, int n);
 /* The conversions between double and float that the single-precision passes
- * make with integer operations, on the current device for n host values:
- * out[0..n) x truncated to float, out[n..2n) x rounded to the nearest float (a
- * tie away from zero), both infinite or NaN where x is not finite or lies
- * beyond the floats, and below 2^-126 where x does; out[2n..3n) the double of
- * (float)x, a subnormal one as zero.  No counterpart in the reference. */
+ * and the float-pair arithmetic make with integer operations, on the current
+ * device for n host values: out[0..n) x rounded to the nearest float (a tie
+ * away from zero), infinite or NaN where x is not finite or lies beyond the
+ * floats, and at most 2^-126 where |x| is below that; out[n..2n) the double of
+ * (float)x, a subnormal one as zero; out[2n..3n) the sum and out[3n..4n) the
+ * leading float of the pair that stands for x (|x| < 2^128).  No counterpart
+ * in the reference. */
 int voce_diag_convert(const double *x, double *out, int n);
 /* The single-precision line FFT of the spectrum passes on the current
  * device: nlines lines of length L, in and out [nlines][L] complex values as

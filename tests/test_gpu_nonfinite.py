@@ -24,32 +24,35 @@ def test_conversions_over_the_whole_double_range(voce_lib):
                          np.nextafter(2.0 ** -126, 0.0), np.nextafter(2.0 ** 128, 0.0),
                          float(np.finfo(np.float32).max), 1.7976931348623157e308]])
     x = np.concatenate([x, -x])
-    rz, rn, back = capi.diag_convert(x)
+    rn, back, pair, head = capi.diag_convert(x)
     with np.errstate(over="ignore"):
         f = x.astype(np.float32)
     lo, hi = 2.0 ** -126, 2.0 ** 128
     big = ~(np.abs(x) < hi)                                    # NaN, infinity, beyond the floats
-    assert not np.isfinite(rz[big]).any() and not np.isfinite(rn[big]).any()
+    assert not np.isfinite(rn[big]).any()
     assert not np.isfinite(back[~np.isfinite(f)]).any()
     small = np.abs(x) < lo
-    assert (np.abs(rz[small]) < lo).all() and (np.abs(rn[small]) <= lo).all()
-    assert np.all(rz[x == 0.0] == 0.0) and np.all(rn[x == 0.0] == 0.0)
+    assert (np.abs(rn[small]) <= lo).all() and np.all(rn[x == 0.0] == 0.0)
     n = ~big & ~small
     fn = f[n].astype(np.float64)
     assert n.sum() > 2000
     assert np.array_equal(rn[n], fn)                           # (no value is a tie)
-    down = np.where(np.abs(fn) > np.abs(x[n]), np.nextafter(f[n], np.float32(0)), f[n]).astype(np.float64)
-    assert np.array_equal(rz[n], down)                         # toward zero
     normal = np.isfinite(f) & (np.abs(f) >= lo)
     assert np.array_equal(back[normal], f[normal].astype(np.float64))
     assert np.all(back[np.abs(f) < lo] == 0.0)
     s = ~np.isnan(x)
-    assert np.array_equal(np.signbit(rn[s]), np.signbit(x[s])) and np.array_equal(np.signbit(rz[s]), np.signbit(x[s]))
+    assert np.array_equal(np.signbit(rn[s]), np.signbit(x[s]))
+    # the float pair: the nearest float, and a remainder (at most 2^-24 of x's
+    # power of two) rounded to a float's 24 bits
+    p = (np.abs(x) >= 2.0 ** -74) & (np.abs(x) < np.nextafter(hi, 0.0))
+    assert np.array_equal(head[p], f[p].astype(np.float64))
+    assert np.all(np.abs(pair[p] - x[p]) <= 2.0 ** -49 * np.abs(x[p]))
 
 
 def test_a_tie_rounds_away_from_zero(voce_lib):
     x = np.array([1.0 + 2.0 ** -24, -1.0 - 3 * 2.0 ** -24, 2.0 - 2.0 ** -24])
-    _, rn, _ = capi.diag_convert(x)
+    rn, _, pair, head = capi.diag_convert(x)
+    assert head.tolist() == rn.tolist() and pair.tolist() == x.tolist()
     assert rn.tolist() == [1.0 + 2.0 ** -23, -1.0 - 2.0 ** -22, 2.0]
 
 

@@ -314,12 +314,13 @@ def diag_sqrt(x: np.ndarray) -> np.ndarray:
 
 
 def diag_convert(x: np.ndarray):
-    """x truncated to float, x rounded to float, and the double of np.float32(x),
-    by the device's integer conversions (voce_diag_convert)."""
+    """By the device's integer conversions (voce_diag_convert): x rounded to
+    float, the double of np.float32(x), the sum and the leading float of x's
+    float pair."""
     x = np.ascontiguousarray(x, dtype=np.float64).ravel()
-    out = np.empty((3, x.size))
+    out = np.empty((4, x.size))
     _check(load().voce_diag_convert(_dptr(x), _dptr(out), x.size))
-    return out[0], out[1], out[2]
+    return out[0], out[1], out[2], out[3]
 
 
 def diag_rcp(x: np.ndarray) -> np.ndarray:

@@ -2272,10 +2272,10 @@ int voce_diag_convert(const double *x, double *out, int n)
     if (n < 0 || (n > 0 && (!x || !out))) return fail(VOCE_ERR_ARG, "bad argument");
     if (n == 0) return VOCE_OK;
     double *d = nullptr;
-    CUDA_TRY(cudaMalloc(&d, sizeof(double) * 4 * (size_t)n));
+    CUDA_TRY(cudaMalloc(&d, sizeof(double) * 5 * (size_t)n));
     cudaError_t e = cudaMemcpy(d, x, sizeof(double) * n, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = launch_convert_probe(d, d + n, n, 0);
-    if (e == cudaSuccess) e = cudaMemcpy(out, d + n, sizeof(double) * 3 * (size_t)n, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + n, sizeof(double) * 4 * (size_t)n, cudaMemcpyDeviceToHost);
     cudaFree(d);
     if (e != cudaSuccess) return fail(VOCE_ERR_CUDA, "convert probe: %s", cudaGetErrorString(e));
     return VOCE_OK;

@@ -209,13 +209,6 @@ __device__ __forceinline__ unsigned float_hi(unsigned hi)
     return (unsigned)max(min(w, 0x0ff80000), 0);
 }
 
-// x truncated
-__device__ __forceinline__ float d2f(double x)
-{
-    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    return __uint_as_float(__funnelshift_l(lo, float_hi(hi), 3) | (hi & 0x80000000u));
-}
-
 // x rounded to nearest (a tie away from zero)
 __device__ __forceinline__ float d2f_rn(double x)
 {

@@ -1036,7 +1036,7 @@ __device__ void nr_unit(const RveDesc &d, int unit, int nunits)
 // last matrix; 64^3 363 -> 213 us, 256^3 29.9 -> 14.6 ms.  FCC_NR32
 // (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 306 us.  Nothing is staged
 // in shared memory: the single-precision steps read 15 + 12 floats per voxel
-// instead of 21 + 72.  Conversions go through the integer pipe (d2f, f2d:
+// instead of 21 + 72.  Conversions go through the integer pipe (d2f_rn, f2d:
 // with the hardware's, 239 and 331 us).
 //
 // kb_nr stays for every other slip table and for non-integral exponents.
@@ -1170,7 +1170,7 @@ __device__ __forceinline__ void fcc_newton_ir(const RveDesc &d, long long v, boo
             }
             if (!fp64) {
 #pragma unroll
-                for (int c = 0; c < 5; ++c) xf[c] = d2f(x[c]);
+                for (int c = 0; c < 5; ++c) xf[c] = d2f_rn(x[c]);
                 fcc_solve<float>(L, xf);
                 // a correction that is not finite in float (a residual beyond
                 // the floats or broken, or an overflowed Jacobian) is solved
@@ -1263,7 +1263,7 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
 #pragma unroll
                 for (int q = 0; q < 15; ++q) P[q] = __ldg(d.sgp32 + (long long)q * nv + v);
 #pragma unroll
-                for (int c = 0; c < 5; ++c) { yf[c] = d2f(yl[c]); ccf[c] = d2f(cc[c]); }
+                for (int c = 0; c < 5; ++c) { yf[c] = d2f_rn(yl[c]); ccf[c] = d2f_rn(cc[c]); }
                 // before a float-float step single precision stops at a
                 // relative update of 1e-4 (its rounding floor can lie near
                 // 1e-5), alone at 1e-5
@@ -1304,9 +1304,9 @@ __device__ void nr_fcc_unit(const RveDesc &d, int unit, int nunits)
             // in single precision: they only steer the Green iteration's stop
             // test at 1e-5
             float dy[5], te[5] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
-            float d5 = d2f(s5 - s5l), r5 = 0.0f;
+            float d5 = d2f_rn(s5 - s5l), r5 = 0.0f;
 #pragma unroll
-            for (int c = 0; c < 5; ++c) dy[c] = d2f(y[c] - yl[c]);
+            for (int c = 0; c < 5; ++c) dy[c] = d2f_rn(y[c] - yl[c]);
             ncs = (double)sqrtf(fmaf(d5, d5, fcc_norm2<float>(dy)));
             if (!converged) {   // (a point taken as converged: yp = y, no residual)
 #pragma unroll
@@ -2763,16 +2763,19 @@ cudaError_t launch_sqrt_probe(const double *x, double *out, int n, cudaStream_t 
     return cudaGetLastError();
 }
 
-// out[0..n): d2f, out[n..2n): d2f_rn, out[2n..3n): f2d of (float)x where that
-// is finite, (float)x itself where it is not
+// out[0..n): d2f_rn, out[n..2n): f2d of (float)x where that is finite, (float)x
+// itself where it is not, out[2n..3n): the sum and out[3n..4n): the first
+// part of the float pair d2ff
 __global__ void k_convert_probe(const double *__restrict__ x, double *__restrict__ out, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        out[i] = (double)d2f(x[i]);
-        out[n + i] = (double)d2f_rn(x[i]);
         const float f = (float)x[i];
-        out[2 * n + i] = finite_f(f) ? f2d(f) : (double)f;
+        const ff32 p = d2ff(x[i]);
+        out[i] = (double)d2f_rn(x[i]);
+        out[n + i] = finite_f(f) ? f2d(f) : (double)f;
+        out[2 * n + i] = (double)p.h + (double)p.l;
+        out[3 * n + i] = (double)p.h;
     }
 }
 
