@@ -78,9 +78,12 @@ int voce_diag_convert(const double *x, double *out, int n);
  * device: nlines lines of length L, in and out [nlines][L] complex values as
  * interleaved (re, im) doubles (rounded to float on the way in), transformed
  * by candidate `schedule` of a single-precision axis of length L (see the
- * schedules below; 0 is the default), sign -1 forward, +1 inverse,
- * unnormalised.  2 L (nlines | 1) complex floats must fit in 200 KB. */
+ * schedules below; 0 is the default, and -1 the default Stockham order where
+ * the default runs the register FFT in its place), sign -1 forward, +1
+ * inverse, unnormalised.  2 L (nlines | 1) complex numbers must fit in 200 KB.
+ * voce_diag_fft64: the same of an FP64 axis. */
 int voce_diag_fft(int L, int nlines, int sign, int schedule, const double *in, double *out);
+int voce_diag_fft64(int L, int nlines, int sign, int schedule, const double *in, double *out);
 
 /* FFT tile tuning.  voce_rve_create times the forward-pass FFT phases with
  * a few tile sizes (lines per block) on the new RVE and keeps the fastest,
@@ -112,9 +115,13 @@ int voce_fft_smem(const int dims[3], int precision, const int tiles[6], long lon
  * 256 has one more candidate, placed first: the register FFT, two passes of
  * small DFTs of lengths N1 x N2 = L held in registers (4x4, 4x6, 4x8, 6x8,
  * 8x8, 8x12, 8x16, 12x16, 16x16).  Candidate 0 is the default.
- * In the FP64 form candidate 0 of those lengths, and in every form candidate 0
- * of 8, 12, 18, 27, 36, 54, 72, 81, 108 and 144, is computed by the register
- * FFT too; it is counted and reported as the default Stockham order.
+ * On the other axes candidate 0 is the default Stockham order, and the register
+ * FFT stands in for it where it has the length: in the FP64 form those
+ * lengths, in every form 8, 12, 18, 27, 36, 54, 72, 81, 108 and 144.  An axis
+ * that nobody set then runs the register FFT, while the order's radices are
+ * what voce_rve_get_fft_schedule reports; voce_rve_get_fft_split tells which
+ * of the two runs, and voce_rve_set_fft_schedule(r, axis, 0) runs the order's
+ * stages themselves.
  * Unlike the tiles, the schedule changes results in the last bits (a
  * different order of roundings).  So the FP64 form never tunes it: its RVEs
  * run the default schedule of every axis unless the caller sets one, and its
@@ -165,6 +172,9 @@ int voce_set_newton_chord(int on);
  * Green iterate.  On (1) by default; applies to RVEs created afterwards. */
 int voce_set_ir_predictor(int on);
 int voce_rve_get_fft_schedule(const voce_rve *r, int axis, int *radices, int max);
+/* N1 where axis runs the register FFT of L = N1 x (L / N1), 0 where it runs
+ * Stockham stages, < 0 on error. */
+int voce_rve_get_fft_split(const voce_rve *r, int axis);
 int voce_rve_set_fft_schedule(voce_rve *r, int axis, int k);
 
 #ifdef __cplusplus

@@ -29,7 +29,14 @@ def _create(dims, prec, seed, mixed_load=True):
     slip.tau0f, slip.tau0b, slip.tau1, slip.thet0, slip.thet1 = m.tau0f, m.tau0b, m.tau1, m.thet0, m.thet1
     for k, (n, b) in enumerate(synth.FCC_111_110):
         slip.bn[k][:], slip.bb[k][:] = n, b
-    return capi.Rve.create(nl, slip, mesh.euler_deg, mesh.grain, mesh.phase, prec)
+    # the single-precision forms' timed schedules change the rounding: their
+    # defaults, with the fixed-budget tiles; the FP64 form with the timed tiles
+    lib = capi.load()
+    lib.voce_set_autotune(int(prec == capi.PREC_FP64))
+    try:
+        return capi.Rve.create(nl, slip, mesh.euler_deg, mesh.grain, mesh.phase, prec)
+    finally:
+        lib.voce_set_autotune(1)
 
 
 def _solve(r):
@@ -47,15 +54,9 @@ def _solve(r):
 ])
 def test_long_x_edges_over_short_y_edges(dims, prec, yxt, voce_lib):
     with _create(dims, prec, 96) as r:
-        if prec != capi.PREC_FP64:             # the timed schedules aside, which change the rounding
-            for a in range(3):
-                r.set_fft_schedule(a, 0)
         want = _solve(r)
         assert np.all(np.isfinite(want[1]))
     with _create(dims, prec, 96) as r:
-        if prec != capi.PREC_FP64:
-            for a in range(3):
-                r.set_fft_schedule(a, 0)
         t = r.tiles()
         for ty in (yxt, 1):                    # past the stream's size, and a small one
             t[1] = ty
@@ -78,9 +79,7 @@ def test_long_x_edges_over_short_y_edges(dims, prec, yxt, voce_lib):
 @pytest.mark.parametrize("mixed_load", [False, True])     # with and without a mean correction of the gradient
 def test_tiles_beyond_the_register_layout(dims, prec, tiles, mixed_load, voce_lib):
     with _create(dims, prec, 97, mixed_load) as r:
-        for a in range(3):
-            if prec != capi.PREC_FP64:
-                r.set_fft_schedule(a, 0)
+        assert all(r.fft_split(a) > 0 for a in range(3))
         t = r.tiles()
         got = []
         for use in (tiles, [1, 1, 1, 1]):

@@ -131,6 +131,7 @@ PROTOTYPES = [
     ("voce_diag_sqrt", C.c_int, [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int]),
     ("voce_diag_convert", C.c_int, [C.POINTER(C.c_double), C.POINTER(C.c_double), C.c_int]),
     ("voce_diag_fft", C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
+    ("voce_diag_fft64", C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p]),
     # voce_batch.h
     ("voce_batch_create", C.c_int, [C.c_int, C.POINTER(C.c_void_p)]),
     ("voce_batch_add", C.c_int, [C.c_void_p, C.c_void_p, C.c_int]),
@@ -171,6 +172,7 @@ PROTOTYPES = [
     ("voce_set_newton_chord", C.c_int, [C.c_int]),
     ("voce_set_ir_predictor", C.c_int, [C.c_int]),
     ("voce_rve_get_fft_schedule", C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.c_int]),
+    ("voce_rve_get_fft_split", C.c_int, [C.c_void_p, C.c_int]),
     ("voce_rve_set_fft_schedule", C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     ("voce_server_set_quantum", C.c_int, [C.c_void_p, C.c_int]),
     ("voce_server_set_active_limit", C.c_int, [C.c_void_p, C.c_longlong]),
@@ -331,12 +333,14 @@ def diag_rcp(x: np.ndarray) -> np.ndarray:
     return out
 
 
-def diag_fft(x: np.ndarray, sign: int = -1, schedule: int = 0) -> np.ndarray:
-    """The single-precision line FFT of the spectrum passes (voce_diag_fft)
-    of every row of the complex array x [nlines, L], unnormalised."""
+def diag_fft(x: np.ndarray, sign: int = -1, schedule: int = 0, fp64: bool = False) -> np.ndarray:
+    """The line FFT of the single-precision spectrum passes (voce_diag_fft), or
+    of the FP64 ones (voce_diag_fft64), of every row of the complex array
+    x [nlines, L], unnormalised."""
     x = np.ascontiguousarray(x, dtype=np.complex128)
     out = np.empty_like(x)
-    _check(load().voce_diag_fft(x.shape[1], x.shape[0], sign, schedule, x.ctypes.data, out.ctypes.data))
+    f = load().voce_diag_fft64 if fp64 else load().voce_diag_fft
+    _check(f(x.shape[1], x.shape[0], sign, schedule, x.ctypes.data, out.ctypes.data))
     return out
 
 
@@ -515,6 +519,14 @@ class Rve:
         if n < 0:
             _check(-n)
         return list(buf[:n])
+
+    def fft_split(self, axis: int) -> int:
+        """N1 where axis runs the register FFT of N1 x (L / N1), 0 where it
+        runs Stockham stages."""
+        n = load().voce_rve_get_fft_split(self._h, axis)
+        if n < 0:
+            _check(-n)
+        return n
 
     def set_fft_schedule(self, axis: int, k: int) -> None:
         _check(load().voce_rve_set_fft_schedule(self._h, axis, k))

@@ -249,6 +249,10 @@ int axis_schedules(int L, bool mixed, FftPlan1 *out, int max)
     return total;
 }
 
+// whether candidate 0 of an axis is a Stockham order in whose place the
+// default runs the register FFT
+bool stands_in(int L, bool mixed) { return reg_fft_any(L) && !(mixed && reg_fft_split(L)); }
+
 }  // namespace
 
 // ===========================================================================
@@ -1084,12 +1088,30 @@ int g_ir_predictor = 1;   // single-precision start of the FP64 steps in new VOC
 
 constexpr int kMaxSchedules = 5;
 
+// Schedule index of candidate 0 by its Stockham stages, on an axis where the
+// untouched default runs the register FFT in their place (voce_rve_set_fft_schedule).
+constexpr int kStockham0 = -1;
+
 // schedule index k of an axis of length L (the default when out of range)
 FftPlan1 schedule_of(int L, bool mixed, int k)
 {
     FftPlan1 c[kMaxSchedules];
     const int n = axis_schedules(L, mixed, c, kMaxSchedules);
+    if (k == kStockham0 && stands_in(L, mixed)) c[0].n1 = 0;
     return c[(k >= 0 && k < n) ? k : 0];
+}
+
+// the schedule index that makes plan p, or -2 when none does
+int schedule_index(const FftPlan1 &p, bool mixed)
+{
+    FftPlan1 c[kMaxSchedules];
+    const int n = axis_schedules(p.L, mixed, c, kMaxSchedules);
+    for (int k = 0; k < n; ++k) {
+        if (c[k].nst != p.nst || std::memcmp(c[k].rad, p.rad, sizeof(int) * c[k].nst) != 0) continue;
+        if (c[k].n1 == p.n1) return k;
+        if (k == 0 && p.n1 == 0 && stands_in(p.L, mixed)) return kStockham0;
+    }
+    return -2;
 }
 
 // the tiles and schedule indices an RVE descriptor runs (a restored RVE's)
@@ -1100,16 +1122,7 @@ Tiles tiles_of(const RveDesc &d)
     t.xkc3 = d.xkc3; t.zirows = d.zirows; t.zirows3 = d.zirows3;
     const FftPlan1 *pl[3] = {&d.plx, &d.ply, &d.plz};
     int *slot[3] = {&t.sx, &t.sy, &t.sz};
-    for (int a = 0; a < 3; ++a) {
-        FftPlan1 c[kMaxSchedules];
-        const int n = axis_schedules(pl[a]->L, d.mixed, c, kMaxSchedules);
-        for (int k = 0; k < n; ++k)
-            if (c[k].n1 == pl[a]->n1 && c[k].nst == pl[a]->nst &&
-                std::memcmp(c[k].rad, pl[a]->rad, sizeof(int) * c[k].nst) == 0) {
-                *slot[a] = k;
-                break;
-            }
-    }
+    for (int a = 0; a < 3; ++a) *slot[a] = std::max(schedule_index(*pl[a], d.mixed), kStockham0);
     return t;
 }
 
@@ -1754,15 +1767,8 @@ const char *snapshot_desc_problem(const SnapHead &h, const RveDesc &d, const voc
     // each axis runs one of its transform candidates
     const FftPlan1 *pl[3] = {&d.plx, &d.ply, &d.plz};
     const int L[3] = {d.nx, d.ny, d.nz};
-    for (int a = 0; a < 3; ++a) {
-        FftPlan1 c[kMaxSchedules];
-        const int n = axis_schedules(L[a], d.mixed != 0, c, kMaxSchedules);
-        bool found = false;
-        for (int k = 0; k < n && !found; ++k)
-            found = pl[a]->L == L[a] && c[k].n1 == pl[a]->n1 && c[k].nst == pl[a]->nst &&
-                    std::memcmp(c[k].rad, pl[a]->rad, sizeof(int) * c[k].nst) == 0;
-        if (!found) return "FFT schedule";
-    }
+    for (int a = 0; a < 3; ++a)
+        if (pl[a]->L != L[a] || schedule_index(*pl[a], d.mixed != 0) < kStockham0) return "FFT schedule";
     // the tiles: the rule voce_rve_set_tiles applies
     if (tiles_problem(d) >= 0) return "FFT tiles";
     if (h.npart < 1 || d.npart != h.npart || h.npart > std::max<long long>(1, (d.nv + 127) / 128))
@@ -2062,13 +2068,19 @@ int voce_rve_get_fft_schedule(const voce_rve *r, int axis, int *radices, int max
 {
     if (!r || axis < 0 || axis > 2) return -fail(VOCE_ERR_ARG, "bad argument");
     const FftPlan1 &p = axis == 0 ? r->d.plx : axis == 1 ? r->d.ply : r->d.plz;
-    if (p.n1 > 0 && r->d.mixed && reg_fft_split(p.L)) {   // the register FFT: its two passes
+    if (p.n1 > 0 && !stands_in(p.L, r->d.mixed)) {   // the register FFT: its two passes
         const int rr[2] = {p.n1, p.L / p.n1};
         for (int k = 0; k < 2 && k < max && radices; ++k) radices[k] = rr[k];
         return 2;
     }
     for (int k = 0; k < p.nst && k < max && radices; ++k) radices[k] = p.rad[k];
     return p.nst;
+}
+
+int voce_rve_get_fft_split(const voce_rve *r, int axis)
+{
+    if (!r || axis < 0 || axis > 2) return -fail(VOCE_ERR_ARG, "bad argument");
+    return (axis == 0 ? r->d.plx : axis == 1 ? r->d.ply : r->d.plz).n1;
 }
 
 int voce_rve_set_fft_schedule(voce_rve *r, int axis, int k)
@@ -2080,7 +2092,7 @@ int voce_rve_set_fft_schedule(voce_rve *r, int axis, int k)
     if (k < 0 || k >= n) return fail(VOCE_ERR_ARG, "schedule %d of %d for length %d", k, n, L);
     CUDA_TRY(cudaStreamSynchronize(r->stream));
     Tiles t = r->tiles;
-    (axis == 0 ? t.sx : axis == 1 ? t.sy : t.sz) = k;
+    (axis == 0 ? t.sx : axis == 1 ? t.sy : t.sz) = k == 0 && stands_in(L, r->d.mixed) ? kStockham0 : k;
     apply_tiles(r, t);
     if (r->graph_exec) { cudaGraphExecDestroy(r->graph_exec); r->graph_exec = nullptr; }
     if (r->graph) { cudaGraphDestroy(r->graph); r->graph = nullptr; }
@@ -2281,27 +2293,49 @@ int voce_diag_convert(const double *x, double *out, int n)
     return VOCE_OK;
 }
 
-int voce_diag_fft(int L, int nlines, int sign, int schedule, const double *in, double *out)
+}  // extern "C"
+
+namespace {
+
+template <typename C, typename R>
+int diag_fft(int L, int nlines, int sign, int schedule, const double *in, double *out)
 {
     if (nlines < 1 || (sign != 1 && sign != -1) || !in || !out) return fail(VOCE_ERR_ARG, "bad argument");
+    const bool f32 = sizeof(R) == 4;
     FftPlan1 c[kMaxSchedules];
-    const int n = axis_schedules(L, true, c, kMaxSchedules);
-    if (schedule < 0 || schedule >= n) return fail(VOCE_ERR_ARG, "schedule %d of %d for length %d", schedule, n, L);
-    if ((size_t)2 * L * (nlines | 1) * sizeof(float2) > 200 * 1024)
+    const int n = axis_schedules(L, f32, c, kMaxSchedules);
+    const bool stages = schedule == kStockham0 && stands_in(L, f32);
+    if (!stages && (schedule < 0 || schedule >= n))
+        return fail(VOCE_ERR_ARG, "schedule %d of %d for length %d", schedule, n, L);
+    if ((size_t)2 * L * (nlines | 1) * sizeof(C) > 200 * 1024)
         return fail(VOCE_ERR_ARG, "%d lines of length %d do not fit in shared memory", nlines, L);
     const size_t bytes = sizeof(double) * 2 * (size_t)L * nlines;
-    const auto tw = twiddles<float2, float>(L);
+    const auto tw = twiddles<C, R>(L);
     char *buf = nullptr;
-    CUDA_TRY(cudaMalloc(&buf, 2 * bytes + tw.size() * sizeof(float2)));
+    CUDA_TRY(cudaMalloc(&buf, 2 * bytes + tw.size() * sizeof(C)));
     double *din = reinterpret_cast<double *>(buf), *dout = reinterpret_cast<double *>(buf + bytes);
     void *dtw = buf + 2 * bytes;
     cudaError_t e = cudaMemcpy(din, in, bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(dtw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = launch_fft_probe(c[schedule], dtw, din, dout, nlines, sign, 0);
+    if (e == cudaSuccess) e = cudaMemcpy(dtw, tw.data(), tw.size() * sizeof(C), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = launch_fft_probe(schedule_of(L, f32, schedule), f32, dtw, din, dout, nlines, sign, 0);
     if (e == cudaSuccess) e = cudaMemcpy(out, dout, bytes, cudaMemcpyDeviceToHost);
     cudaFree(buf);
     if (e != cudaSuccess) return fail(VOCE_ERR_CUDA, "fft probe: %s", cudaGetErrorString(e));
     return VOCE_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int voce_diag_fft(int L, int nlines, int sign, int schedule, const double *in, double *out)
+{
+    return diag_fft<float2, float>(L, nlines, sign, schedule, in, out);
+}
+
+int voce_diag_fft64(int L, int nlines, int sign, int schedule, const double *in, double *out)
+{
+    return diag_fft<double2, double>(L, nlines, sign, schedule, in, out);
 }
 
 }  // extern "C"

@@ -1,4 +1,4 @@
-// The displacement fluctuation, and the probe of the single-precision line FFT.
+// The displacement fluctuation, and the probe of the line FFT.
 #include "voce_fft.cuh"
 
 namespace voce {
@@ -157,39 +157,48 @@ cudaError_t launch_disp_fluct(const RveDesc &d, void *work, double *out, cudaStr
     return d.mixed ? disp_fluct_t<float>(d, work, out, s) : disp_fluct_t<double>(d, work, out, s);
 }
 
-// One block transforms nl lines of length pl.L with the single-precision
-// line FFT of the spectrum passes: in and out are [nl][L] complex doubles,
-// rounded to float on the way in.
-__global__ void __launch_bounds__(256) k_fft_probe(FftPlan1 pl, const float2 *__restrict__ tw,
+// One block transforms nl lines of length pl.L with the line FFT of the
+// spectrum passes: in and out are [nl][L] complex doubles, rounded to R on
+// the way in.
+template <typename R>
+__global__ void __launch_bounds__(256) k_fft_probe(FftPlan1 pl, const typename Cx<R>::T *__restrict__ tw,
                                                    const double2 *__restrict__ in, double2 *__restrict__ out,
                                                    int nl, int sign)
 {
+    typedef typename Cx<R>::T C;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float2 *a = reinterpret_cast<float2 *>(smem_raw);
+    C *a = reinterpret_cast<C *>(smem_raw);
     const int L = pl.L, ldl = nl | 1;
-    float2 *b = a + L * ldl;
+    C *b = a + L * ldl;
     for (int e = threadIdx.x; e < nl * L; e += blockDim.x) {
         const int l = e / L, i = e - l * L;
-        a[i * ldl + l] = make_float2((float)in[e].x, (float)in[e].y);
+        a[i * ldl + l] = mkc<C>((R)in[e].x, (R)in[e].y);
     }
     __syncthreads();
-    const float2 *res = fft_lines<float>(a, b, nl, ldl, pl, tw, sign);
+    const C *res = fft_lines<R>(a, b, nl, ldl, pl, tw, sign);
     for (int e = threadIdx.x; e < nl * L; e += blockDim.x) {
         const int l = e / L, i = e - l * L;
-        const float2 v = res[i * ldl + l];
+        const C v = res[i * ldl + l];
         out[e] = make_double2(v.x, v.y);
     }
 }
 
-cudaError_t launch_fft_probe(const FftPlan1 &pl, const void *tw, const double *in, double *out, int nl, int sign,
-                             cudaStream_t s)
+template <typename R>
+static cudaError_t fft_probe_t(const FftPlan1 &pl, const void *tw, const double *in, double *out, int nl, int sign,
+                               cudaStream_t s)
 {
-    const size_t smem = (size_t)2 * pl.L * (nl | 1) * sizeof(float2);
-    cudaError_t e = cudaFuncSetAttribute((const void *)k_fft_probe, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    const size_t smem = smem_lines<R>(pl.L, nl);
+    cudaError_t e = cudaFuncSetAttribute((const void *)k_fft_probe<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    k_fft_probe<<<1, 256, smem, s>>>(pl, (const float2 *)tw, (const double2 *)in, (double2 *)out, nl, sign);
+    k_fft_probe<R><<<1, 256, smem, s>>>(pl, (const typename Cx<R>::T *)tw, (const double2 *)in, (double2 *)out, nl, sign);
     return cudaGetLastError();
+}
+
+cudaError_t launch_fft_probe(const FftPlan1 &pl, bool f32, const void *tw, const double *in, double *out, int nl,
+                             int sign, cudaStream_t s)
+{
+    return f32 ? fft_probe_t<float>(pl, tw, in, out, nl, sign, s) : fft_probe_t<double>(pl, tw, in, out, nl, sign, s);
 }
 
 }  // namespace voce

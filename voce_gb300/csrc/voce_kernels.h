@@ -147,10 +147,10 @@ double measure_fp64_tflops();
 cudaError_t launch_rcp_probe(const double *x, double *out, int n, cudaStream_t s);
 cudaError_t launch_sqrt_probe(const double *x, double *out, int n, cudaStream_t s);
 cudaError_t launch_convert_probe(const double *x, double *out, int n, cudaStream_t s);
-// nl lines of length pl.L through the single-precision line FFT (one block;
-// 2 L (nl | 1) complex floats of shared memory): in, out [nl][L] complex
-// doubles on the device, tw the length's float twiddles
-cudaError_t launch_fft_probe(const FftPlan1 &pl, const void *tw, const double *in, double *out, int nl, int sign,
+// nl lines of length pl.L through the line FFT in single (f32) or double
+// precision (one block; 2 L (nl | 1) complex numbers of shared memory): in,
+// out [nl][L] complex doubles on the device, tw the length's twiddles
+cudaError_t launch_fft_probe(const FftPlan1 &pl, bool f32, const void *tw, const double *in, double *out, int nl, int sign,
                              cudaStream_t s);
 cudaError_t launch_setup(const RveDesc &d, const SetupConst &sc, const double *euler, int npart,
                          cudaStream_t s);
