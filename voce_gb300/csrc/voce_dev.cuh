@@ -998,10 +998,10 @@ __device__ __forceinline__ void sdft(C (&x)[M])
         const C x0 = x[O], x1 = x[O + T], x2 = x[O + 2 * T];
         const C u = mkc<C>(x1.x + x2.x, x1.y + x2.y);
         const C w = mkc<C>(x1.x - x2.x, x1.y - x2.y);
-        const C m = mkc<C>(x0.x - R(0.5) * u.x, x0.y - R(0.5) * u.y);
+        const C m = mkc<C>(fma_(R(-0.5), u.x, x0.x), fma_(R(-0.5), u.y, x0.y));
         x[O] = mkc<C>(x0.x + u.x, x0.y + u.y);
-        x[O + T] = mkc<C>(m.x - s3 * w.y, m.y + s3 * w.x);
-        x[O + 2 * T] = mkc<C>(m.x + s3 * w.y, m.y - s3 * w.x);
+        x[O + T] = mkc<C>(fma_(-s3, w.y, m.x), fma_(s3, w.x, m.y));
+        x[O + 2 * T] = mkc<C>(fma_(s3, w.y, m.x), fma_(-s3, w.x, m.y));
     } else if constexpr (N == 4) {
         const C x0 = x[O], x1 = x[O + T], x2 = x[O + 2 * T], x3 = x[O + 3 * T];
         const C t0 = mkc<C>(x0.x + x2.x, x0.y + x2.y);
