@@ -63,7 +63,7 @@ DTYPE = {"fp64": "f64", "mixed": "f32 spectrum+f64 newton",
          "mixed_ir": "f32 spectrum+f64 newton residual+f32 newton correction",
          "mixed_ir_strict": "f32 spectrum+f64 newton residual+f32 newton correction",
          "mixed_nr32": "f32 spectrum+f32 newton+f64 acceptance"}
-FORM_DOC = {"mixed": "FP32 spectrum and Green operator; FP64 Newton, hardening, norms, averages",
+FORM_DOC = {"mixed": "FP32 spectrum and Green operator; Newton as in fp64; FP64 hardening, norms, averages",
             "mixed_ir": "FP32 spectrum and Green operator; Newton: FP32 steps choose the start, "
                         "then every accepted step evaluates the residual and flow rule in FP64 with "
                         "the FP64 stop test, its Jacobian and LDL^T correction in FP32; hardening, "
@@ -244,7 +244,7 @@ def measured_peaks():
 # written by one launch over 262144 voxels, and the FP64 flops (FMA = 2) per
 # Newton iteration of a voxel and per voxel per launch (instruction counts of 62
 # launches fitted against their Newton iterations).
-KB_NR_FP64_DRAM_BYTES = 228.1e6
+KB_NR_FP64_DRAM_BYTES = 228.3e6
 KB_NR_FP64_VOXELS = 262144
 KB_NR_FP64_FLOPS_PER_NEWTON = 212
 KB_NR_FP64_FLOPS_PER_VOXEL = 300.6
@@ -254,8 +254,8 @@ KB_NR_FP64_FLOPS_PER_VOXEL = 300.6
 # profiles/kb_nr_nr32_cfg2_64.md) and the mixed_ir form's (kb_nr_fcc<1>,
 # profiles/kb_nr_mixed_ir_cfg2_64.md); the mixed form runs the FP64 form's
 # kernel (profiles/kb_nr_mixed_cfg2_64.md).
-KB_NR_NR32_DRAM_BYTES = 244.4e6
-KB_NR_IR_DRAM_BYTES = 349.7e6
+KB_NR_NR32_DRAM_BYTES = 244.8e6
+KB_NR_IR_DRAM_BYTES = 350.3e6
 
 
 def profiled_traffic(precision="fp64"):

@@ -56,7 +56,12 @@ enum {
 };
 
 /* Precision forms.
- *   VOCE_PREC_FP64        the reference's arithmetic: FP64 throughout.
+ *   VOCE_PREC_FP64        every quantity in FP64.  One intermediate is not: for
+ *                         the {111}<110> slip family the Newton correction (the
+ *                         tangent, its LDL^T factors and the solve) is computed
+ *                         in pairs of floats, about 2^-44 an operation; the
+ *                         residual that judges every iterate, the flow rule, the
+ *                         stop test and the iterates are FP64.
  *   VOCE_PREC_MIXED       spectrum and Green-operator convolution in FP32; the
  *                         Newton-Raphson (the FP64 form's own code), the Voce
  *                         hardening, the averages and the error norms in FP64.

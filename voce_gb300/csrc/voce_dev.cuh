@@ -878,10 +878,12 @@ __host__ __device__ inline int reg_fft_split(int L)
     }
 }
 
-// The split of every length the register FFT can run: the ones above, and the
-// others below 256 whose factors the small DFTs have (2, 3, 4, 6, 8, 9, 12,
-// 16; an even length has an even N1).  Those run it in place of the default
-// Stockham order, under that order's name.
+// The split of every length the register FFT runs: the ones above, and the
+// other lengths of 8 to 256 with two factors that the small DFTs have (2, 3,
+// 4, 6, 8, 9, 12, 16; an even length has an even N1), but for 9 itself, which
+// like 2, 3, 4 and 6 keeps its one or two Stockham stages.  (162, 216 and 243
+// have no such factors.)  Those run it in place of the default Stockham order,
+// under that order's name.
 __host__ __device__ inline int reg_fft_any(int L)
 {
     switch (L) {

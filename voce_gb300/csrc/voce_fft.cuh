@@ -673,7 +673,7 @@ static __device__ void fft_z_inv_dgs_f32(const RveDesc &d, int rows, int unit)
 // each direction than through fft_lines and a tile needs two block barriers
 // fewer.  Everything is staged by asynchronous copies.
 // us per launch, forward / inverse, against the passes through fft_lines:
-// single precision 256^3 461 / 950 -> 376 / 645, 96^3 34 / 64 -> 28 / 42; FP64
+// single precision 256^3 461 / 950 -> 376 / 667, 96^3 34 / 64 -> 32 / 44; FP64
 // 128^3 359 / 408 -> 321 / 329.  Those passes stay for the Stockham stages
 // and for tiles that do not fit in a block in this layout (zf_fits, zi_fits).
 // ---------------------------------------------------------------------------

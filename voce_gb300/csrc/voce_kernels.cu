@@ -1025,16 +1025,16 @@ __device__ void nr_unit(const RveDesc &d, int unit, int nunits)
 // 72 for the powers, 25 for P y (the pressure decouples); the tangent and the
 // 5x5 solve, 240 + 125 there, run in float pairs on the FP32 pipe beside it.
 // Measured per launch against kb_nr (FP64 form, first increment): 64^3 879 ->
-// 343 us (477 with the solve in FP64), 128^3 10.4 -> 3.8 ms, 16^3 (a grain
-// per voxel) 86 -> 44 us.
+// 347 us (477 with the solve in FP64), 128^3 10.4 -> 3.8 ms, 16^3 (a grain
+// per voxel) 86 -> 46 us.
 // With the solve off the FP64 pipe a chord step saves nothing, so d.chord is
 // not looked at here.
 //
 // FCC_IR (VOCE_PREC_MIXED_IR): newton_ir in the same variables: the start in
 // single precision and float pairs, then steps whose residual, flow rule and
 // stop test are FP64 and whose correction is solved in FP32 with the start's
-// last matrix; 64^3 363 -> 213 us, 256^3 29.9 -> 14.6 ms.  FCC_NR32
-// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 306 us.  Nothing is staged
+// last matrix; 64^3 363 -> 214 us, 256^3 29.9 -> 14.8 ms.  FCC_NR32
+// (VOCE_PREC_MIXED_NR32): mixed_newton; 96^3 394 -> 315 us.  Nothing is staged
 // in shared memory: the single-precision steps read 15 + 12 floats per voxel
 // instead of 21 + 72.  Conversions go through the integer pipe (d2f_rn, f2d:
 // with the hardware's, 239 and 331 us).
@@ -1782,8 +1782,8 @@ __device__ __forceinline__ double tan_small(double x)
 // crystal axes and turned once (it was 12 products of 3 x 3 matrices), the
 // reorientation works on axial vectors, and the Voce factor, the same for all
 // systems of a slip mode, is computed once instead of twelve times.
-// Third increment (reorientation and hardening): 37 ms at 256^3 (mixed_ir),
-// 4.4 ms at 128^3 (FP64); the whole 256^3 increment of eight Green iterations
+// Third increment (reorientation and hardening): 35 ms at 256^3 (mixed_ir),
+// 4.3 ms at 128^3 (FP64); the whole 256^3 increment of eight Green iterations
 // went from 298 to 202 ms.
 // ---------------------------------------------------------------------------
 __device__ void incr_end_fcc_unit(const RveDesc &d, int unit, int nunits)
